@@ -50,7 +50,7 @@ struct PeakDesc {
   int fc, hc;              // face nodes (any local coordinate 0) and upper-halo nodes per super-tile
   int gradient;            // 0 spectral (reference), 1 two-point finite difference, 2 four-point
   int full_every;          // every super-tile's particles re-sorted by cell every this many steps (0: never)
-  int native_fft;          // 1: the native 256^3 transform carries the Green multiply (no k_green)
+  int native_fft;          // 1: the native solve makes the forces (no cuFFT, no k_green)
   int bin_shift, bin_min;  // bin capacity: count + (count >> bin_shift) + bin_min, rounded up to BIN_ALIGN
   int bin_grow;            // relayout: room for this many more steps of a bin's growth (region allowing)
   int pad_bg;
@@ -71,6 +71,7 @@ struct PeakDesc {
   float2* spec;            // N*N*(N/2+1) complex spectrum (R2C output)
   float2* gspec;           // 3 gradient spectra
   float* force;            // 3 force grids of N^3 (C2R output)
+  const float* gtab;       // finite-difference gradient factor of each line index (N floats; null: spectral)
 };
 
 struct PeakClock {

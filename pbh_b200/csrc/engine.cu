@@ -44,7 +44,7 @@ struct MeshClass {
   // Dynamic mode: plans for every batch size 1..B over the leading slots, one shared work area.
   std::vector<cufftHandle> r2c_b, c2r_b;
   void* work = nullptr;
-  // The native transform (native_fft.cu) instead of cuFFT, Green multiply fused into it.
+  // The native solve (native_fft.cu) instead of cuFFT and the Green kernel.
   bool native = false;
   int* slot_peak = nullptr;  // device: peak index of each slot
 };
@@ -71,6 +71,7 @@ struct pm_engine {
   long long* d_mode_base = nullptr;
   long long* d_green_base = nullptr;  // Green blocks of the peaks that k_green serves
   int* d_green_peak = nullptr;
+  float* d_gtab = nullptr;            // finite-difference gradient factors of the native peaks
   int ngreen = 0;
   long long ngreenblk = 0;
   long long rtot = 0;                          // slots of each bin buffer
@@ -172,10 +173,8 @@ struct pm_engine {
   }
   int fft_r2c() {
     for (auto& c : classes) {
-      if (c.native) {
-        const int x = (flags & 4) ? extent(c) : (int)c.peaks.size();
-        if (int r = fft_native_r2c(c.N, c.delta, c.spec, x, stream)) return r;
-      } else if (flags & 4) {
+      if (c.native) continue;
+      if (flags & 4) {
         const int x = extent(c);
         if (x) CF(cufftExecR2C(c.r2c_b[x - 1], c.delta, (cufftComplex*)c.spec));
       } else {
@@ -184,12 +183,14 @@ struct pm_engine {
     }
     return 0;
   }
-  int fft_c2r() {
+  // Force grids: the native solve of the native classes, cuFFT's inverse of the others.
+  int forces() {
     const StepArgs A = args();
     for (auto& c : classes) {
       if (c.native) {
         const int x = (flags & 4) ? extent(c) : (int)c.peaks.size();
-        if (int r = fft_native_green_c2r(c.N, c.spec, c.gspec, c.force, A, c.slot_peak, x, stream)) return r;
+        if (int r = fft_native_solve(c.N, c.delta, c.spec, c.gspec, c.force, A, c.slot_peak, x, stream))
+          return r;
       } else if (flags & 4) {
         const int x = extent(c);
         if (x) CF(cufftExecC2R(c.c2r_b[x - 1], (cufftComplex*)c.gspec, c.force));
@@ -202,7 +203,7 @@ struct pm_engine {
 
   // One step for every peak.  With ev != nullptr an event is recorded after each phase and the
   // phase times (push, energy + advance, relayout, priming sort and refresh, deposit with its face
-  // fix-up, R2C, Green, C2R) are accumulated.
+  // fix-up, R2C and Green of the cuFFT classes, native solves and C2R) are accumulated.
   int launch_step(bool with_sort, cudaEvent_t* ev = nullptr, double* phase_ms = nullptr) {
     const StepArgs A = args();
     int k = 0;
@@ -228,9 +229,9 @@ struct pm_engine {
     CU(mark());
     if ((r = fft_r2c())) return r;
     CU(mark());
-    if (ngreenblk) launch_green(A, ngreenblk, stream);  // the native transform does its own
+    if (ngreenblk) launch_green(A, ngreenblk, stream);  // the native solve does its own
     CU(mark());
-    if ((r = fft_c2r())) return r;
+    if ((r = forces())) return r;
     CU(mark());
     CU(cudaGetLastError());
     if (ev) {
@@ -307,7 +308,7 @@ struct pm_engine {
       if (sn.done) cudaEventDestroy(sn.done);
     }
     cudaFree(sort_dbg);
-    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_peak, d_p_base, d_mode_base, d_green_base, d_green_peak, epart,
+    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_peak, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
                     wpart, eslice, ecount, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
                     fill[0], fill[1], ovf_n, ovf_in, keys[0], keys[1], vals[0], vals[1], sstart,
                     sort_gate, layout_gate, refresh_gate, face, halo};
@@ -470,7 +471,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
       P.force = mc.force + 3 * k * N3;
     }
     int n[3] = {(int)N, (int)N, (int)N};
-    if ((E->flags & 8) && fft_native_size((int)N)) {
+    if ((E->flags & 8) && fft_solve_size((int)N)) {
       mc.native = true;
       if ((r = E->alloc(&mc.slot_peak, (size_t)B))) return r;
       CU(cudaMemcpy(mc.slot_peak, mc.peaks.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
@@ -514,6 +515,25 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   }
 
   int r;
+  {
+    // Transfer functions of the finite-difference gradients, in units of 1/length, per line index.
+    std::vector<float> tab;
+    std::vector<std::pair<int, size_t>> at;
+    for (int i = 0; i < npeaks; ++i) {
+      const PeakDesc& P = E->peaks[i];
+      if (!P.native_fft || P.gradient == 0) continue;
+      at.emplace_back(i, tab.size());
+      for (int q = 0; q < P.N; ++q) {
+        const double th = 2.0 * M_PI * (double)(q < P.N / 2 ? q : q - P.N) / (double)P.N;  // k dx
+        tab.push_back((float)(P.gradient == 1 ? sin(th) / P.dx : (8.0 * sin(th) - sin(2.0 * th)) / (6.0 * P.dx)));
+      }
+    }
+    if (!at.empty()) {
+      if ((r = E->alloc(&E->d_gtab, tab.size()))) return r;
+      CU(cudaMemcpy(E->d_gtab, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice));
+      for (auto& p : at) E->peaks[p.first].gtab = E->d_gtab + p.second;
+    }
+  }
   if ((r = E->alloc(&E->d_peaks, npeaks))) return r;
   if ((r = E->alloc(&E->d_clocks, npeaks))) return r;
   if ((r = E->alloc(&E->d_stats, npeaks))) return r;

@@ -1,5 +1,5 @@
-// Native 3D real FFT for meshes of 64^3 to 512^3 (sm_100a), with the Green's-function gradient
-// (pm3d.py:105-112) fused into the inverse.
+// Native 3D real FFT for meshes of 64^3 to 512^3 (sm_100a), and the Poisson solve built from it
+// (pm3d.py:104-112: transform, Green's function, gradient, inverse transforms).
 //
 // Layouts (one field; fields of a batch are consecutive), N = 64, 128, 256 or 512:
 //   real field      r[x][y][z]          N^3 float (the deposit's delta, the force grids)
@@ -18,18 +18,29 @@
 // every exchange hit distinct shared-memory banks within each half-warp (for the 64^3 Z pass,
 // at most two-way).
 //
-// Forward (R2C), three passes over HBM.  Pass Z: a real FFT along z of 256/T consecutive (x, y)
-// lines per CTA (T = N/32) -- a complex FFT of the N/2 packed (even, odd) pairs, then the split
-// into N/2+1 outputs -- written transposed into the kz planes.  Pass Y: 256/(N/16) rows of a kz
-// plane per CTA, in place.  Pass X: the same number of columns of a kz plane per CTA, in place.
-// Every
-// kernel: 256 threads, at most 43 KB of static shared memory, 64 registers, 4 CTAs per SM, no
-// inter-CTA communication.
-// Inverse (C2R).  Pass Y with the Green multiply on load (-i k_i G(k) delta_k / N^3, the
-// Hermitian projection of the kz = 0, N/2 planes, the potential-energy partials), one CTA per
-// row block and gradient component (the three components of a row block adjacent in the grid,
-// so the spectrum is read from HBM once); pass X in place; pass Z, the real inverse along z,
-// written as force rows.
+// The engine's Poisson solve (delta -> three force grids) is five launches:
+//   k_fft_z_r2c   a real FFT along z of CTA/T consecutive (x, y) lines per CTA (T = N/32): a complex
+//                 FFT of the N/2 packed (even, odd) pairs, then the split into N/2+1 outputs,
+//                 written transposed into the kz planes
+//   k_fft_rows    forward Y of the planes' rows, in place
+//   k_solve_cols  per column of a plane: forward X, the Green multiply, inverse X of two fields
+//   k_solve_rows  inverse Y of the three components
+//   k_fft_z_c2r   the real inverse along z of the three components, written as force rows
+// The inverse along x comes first, so the x transform, the Green multiply and the inverse x
+// transform of a column need no pass over memory between them; and because the y and z
+// gradients multiply by factors that do not depend on kx, only two fields leave that pass
+// (A = -i G delta_k and B = g(kx) A; the y and z components are g(ky) A and g(kz) A, multiplied
+// where A is next read) instead of three.  Per cell the passes move 8 + 8 + 12 + 20 + 24 = 72 bytes;
+// the six passes this replaced (Y before X on the way back) moved 88 and did the multiply once per
+// component: 296 -> 244 us at 256^3, 2431 -> 2062 at 512^3, 72 -> 55 at 128^3 (events around the
+// whole solve), with the same errors against float64.  HBM bounds the row and Z passes (5.1-6.9
+// TB/s of these bytes at 256^3); the column pass (55 us for 202 MB) waits on its exchanges.
+// Chaining the plane passes in one persistent kernel, plane by plane so that L2 holds a plane from
+// pass to pass, was slower (350 us at 256^3: its item claims, waits and fences cost more than
+// the HBM traffic they save).
+// The plain transforms (pm_rfft3_native, pm_irfft3_native) are three launches each: the Z passes
+// above and one launch per axis of the planes (k_fft_rows, k_fft_cols), in place.
+// No kernel communicates between CTAs.
 // Twiddles come from a 512-entry table of W_512^e computed in double precision on the host; the
 // register DFTs use the exact constants cos(pi/8), cos(pi/4), cos(3 pi/8).
 // Transforms are unnormalised like cuFFT's; the Green factor carries numpy's 1/N^3.
@@ -43,7 +54,12 @@
 namespace {
 
 constexpr int TWN = 512;           // entries of the twiddle table
-constexpr int CTA = 256;           // threads of every kernel here
+
+// Threads per CTA for mesh N: 256, fewer where the mesh has few lines, so that a single small mesh
+// still spreads over the SMs (a pass over the planes of one 64^3 mesh is 132 CTAs of 64 threads
+// rather than 33 of 256; its five launches 34.8 -> 33.7 us, 58 -> 55 us at 128^3).
+template <int N>
+__host__ __device__ constexpr int cta() { return N <= 64 ? 64 : N == 128 ? 128 : 256; }
 
 __device__ float2 g_tw[TWN];       // exp(-2 pi i e / 512) of this device
 
@@ -132,16 +148,20 @@ __device__ __forceinline__ int line_slot(int k1, int t) {
 
 // The transform of one line of L = 16 T points shared by its T threads: thread t holds v[n1] =
 // x[T n1 + t] on entry and u[p] = X[line_k<T>(t, p)] on exit.  row: the line's exchange row in
-// shared memory (16 T values); tl: W_L^{t k1} at [k1 * T + t].  The threads of a line are
+// shared memory (16 T values); tl: W_L^{t k1} at [k1 * T + t] (the forward ones, conjugated here
+// for the inverse).  The threads of a line are
 // consecutive lanes of one warp (T = 32: the whole warp).  Ends after the exchange has been read:
 // the caller must barrier before it writes the row again.
+template <bool INV>
+__device__ __forceinline__ float2 twc(float2 w) { return INV ? cconj(w) : w; }
+
 template <bool INV, int T>
 __device__ __forceinline__ void line_fft(float2 (&v)[16], float2 (&u)[16], float2* row, const float2* tl, int t) {
   dft_reg<INV, 16, 0, 16>(v);
 #pragma unroll
   for (int p = 0; p < 16; ++p) {
     const int k1 = brev(p, 4);
-    row[line_slot<T>(k1, t)] = k1 ? cmul(v[p], tl[k1 * T + t]) : v[p];
+    row[line_slot<T>(k1, t)] = k1 ? cmul(v[p], twc<INV>(tl[k1 * T + t])) : v[p];
   }
   __syncthreads();
   if constexpr (T <= 16) {
@@ -159,7 +179,7 @@ __device__ __forceinline__ void line_fft(float2 (&v)[16], float2 (&u)[16], float
     dft_reg<INV, 16, 0, 16>(u);  // u[p] = A_t0[m], m = brev(p)
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
-      if (t0) u[p] = cmul(u[p], tl[brev(p, 4) * 32 + 16]);  // W_32^m = W_512^{16 m}
+      if (t0) u[p] = cmul(u[p], twc<INV>(tl[brev(p, 4) * 32 + 16]));  // W_32^m = W_512^{16 m}
       const float ox = __shfl_xor_sync(0xffffffffu, u[p].x, 1), oy = __shfl_xor_sync(0xffffffffu, u[p].y, 1);
       // X[k1 + 16 m] = A_0 + W_32^m A_1 (even lane), X[k1 + 16 m + 256] = A_0 - W_32^m A_1 (odd lane)
       u[p] = t0 ? make_float2(ox - u[p].x, oy - u[p].y) : make_float2(u[p].x + ox, u[p].y + oy);
@@ -170,7 +190,7 @@ __device__ __forceinline__ void line_fft(float2 (&v)[16], float2 (&u)[16], float
 // Z pass geometry for mesh N: a z line is M = N/2 packed pairs shared by T = M/16 threads.
 template <int N>
 struct ZGeo {
-  static constexpr int M = N / 2, NH = N / 2 + 1, T = M / 16, L = CTA / T;  // L lines per CTA
+  static constexpr int CTA = cta<N>(), M = N / 2, NH = N / 2 + 1, T = M / 16, L = CTA / T;  // L lines per CTA
   // Row stride (float2) of a line in shared memory and the swizzle of its natural-order row,
   // chosen so that the exchange, the row writes and the column reads of the split are free of
   // bank conflicts (T = 2: at most two-way).
@@ -182,12 +202,13 @@ struct ZGeo {
   __device__ static int sw(int l) { return T >= 8 ? (l >> 1) & 7 : (l & 15); }
 };
 
-// Shared twiddle tables of the Z passes: tw[e] = W_N^e (e <= N/2), tl[k1 * T + t] = W_M^{t k1}.
+// Shared twiddle tables of the Z passes: tw[e] = W_N^e (e <= N/2, conjugated for the inverse),
+// tl[k1 * T + t] = W_M^{t k1}.
 template <bool INV, int N>
 __device__ __forceinline__ void load_ztw(float2* tw, float2* tl) {
   using G = ZGeo<N>;
-  for (int i = threadIdx.x; i <= G::M; i += CTA) tw[i] = tw_global<INV, N>(i);
-  for (int i = threadIdx.x; i < 16 * G::T; i += CTA) tl[i] = tw_global<INV, G::M>((i / G::T) * (i % G::T));
+  for (int i = threadIdx.x; i <= G::M; i += G::CTA) tw[i] = tw_global<INV, N>(i);
+  for (int i = threadIdx.x; i < 16 * G::T; i += G::CTA) tl[i] = tw_global<false, G::M>((i / G::T) * (i % G::T));
 }
 
 __device__ __forceinline__ void cpa16(void* dst, const void* src) {
@@ -196,11 +217,20 @@ __device__ __forceinline__ void cpa16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// Whether the peak of an engine slot deposited this step (only then have its density and, after
+// the solve, its forces changed).
+__device__ __forceinline__ bool slot_active(const StepArgs& A, const int* slot_peak, int slot) {
+  return A.clocks[slot_peak[slot]].dep != 0;
+}
+
 // Pass Z forward: fields in[f][x][y][z] -> planes out[f][kz][x][y].  A CTA takes L consecutive
-// (x, y) lines.  grid (N^2/L, nf).
+// (x, y) lines.  grid (N^2/L, nf).  slot_peak (engine solve): field f is slot f's density, idle
+// slots are skipped.
 template <int N>
-__global__ void __launch_bounds__(CTA, 4) k_fft_z_r2c(const float* __restrict__ in, float2* __restrict__ out) {
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_z_r2c(const float* __restrict__ in, float2* __restrict__ out,
+                                                       StepArgs A, const int* slot_peak) {
   using G = ZGeo<N>;
+  if (slot_peak && !slot_active(A, slot_peak, blockIdx.y)) return;
   __shared__ float2 tw[G::M + 1], tl[16 * G::T];
   __shared__ __align__(16) float2 xb[G::L * G::X];
   load_ztw<false, N>(tw, tl);
@@ -223,7 +253,7 @@ __global__ void __launch_bounds__(CTA, 4) k_fft_z_r2c(const float* __restrict__ 
   __syncthreads();
   // X_k = E_k + W_N^k O_k with E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2
   float2* dst = out + (long long)f * G::NH * G::N2 + g0;
-  for (int e = threadIdx.x; e < G::NH * G::L; e += CTA) {
+  for (int e = threadIdx.x; e < G::NH * G::L; e += G::CTA) {
     const int k = e / G::L, ll = e - k * G::L, sl = G::sw(ll);
     const float2* zr = xb + ll * G::X;
     const float2 zk = zr[(k & (G::M - 1)) ^ sl];
@@ -234,31 +264,58 @@ __global__ void __launch_bounds__(CTA, 4) k_fft_z_r2c(const float* __restrict__ 
   }
 }
 
-// Pass Z inverse: planes in[f][kz][x][y] -> fields out[f][x][y][z].  A CTA takes L consecutive
-// (x, y) lines.  grid (N^2/L, nf).
 template <int N>
-__global__ void __launch_bounds__(CTA, 4) k_fft_z_c2r(const float2* __restrict__ in, float* __restrict__ out) {
+__device__ __forceinline__ float kl(int i, float kf) { return kf * (float)(i < N / 2 ? i : i - N); }
+// Gradient factor of line index i: the spectral k (gtab null), or the tabulated transfer function
+// of a finite difference (a table, because sinf unrolled over a thread's 16 values would fill the
+// instruction cache).
+template <int N>
+__device__ __forceinline__ float gfac(int i, float kf, const float* __restrict__ gtab) {
+  return gtab ? __ldg(gtab + i) : kl<N>(i, kf);
+}
+
+// Pass Z inverse: planes in[f][kz][x][y] -> fields out[f][x][y][z].  A CTA takes L consecutive
+// (x, y) lines.  grid (N^2/L, nf).  slot_peak (engine solve): field 3 s + c is component c of
+// slot s, idle slots are skipped, and the z component arrives without its gradient factor g(kz),
+// which is applied to each line here.
+template <int N>
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_z_c2r(const float2* __restrict__ in, float* __restrict__ out,
+                                                       StepArgs A, const int* slot_peak) {
   using G = ZGeo<N>;
   __shared__ float2 tw[G::M + 1], tl[16 * G::T];
   __shared__ __align__(16) float2 xb[G::TILE];  // the kz-major tile, later the exchange rows
   const long long g0 = (long long)blockIdx.x * G::L;
   const int f = blockIdx.y;
+  if (slot_peak && !slot_active(A, slot_peak, f / 3)) return;
   const float2* src = in + (long long)f * G::NH * G::N2 + g0;
-  for (int e = threadIdx.x; e < G::NH * G::L / 2; e += CTA) {  // two complex values (16 bytes) per copy
+  for (int e = threadIdx.x; e < G::NH * G::L / 2; e += G::CTA) {  // two complex values (16 bytes) per copy
     const int k = e / (G::L / 2), ll = 2 * (e - k * (G::L / 2));
     cpa16(xb + k * G::C + ll, src + (long long)k * G::N2 + ll);
   }
   load_ztw<true, N>(tw, tl);
+  const bool zgrad = slot_peak && f % 3 == 2;
+  float kf = 0.f;
+  const float* gtab = nullptr;
+  if (zgrad) {
+    const PeakDesc& P = A.peaks[slot_peak[f / 3]];
+    kf = (float)(2.0 * M_PI / P.L);
+    gtab = P.gtab;
+  }
   cpa_wait();
   __syncthreads();
   const int t = threadIdx.x % G::T, l = threadIdx.x / G::T;
   // Z_n = E_n + i O_n with E = X_n + conj X_{M-n}, O = (X_n - conj X_{M-n}) W_N^{-n}; a C2R
-  // reads only the real parts of X_0 and X_M.
+  // reads only the real parts of X_0 and X_M (numpy's irfftn does the same after its complex
+  // transforms along x and y).
   float2 v[16], u[16];
 #pragma unroll
   for (int n1 = 0; n1 < 16; ++n1) {
     const int n = G::T * n1 + t;
     float2 xk = xb[n * G::C + l], xm = cconj(xb[(G::M - n) * G::C + l]);
+    if (zgrad) {
+      xk = cscale(xk, gtab ? __ldg(gtab + n) : kf * (float)n);
+      xm = cscale(xm, gtab ? __ldg(gtab + G::M - n) : kf * (float)(G::M - n));
+    }
     if (n == 0) {
       xk.y = 0.f;
       xm.y = 0.f;
@@ -273,154 +330,34 @@ __global__ void __launch_bounds__(CTA, 4) k_fft_z_c2r(const float2* __restrict__
   for (int p = 0; p < 16; ++p) dst[line_k<G::T>(t, p)] = u[p];  // (r[2n], r[2n+1])
 }
 
-// Green's-function multiply of one spectral value (the per-mode work of k_green).
-struct GreenPlane {
-  float s_c, kf, dx, sd2;
-  int gm;
-};
-template <int N>
-__device__ __forceinline__ float kl(int i, float kf) { return kf * (float)(i < N / 2 ? i : i - N); }
-__device__ __forceinline__ float gk(float k, float dx, int mode) {
-  if (mode == 1) return sinf(k * dx) / dx;
-  if (mode == 2) return (8.0f * sinf(k * dx) - sinf(2.0f * k * dx)) / (6.0f * dx);
-  return k;
-}
-// -i g_comp(k) G(k) delta_k at mode (x, y, kz) of a plane whose values start at plane; adds the
-// mode's weight in the potential energy to w (component 0).
-template <int N>
-__device__ __forceinline__ float2 green_mode(float2 v, int x, int y, int kz, int comp, const GreenPlane& gp,
-                                             const float2* plane, double& w) {
-  const float kx = kl<N>(x, gp.kf), ky = kl<N>(y, gp.kf), kzv = gp.kf * (float)kz;
-  const float k2 = kx * kx + ky * ky + kzv * kzv;
-  if (x == 0 && y == 0 && kz == 0) return make_float2(0.f, 0.f);
-  float G = gp.s_c / k2;
-  if (gp.sd2 > 0.f) G *= expf(-0.5f * k2 * gp.sd2);
-  const float kc = comp == 0 ? kx : (comp == 1 ? ky : kzv);
-  const float g = gk(kc, gp.dx, gp.gm) * G;
-  if (comp == 0) w += (double)(((kz == 0 || kz == N / 2) ? 1.0f : 2.0f) * G * (v.x * v.x + v.y * v.y));
-  float2 o = make_float2(g * v.y, -g * v.x);  // -i g v
-  if (kz == 0 || kz == N / 2) {  // (o + conj(o at -k)) / 2: numpy's C2R sees this plane's Hermitian part
-    const int px = (-x) & (N - 1), py = (-y) & (N - 1);
-    const float2 dp = plane[(long long)px * N + py];
-    const float kpc = comp == 0 ? kl<N>(px, gp.kf) : (comp == 1 ? kl<N>(py, gp.kf) : kzv);
-    const float h = gk(kpc, gp.dx, gp.gm) * G;
-    o = make_float2(0.5f * (o.x + h * dp.y), 0.5f * (o.y + h * dp.x));
-  }
-  return o;
-}
-
 // Plane-pass geometry for mesh N: a line (row or column) of N points shared by T = N/16 threads,
-// B = 256/T lines per CTA.
+// B = CTA/T lines per CTA, R = N/B blocks of lines per plane.
 template <int N>
 struct PGeo {
-  static constexpr int T = N / 16, B = CTA / T, NH = N / 2 + 1;
+  static constexpr int CTA = cta<N>(), T = N / 16, B = CTA / T, NH = N / 2 + 1, R = N / B;
   static constexpr int RS = N + (T <= 8 ? T : 0);  // row stride in shared memory (bank-conflict free)
+  static constexpr size_t COLS_SMEM = sizeof(float2) * (16 * T * B + 16 * CTA + 16 * T);  // k_solve_cols
   static constexpr long long N2 = (long long)N * N, N3 = N2 * N;
   static_assert(B <= N, "a CTA's rows (columns) lie in one plane");
 };
 
-template <bool INV, int N>
+template <int N>
 __device__ __forceinline__ void load_ptw(float2* tl) {
   constexpr int T = PGeo<N>::T;
-  for (int i = threadIdx.x; i < 16 * T; i += CTA) tl[i] = tw_global<INV, N>((i / T) * (i % T));
+  for (int i = threadIdx.x; i < 16 * T; i += cta<N>()) tl[i] = tw_global<false, N>((i / T) * (i % T));
 }
 
-// Pass Y: rows x = B rb + r of one kz plane, T threads per row.  Forward: in = out =
-// planes[slot][kz][x][y] (in place: a CTA reads its rows before it writes them).  Inverse with
-// GREEN: in = spectrum planes[slot][kz][kx][ky], out = planes[slot][comp][kz][kx][y], the
-// multiply applied on load; slot_peak maps a slot to its peak.  Inverse without GREEN: in and
-// out [f][kz][.][.].  grid (N/B * nslots * NH * ncomp), block index
-// ((slot * NH + kz) * (N/B) + rb) * ncomp + comp (the components of a row block adjacent).
-template <int N, bool INV, bool GREEN>
-__global__ void __launch_bounds__(CTA, 4) k_fft_rows(const float2* in, float2* out, StepArgs A, const int* slot_peak,
-                                                      int ncomp) {
-  using G = PGeo<N>;
-  constexpr int T = G::T, B = G::B;
-  __shared__ float2 tl[16 * T];
-  __shared__ __align__(16) float2 buf[B * G::RS];
-  load_ptw<INV, N>(tl);
-  const int bi = blockIdx.x, comp = bi % ncomp, q = bi / ncomp, rb = q % (N / B), pl = q / (N / B);
-  const int slot = pl / G::NH, kz = pl - slot * G::NH;
-  GreenPlane gp{};
-  int pk = 0;
-  if (GREEN) {
-    pk = slot_peak[slot];
-    if (!A.clocks[pk].has_delta) return;
-    const PeakDesc& P = A.peaks[pk];
-    gp.s_c = (float)(-1.5 * PM_H_I * PM_H_I / A.clocks[pk].a_grid / (double)G::N3);
-    gp.kf = (float)(2.0 * M_PI / P.L);
-    gp.dx = (float)P.dx;
-    gp.sd2 = P.smooth > 0 ? (float)(P.smooth * P.dx) * (float)(P.smooth * P.dx) : 0.f;
-    gp.gm = P.gradient;
-  }
-  const int t = threadIdx.x % T, r = threadIdx.x / T, x = B * rb + r;
-  const float2* plane = in + (long long)pl * G::N2;
-  float2 v[16], u[16];
-#pragma unroll
-  for (int n1 = 0; n1 < 16; ++n1) v[n1] = plane[(long long)x * N + T * n1 + t];
-  float2* row = buf + r * G::RS;
-  double w = 0.0;
-  if (GREEN) {
-    if (kz != 0 && kz != N / 2 && (gp.gm == 0 || comp != 1)) {
-      // Interior planes (no Hermitian partner, k != 0), with the gradient factor constant along
-      // the row (components x and z) or the spectral ky (component y): unrolled, in registers.
-      const float kx = kl<N>(x, gp.kf), kzv = gp.kf * (float)kz, a = kx * kx + kzv * kzv;
-      const float gc = gk(comp == 0 ? kx : kzv, gp.dx, gp.gm);
-#pragma unroll
-      for (int n1 = 0; n1 < 16; ++n1) {
-        const float ky = kl<N>(T * n1 + t, gp.kf), k2 = a + ky * ky;
-        float Gk = gp.s_c / k2;
-        if (gp.sd2 > 0.f) Gk *= expf(-0.5f * k2 * gp.sd2);
-        const float g = (comp == 1 ? ky : gc) * Gk;
-        const float2 d = v[n1];
-        if (comp == 0) w += (double)(2.0f * Gk * (d.x * d.x + d.y * d.y));
-        v[n1] = make_float2(g * d.y, -g * d.x);  // -i g d
-      }
-    } else {
-      // The general multiply in a rolled loop over this thread's slots of its row in shared
-      // memory (one copy of its code keeps the kernel within the instruction cache).
-      float2* own = row + t;
-#pragma unroll
-      for (int n1 = 0; n1 < 16; ++n1) own[T * n1] = v[n1];
-#pragma unroll 1
-      for (int n1 = 0; n1 < 16; ++n1) own[T * n1] = green_mode<N>(own[T * n1], x, T * n1 + t, kz, comp, gp, plane, w);
-#pragma unroll
-      for (int n1 = 0; n1 < 16; ++n1) v[n1] = own[T * n1];
-    }
-    if (comp == 0)
-      for (int d = 16; d > 0; d >>= 1) w += __shfl_down_sync(0xffffffffu, w, d);
-  }
-  __syncthreads();  // table; the rolled Green loop's slots
-  line_fft<INV, T>(v, u, row, tl, t);
-  float2* dst = out + ((long long)(slot * ncomp + comp) * G::NH + kz) * G::N2 + (long long)x * N;
-#pragma unroll
-  for (int p = 0; p < 16; ++p) dst[line_k<T>(t, p)] = u[p];
-  if (GREEN && comp == 0 && (threadIdx.x & 31) == 0)
-    A.wpart[A.peaks[pk].mode_base * (PM_THREADS / 32) + ((long long)kz * (N / B) + rb) * (CTA / 32) + (threadIdx.x >> 5)] = w;
-}
-
-// Pass X, in place: columns ky = B cb + j of one kz plane, T threads per column.  Consecutive
-// lanes hold consecutive columns, so each warp access covers 32/B rows, B columns (8 B bytes)
-// of each.  grid (N/B * nplanes).
-template <int N, bool INV>
-__global__ void __launch_bounds__(CTA, 4) k_fft_cols(float2* io) {
-  using G = PGeo<N>;
-  constexpr int T = G::T, B = G::B;
-  __shared__ float2 tl[16 * T];
-  __shared__ __align__(16) float2 buf[16 * T * B];  // [k1][t][j]
-  load_ptw<INV, N>(tl);
-  const int cb = blockIdx.x % (N / B), pl = blockIdx.x / (N / B);
-  const int j = threadIdx.x % B, t = threadIdx.x / B, ky = B * cb + j;
-  float2* plane = io + (long long)pl * G::N2 + ky;
-  float2 v[16], u[16];
-#pragma unroll
-  for (int n1 = 0; n1 < 16; ++n1) v[n1] = plane[(long long)(T * n1 + t) * N];
-  __syncthreads();
+// The transform of a column shared by T threads of different warps (consecutive lanes hold
+// consecutive columns): v[n1] = x[T n1 + t] on entry, u[p] = X[line_k<T>(t, p)] on exit.  buf:
+// [k1][t][j], the whole CTA's.  LEAD: a barrier first, when buf may still be read.
+template <bool INV, int T, int B, bool LEAD>
+__device__ __forceinline__ void col_fft(float2 (&v)[16], float2 (&u)[16], float2* buf, const float2* tl, int t, int j) {
   dft_reg<INV, 16, 0, 16>(v);
+  if (LEAD) __syncthreads();
 #pragma unroll
   for (int p = 0; p < 16; ++p) {
     const int k1 = brev(p, 4);
-    buf[(k1 * T + t) * B + j] = k1 ? cmul(v[p], tl[k1 * T + t]) : v[p];
+    buf[(k1 * T + t) * B + j] = k1 ? cmul(v[p], twc<INV>(tl[k1 * T + t])) : v[p];
   }
   __syncthreads();
   if constexpr (T <= 16) {
@@ -431,56 +368,208 @@ __global__ void __launch_bounds__(CTA, 4) k_fft_cols(float2* io) {
       for (int i = 0; i < T; ++i) u[T * s + i] = buf[((t + T * s) * T + i) * B + j];
     dft_groups<INV, T>(u);
   } else {
-    static_assert(T == 32, "column pass for N <= 512");
+    static_assert(T <= 32, "column pass for N <= 512");
     const int k1 = t >> 1, t0 = t & 1;
 #pragma unroll
     for (int i = 0; i < 16; ++i) u[i] = buf[(k1 * 32 + 2 * i + t0) * B + j];
     dft_reg<INV, 16, 0, 16>(u);
 #pragma unroll
     for (int p = 0; p < 16; ++p) {
-      if (t0) u[p] = cmul(u[p], tl[brev(p, 4) * 32 + 16]);  // W_32^m
+      if (t0) u[p] = cmul(u[p], twc<INV>(tl[brev(p, 4) * 32 + 16]));  // W_32^m
       // partner: thread t ^ 1 of the same column, B lanes away
       const float ox = __shfl_xor_sync(0xffffffffu, u[p].x, B), oy = __shfl_xor_sync(0xffffffffu, u[p].y, B);
       u[p] = t0 ? make_float2(ox - u[p].x, oy - u[p].y) : make_float2(u[p].x + ox, u[p].y + oy);
     }
   }
+}
+
+// Rows x = B rb + r of kz planes, T threads per row, [f][kz][.][.] (the plain transforms; in place
+// allowed: a CTA reads its rows before it writes them).  grid (N/B * nplanes).
+template <int N, bool INV>
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_rows(const float2* in, float2* out) {
+  using G = PGeo<N>;
+  constexpr int T = G::T;
+  __shared__ float2 tl[16 * T];
+  __shared__ __align__(16) float2 buf[G::B * G::RS];
+  load_ptw<N>(tl);
+  const int rb = blockIdx.x % G::R, pl = blockIdx.x / G::R;
+  const int t = threadIdx.x % T, r = threadIdx.x / T;
+  const long long o = (long long)pl * G::N2 + (long long)(G::B * rb + r) * N;
+  float2 v[16], u[16];
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = in[o + T * n1 + t];
+  __syncthreads();  // table
+  line_fft<INV, T>(v, u, buf + r * G::RS, tl, t);
+#pragma unroll
+  for (int p = 0; p < 16; ++p) out[o + line_k<T>(t, p)] = u[p];
+}
+
+// Columns ky = B cb + j of kz planes, in place (the plain transforms).  Each warp access covers 32/B
+// rows, B columns (8 B bytes) of each.  grid (N/B * nplanes).
+template <int N, bool INV>
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_cols(float2* io) {
+  using G = PGeo<N>;
+  constexpr int T = G::T, B = G::B;
+  __shared__ float2 tl[16 * T];
+  __shared__ __align__(16) float2 buf[16 * T * B];
+  load_ptw<N>(tl);
+  const int cb = blockIdx.x % G::R, pl = blockIdx.x / G::R;
+  const int j = threadIdx.x % B, t = threadIdx.x / B;
+  float2* plane = io + (long long)pl * G::N2 + B * cb + j;
+  float2 v[16], u[16];
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = plane[(long long)(T * n1 + t) * N];
+  __syncthreads();
+  col_fft<INV, T, B, false>(v, u, buf, tl, t, j);
 #pragma unroll
   for (int p = 0; p < 16; ++p) plane[(long long)line_k<T>(t, p) * N] = u[p];
 }
 
+// ------------------------------------------------------------------------------------------
+// Column pass of the solve: columns ky = B cb + j of one kz plane, T threads per column: forward X,
+// A = -i G delta_k, inverse X of B = g(kx) A (to the x component's plane) and of A (in place).
+// A waits in shared memory while B is transformed: kept in registers (32 more) it would leave two
+// CTAs of 256 threads per SM instead of three.  Planes in descending order: the row pass before
+// took them in ascending order, so the ones it left in L2 come first.  grid (N/B * nplanes).
 template <int N>
-int r2c_n(const float* delta, float2* spec, int nslots, cudaStream_t s) {
+__global__ void __launch_bounds__(cta<N>(), 768 / cta<N>())
+    k_solve_cols(float2* spec, float2* gspec, const __grid_constant__ StepArgs A, const int* slot_peak) {
+  using G = PGeo<N>;
+  constexpr int T = G::T, B = G::B, R = G::R;
+  extern __shared__ __align__(16) float2 s_cols[];
+  float2* const buf = s_cols;                              // exchange buffer
+  float2* const keep = buf + 16 * T * B + threadIdx.x;     // this thread's 16 values of A
+  float2* const tl = buf + 16 * T * B + 16 * G::CTA;
+  const int idx = blockIdx.x % R, pl = gridDim.x / R - 1 - blockIdx.x / R;
+  const int slot = pl / G::NH, kz = pl - slot * G::NH, pk = slot_peak[slot];
+  if (!A.clocks[pk].dep) return;
+  load_ptw<N>(tl);
+  const int tid = threadIdx.x, j = tid % B, t = tid / B, ky = B * idx + j;
+  float2* const col = spec + (long long)pl * G::N2 + ky;
+  float2 v[16], u[16];
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = col[(T * n1 + t) * N];
+  __syncthreads();  // table
+  col_fft<false, T, B, false>(v, u, buf, tl, t, j);
+  // The spectrum of this thread's kx = T n1 + t into v.
+  if constexpr (T <= 16) {
+#pragma unroll
+    for (int p = 0; p < 16; ++p) v[p / T + (16 / T) * brev(p % T, log2i<T>())] = u[p];
+  } else {  // a thread's outputs are not its inputs' places: through the exchange buffer
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) buf[line_k<T>(t, p) * B + j] = u[p];
+    __syncthreads();
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = buf[(T * n1 + t) * B + j];
+  }
+  const PeakDesc& P = A.peaks[pk];
+  const float s_c = (float)(-1.5 * PM_H_I * PM_H_I / A.clocks[pk].a_grid / (double)G::N3);
+  const float kf = (float)(2.0 * M_PI / P.L);
+  const float sd2 = P.smooth > 0 ? (float)(P.smooth * P.dx) * (float)(P.smooth * P.dx) : 0.f;
+  const float kyv = kl<N>(ky, kf), kzv = kf * (float)kz, yz2 = kyv * kyv + kzv * kzv;
+  double w = 0.0;  // the modes' potential energy: terms in FP32, summed in FP64
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) {
+    const float kx = kf * (float)(T * n1 + t - (n1 < 8 ? 0 : N)), k2 = kx * kx + yz2;
+    float Gk = s_c / k2;
+    if (sd2 > 0.f) Gk *= expf(-0.5f * k2 * sd2);
+    if (n1 == 0) Gk = k2 == 0.f ? 0.f : Gk;  // the mean
+    const float2 d = v[n1];
+    w += (double)(Gk * (d.x * d.x + d.y * d.y));
+    const float2 a = make_float2(Gk * d.y, -Gk * d.x);  // -i G delta_k
+    keep[n1 * G::CTA] = a;
+    v[n1] = cscale(a, kx);
+  }
+  if (const float* const gtab = P.gtab) {
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = cscale(keep[n1 * G::CTA], __ldg(gtab + T * n1 + t));
+  }
+  for (int d = 16; d > 0; d >>= 1) w += __shfl_down_sync(0xffffffffu, w, d);
+  if ((tid & 31) == 0)
+    A.wpart[P.mode_base * (PM_THREADS / 32) + ((long long)kz * R + idx) * (G::CTA / 32) + (tid >> 5)] =
+        (kz == 0 || kz == N / 2) ? w : 2.0 * w;  // the half spectrum counts 0 < kz < N/2 twice
+  col_fft<true, T, B, true>(v, u, buf, tl, t, j);
+  float2* const outx = gspec + ((long long)(3 * slot) * G::NH + kz) * G::N2 + ky;
+#pragma unroll
+  for (int p = 0; p < 16; ++p) outx[line_k<T>(t, p) * N] = u[p];
+  asm volatile("" ::: "memory");  // A is fetched after B is stored (registers)
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = keep[n1 * G::CTA];
+  col_fft<true, T, B, true>(v, u, buf, tl, t, j);
+#pragma unroll
+  for (int p = 0; p < 16; ++p) col[line_k<T>(t, p) * N] = u[p];
+}
+
+// Row pass of the solve, one component: inverse Y of rows x = B rb + r of one kz plane, the x
+// component from B in place, the y component from g(ky) A, the z component from A (its factor g(kz)
+// is applied by the inverse Z pass).  The three components of a row block are adjacent in the
+// grid, so that A is read from HBM once.  grid (3 * N/B * nplanes).
+template <int N>
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>())
+    k_solve_rows(const float2* spec, float2* gspec, const __grid_constant__ StepArgs A, const int* slot_peak) {
+  using G = PGeo<N>;
+  constexpr int T = G::T, B = G::B, R = G::R;
+  __shared__ float2 tl[16 * T];
+  __shared__ __align__(16) float2 buf[G::B * G::RS];
+  const int comp = blockIdx.x % 3, q = blockIdx.x / 3, rb = q % R, pl = q / R;
+  const int slot = pl / G::NH, kz = pl - slot * G::NH, pk = slot_peak[slot];
+  if (!A.clocks[pk].dep) return;
+  load_ptw<N>(tl);
+  const int t = threadIdx.x % T, r = threadIdx.x / T, o = (B * rb + r) * N;
+  float2* const dst = gspec + ((long long)(3 * slot + comp) * G::NH + kz) * G::N2 + o;
+  const float2* const src = comp == 0 ? dst : spec + (long long)pl * G::N2 + o;
+  float2 v[16], u[16];
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = src[T * n1 + t];
+  if (comp == 1) {
+    const PeakDesc& P = A.peaks[pk];
+    const float kf = (float)(2.0 * M_PI / P.L);
+    const float* const gtab = P.gtab;
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = cscale(v[n1], gfac<N>(T * n1 + t, kf, gtab));
+  }
+  __syncthreads();  // table
+  line_fft<true, T>(v, u, buf + r * G::RS, tl, t);
+#pragma unroll
+  for (int p = 0; p < 16; ++p) dst[line_k<T>(t, p)] = u[p];
+}
+
+template <int N>
+int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
   using Z = ZGeo<N>;
   using G = PGeo<N>;
-  const unsigned planes = (unsigned)(nslots * G::NH), blocks = (unsigned)(N / G::B) * planes;
-  k_fft_z_r2c<N><<<dim3((unsigned)(Z::N2 / Z::L), nslots), CTA, 0, s>>>(delta, spec);
-  k_fft_rows<N, false, false><<<blocks, CTA, 0, s>>>(spec, spec, StepArgs{}, nullptr, 1);
-  k_fft_cols<N, false><<<blocks, CTA, 0, s>>>(spec);
+  const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
+  k_fft_z_r2c<N><<<dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s>>>(x, spec, StepArgs{}, nullptr);
+  k_fft_rows<N, false><<<blocks, G::CTA, 0, s>>>(spec, spec);
+  k_fft_cols<N, false><<<blocks, G::CTA, 0, s>>>(spec);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
 template <int N>
-int green_c2r_n(const float2* spec, float2* gwork, float* force, const StepArgs& A, const int* slot_peak, int nslots,
-                cudaStream_t s) {
+int solve_n(const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A, const int* slot_peak,
+            int nslots, cudaStream_t s) {
   using Z = ZGeo<N>;
   using G = PGeo<N>;
-  const unsigned blocks = (unsigned)(N / G::B) * (unsigned)(nslots * G::NH) * 3u;
-  k_fft_rows<N, true, true><<<blocks, CTA, 0, s>>>(spec, gwork, A, slot_peak, 3);
-  k_fft_cols<N, true><<<blocks, CTA, 0, s>>>(gwork);
-  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), CTA, 0, s>>>(gwork, force);
+  const unsigned blocks = (unsigned)G::R * (unsigned)(nslots * G::NH);
+  k_fft_z_r2c<N><<<dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s>>>(delta, spec, A, slot_peak);
+  k_fft_rows<N, false><<<blocks, G::CTA, 0, s>>>(spec, spec);
+  k_solve_cols<N><<<blocks, G::CTA, G::COLS_SMEM, s>>>(spec, gspec, A, slot_peak);
+  k_solve_rows<N><<<3 * blocks, G::CTA, 0, s>>>(spec, gspec, A, slot_peak);
+  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s>>>(gspec, force, A, slot_peak);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
 template <int N>
-int c2r_n(const float2* spec, float2* gwork, float* out, int nfields, cudaStream_t s) {
+int c2r_n(const float2* spec, float2* work, float* out, int nfields, cudaStream_t s) {
   using Z = ZGeo<N>;
   using G = PGeo<N>;
-  const unsigned blocks = (unsigned)(N / G::B) * (unsigned)(nfields * G::NH);
-  k_fft_rows<N, true, false><<<blocks, CTA, 0, s>>>(spec, gwork, StepArgs{}, nullptr, 1);
-  k_fft_cols<N, true><<<blocks, CTA, 0, s>>>(gwork);
-  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), nfields), CTA, 0, s>>>(gwork, out);
+  const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
+  k_fft_rows<N, true><<<blocks, G::CTA, 0, s>>>(spec, work);
+  k_fft_cols<N, true><<<blocks, G::CTA, 0, s>>>(work);
+  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s>>>(work, out, StepArgs{}, nullptr);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -488,19 +577,44 @@ int c2r_n(const float2* spec, float2* gwork, float* out, int nfields, cudaStream
 }  // namespace
 
 bool fft_native_size(int N) { return N == 64 || N == 128 || N == 256 || N == 512; }
+bool fft_solve_size(int N) { return N == 32 || fft_native_size(N); }
 
-// Per-device set-up: the twiddle table.  Call with the device current.
+// Per-device set-up: the twiddle table and the shared-memory limits.  Call with the device current.
 int fft_native_init() {
   float2 h[TWN];
   for (int k = 0; k < TWN; ++k) {
     const double a = -2.0 * M_PI * (double)k / (double)TWN;
     h[k] = make_float2((float)cos(a), (float)sin(a));
   }
-  const cudaError_t e = cudaMemcpyToSymbol(g_tw, h, sizeof(h));
+  cudaError_t e = cudaMemcpyToSymbol(g_tw, h, sizeof(h));
+  auto smem = [&](auto* kernel, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  smem(k_solve_cols<32>, PGeo<32>::COLS_SMEM);
+  smem(k_solve_cols<64>, PGeo<64>::COLS_SMEM);
+  smem(k_solve_cols<128>, PGeo<128>::COLS_SMEM);
+  smem(k_solve_cols<256>, PGeo<256>::COLS_SMEM);
+  smem(k_solve_cols<512>, PGeo<512>::COLS_SMEM);
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
-// delta fields [slot][x][y][z] -> spectra [slot][kz][kx][ky]
+// delta fields [slot][x][y][z] -> 3 force grids per slot [slot][comp][x][y][z] (the Poisson solve);
+// spec [slot][kz][.][.] and gspec [slot][comp][kz][.][.] are work space.
+int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
+                     const int* slot_peak, int nslots, cudaStream_t s) {
+  if (nslots <= 0) return 0;
+  switch (N) {
+    case 32: return solve_n<32>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    case 64: return solve_n<64>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    case 128: return solve_n<128>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    case 256: return solve_n<256>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    case 512: return solve_n<512>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    default: return -2000;
+  }
+}
+
+namespace {
+// Plain unnormalised forward: fields [f][x][y][z] -> spectra [f][kz][kx][ky].
 int fft_native_r2c(int N, const float* delta, float2* spec, int nslots, cudaStream_t s) {
   if (nslots <= 0) return 0;
   switch (N) {
@@ -508,20 +622,6 @@ int fft_native_r2c(int N, const float* delta, float2* spec, int nslots, cudaStre
     case 128: return r2c_n<128>(delta, spec, nslots, s);
     case 256: return r2c_n<256>(delta, spec, nslots, s);
     case 512: return r2c_n<512>(delta, spec, nslots, s);
-    default: return -2000;
-  }
-}
-
-// spectra [slot][kz][kx][ky] -> 3 force grids per slot [slot][comp][x][y][z] through the
-// Green multiply; gwork holds [slot][comp][kz][x][y].
-int fft_native_green_c2r(int N, const float2* spec, float2* gwork, float* force, const StepArgs& A,
-                         const int* slot_peak, int nslots, cudaStream_t s) {
-  if (nslots <= 0) return 0;
-  switch (N) {
-    case 64: return green_c2r_n<64>(spec, gwork, force, A, slot_peak, nslots, s);
-    case 128: return green_c2r_n<128>(spec, gwork, force, A, slot_peak, nslots, s);
-    case 256: return green_c2r_n<256>(spec, gwork, force, A, slot_peak, nslots, s);
-    case 512: return green_c2r_n<512>(spec, gwork, force, A, slot_peak, nslots, s);
     default: return -2000;
   }
 }
@@ -538,7 +638,6 @@ int fft_native_c2r(int N, const float2* spec, float2* gwork, float* out, int nfi
   }
 }
 
-namespace {
 // Per-device set-up of the twiddle table, once per device; the lock keeps two host threads that
 // make their first call on one device at the same time from racing on it.
 std::mutex g_init_mu;

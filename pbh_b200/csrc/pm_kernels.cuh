@@ -130,14 +130,13 @@ void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64
 void launch_fixup(const StepArgs& A, long long nst, double* rho64, cudaStream_t s);
 void launch_green(const StepArgs& A, long long nblocks, cudaStream_t s);
 
-// Native real FFT of 256^3 and 512^3 meshes (native_fft.cu).  fft_native_init: once per device
-// before use.
+// The native Poisson solve of 32^3 to 512^3 meshes and plain transforms of 64^3 to 512^3
+// (native_fft.cu).  fft_native_init: once per device before use.
 bool fft_native_size(int N);
+bool fft_solve_size(int N);
 int fft_native_init();
-int fft_native_r2c(int N, const float* delta, float2* spec, int nslots, cudaStream_t s);
-int fft_native_green_c2r(int N, const float2* spec, float2* gwork, float* force, const StepArgs& A,
-                         const int* slot_peak, int nslots, cudaStream_t s);
-int fft_native_c2r(int N, const float2* spec, float2* gwork, float* out, int nfields, cudaStream_t s);
+int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
+                     const int* slot_peak, int nslots, cudaStream_t s);
 
 // Host-requested per-peak operations.  reset: new schedule from a0, status and sort error
 // cleared; set_thr = 1 also sets the collapse threshold and its stop flag (else they are kept).
