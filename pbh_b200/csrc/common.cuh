@@ -65,6 +65,7 @@ struct PeakDesc {
   long long halo_off;      // offset of this peak's halo partials (nst * hc)
   long long mode_base;     // first global mode-block of this peak (Green kernel)
   long long nmodes;        // N*N*(N/2+1)
+  long long nwpart;        // potential-energy partials written from mode_base * (PM_THREADS / 32) on
   u32 nh_magic;            // m / (N/2+1) = (umulhi(m, nh_magic) + m) >> nh_shift for 32-bit m
   int nh_shift;
   float* delta;            // N^3 FP32 density contrast (R2C input)
@@ -98,6 +99,22 @@ struct PeakClock {
   double delta_collapse;  // collapse threshold on max delta (<= 0: not tracked)
   double a_collapse;      // first a whose deposit reached delta_collapse (-1: not yet)
 };
+
+// What the kernels over super-tiles and planes need of a peak's clock, in one 32-byte load: the
+// coefficients of its next push and its flags.  Written with every change of the clock
+// (plan_of in pm_kernels.cu), so that a CTA neither reads the whole clock nor derives the
+// coefficients (a chain of FP64 divisions and roots) itself.
+struct __align__(16) PeakPlan {
+  float kA, kB, D, gscale;  // pending closing kick, opening kick, drift (node units), force scale
+  double a;                 // expansion factor of the positions
+  u32 flags;                // PLAN_*
+  u32 pad;
+};
+#define PLAN_PUSH 1u   // the next push moves this peak (state RUN or FINALIZE)
+#define PLAN_RUN 2u    // with an opening kick and a drift (state RUN)
+#define PLAN_SBUF 4u   // clock.sbuf
+#define PLAN_LGEN 8u   // clock.lgen
+#define PLAN_DEP 16u   // clock.dep
 
 // Per-peak device statistics.  Integer fields are reduced with integer atomics
 // (order-independent); FP64 sums are written per block and reduced in a fixed order.
@@ -141,6 +158,29 @@ __device__ __forceinline__ CSum csum_warp(CSum v) {
     csum_merge(v, o);
   }
   return v;
+}
+
+// Step kernels are launched with programmatic stream serialization, which hides part of a launch's
+// latency: pdl_wait() waits until the kernel before has finished and its writes are visible; every
+// CTA calls it before it touches what other kernels write (also before an early return, so that a
+// kernel's end implies the ends of all before it).  No kernel lets its successor in before its
+// end (griddepcontrol.launch_dependents): the early CTAs pile up on the few SMs that have room
+// while the others still work (at the kernels' start: 64^3 step 62 -> 85 us; near their ends: no
+// gain there and 256^3 1.5 % slower).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... Q>
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, Q&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 #define PM_CHECK(x)                                  \

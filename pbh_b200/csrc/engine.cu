@@ -66,7 +66,8 @@ struct pm_engine {
   PeakClock* d_clocks = nullptr;
   PeakStats* d_stats = nullptr;
   long long* d_st_base = nullptr;
-  unsigned short* d_st_peak = nullptr;  // [super-tile] its peak
+  int2* d_st_ref = nullptr;             // [super-tile] {peak, index in the peak}
+  PeakPlan* d_plan = nullptr;           // digests of the clocks
   long long* d_p_base = nullptr;
   long long* d_mode_base = nullptr;
   long long* d_green_base = nullptr;  // Green blocks of the peaks that k_green serves
@@ -83,6 +84,7 @@ struct pm_engine {
   BinFill* fill[2] = {nullptr, nullptr};       // bin fills of the two buffers
   u32* ovf_n = nullptr;                        // [peak] overflow-area particles
   u32* ovf_in = nullptr;                       // [super-tile] overflowed arrivals
+  u32* new_count = nullptr;                    // [super-tile] count after a relayout
   u32* keys[2] = {nullptr, nullptr};
   u32* vals[2] = {nullptr, nullptr};
   u32* sstart = nullptr;
@@ -90,6 +92,8 @@ struct pm_engine {
   double* wpart = nullptr;   // Green partials of the potential energy (per warp)
   double2* eslice = nullptr; // energy slice partials
   u32* ecount = nullptr;     // energy slices done per peak
+  int eslices = 1;           // energy CTAs per peak
+  double* pushed_a = nullptr;  // expansion factor of each peak's push
   u32* sort_gate = nullptr;  // one word: any peak primes by sort this step
   u32* layout_gate = nullptr;   // one word: any peak primes or relayouts this step
   u32* refresh_gate = nullptr;  // one word: any peak re-sorts its super-tiles this step
@@ -119,7 +123,8 @@ struct pm_engine {
     A.stats = d_stats;
     A.sortseg = sort.seg;
     A.st_base = d_st_base;
-    A.st_peak = d_st_peak;
+    A.st_ref = d_st_ref;
+    A.plan = d_plan;
     A.p_base = d_p_base;
     A.mode_base = d_mode_base;
     A.green_base = d_green_base;
@@ -129,6 +134,8 @@ struct pm_engine {
     A.wpart = wpart;
     A.eslice = eslice;
     A.ecount = ecount;
+    A.eslices = eslices;
+    A.pushed_a = pushed_a;
     A.npeaks = npeaks;
     A.pos0 = bpos[0];
     A.mom0 = bmom[0];
@@ -142,6 +149,7 @@ struct pm_engine {
     A.fill[1] = fill[1];
     A.ovf_n = ovf_n;
     A.ovf_in = ovf_in;
+    A.new_count = new_count;
     A.keys_push = keys[0];
     A.keys_sorted = keys[sort_result];
     A.perm = vals[sort_result];
@@ -211,21 +219,23 @@ struct pm_engine {
     CU(mark());
     launch_push(A, nst, smem_push, stream);
     CU(mark());
-    launch_energy(A, stream);
-    launch_advance(A, stream);
+    launch_tick(A, stream);
     CU(mark());
     int r = 0;
     if (with_sort) {  // only steps that prime a peak: no sort launches at all in the steady state
       if ((r = sort_run<u32>(&sort, keys[0], vals[0], keys[1], vals[1], true, true, stream))) return r;
       launch_st_starts(A, ntot, stream);
     }
-    launch_layout(A, nst, ntot, stream);  // layouts of priming peaks; relayouts (gated, rare)
-    if (with_sort) launch_permute(A, ntot, stream);
+    if (with_sort) {
+      launch_layout(A, stream);
+      launch_permute(A, ntot, stream);
+    }
+    launch_relayout(A, nst, stream);  // gated: only when a push overflowed a bin
     CU(mark());
-    launch_tile_sort(A, nst, stream);
+    if ((flags >> 8) & 0xFF) launch_tile_sort(A, nst, stream);  // only with a refresh period
     CU(mark());
-    launch_deposit(A, nst, smem_dep, nullptr, stream);
-    launch_fixup(A, nst, nullptr, stream);
+    launch_deposit(A, nst, smem_dep, nullptr, -1, stream);
+    launch_fixup(A, nst, nullptr, -1, stream);
     CU(mark());
     if ((r = fft_r2c())) return r;
     CU(mark());
@@ -278,8 +288,8 @@ struct pm_engine {
   }
   int write_clock(int pk, const PeakClock& c) {
     if (c.state == PS_PRIME) prime_pending = true;
-    CU(cudaMemcpyAsync(d_clocks + pk, &c, sizeof(PeakClock), cudaMemcpyHostToDevice, stream));
-    CU(cudaStreamSynchronize(stream));
+    launch_write_clock(args(), pk, c, stream);
+    CU(cudaGetLastError());
     return 0;
   }
 
@@ -308,9 +318,9 @@ struct pm_engine {
       if (sn.done) cudaEventDestroy(sn.done);
     }
     cudaFree(sort_dbg);
-    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_peak, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
-                    wpart, eslice, ecount, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
-                    fill[0], fill[1], ovf_n, ovf_in, keys[0], keys[1], vals[0], vals[1], sstart,
+    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_ref, d_plan, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
+                    wpart, eslice, ecount, pushed_a, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
+                    fill[0], fill[1], ovf_n, ovf_in, new_count, keys[0], keys[1], vals[0], vals[1], sstart,
                     sort_gate, layout_gate, refresh_gate, face, halo};
     for (void* b : bufs) cudaFree(b);
     if (stream) cudaStreamDestroy(stream);
@@ -416,6 +426,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
     P.face_off = fo;
     P.halo_off = ho;
     P.nmodes = (long long)c.N * c.N * (c.N / 2 + 1);
+    P.nwpart = (P.nmodes + PM_THREADS * GREEN_MODES - 1) / (PM_THREADS * GREEN_MODES) * (PM_THREADS / 32);
     pm_div_magic((u32)(c.N / 2 + 1), &P.nh_magic, &P.nh_shift);
     P.mode_base = mb;
     st_base[i] = stb;
@@ -475,7 +486,10 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
       mc.native = true;
       if ((r = E->alloc(&mc.slot_peak, (size_t)B))) return r;
       CU(cudaMemcpy(mc.slot_peak, mc.peaks.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
-      for (int k = 0; k < B; ++k) E->peaks[mc.peaks[k]].native_fft = 1;
+      for (int k = 0; k < B; ++k) {
+        E->peaks[mc.peaks[k]].native_fft = 1;
+        E->peaks[mc.peaks[k]].nwpart = fft_solve_partials((int)N);
+      }
       if ((r = fft_native_init())) return r;
     } else if (E->flags & 4) {
       // Dynamic mode: a plan per batch size, all sharing the largest work area, so a step
@@ -534,6 +548,10 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
       for (auto& p : at) E->peaks[p.first].gtab = E->d_gtab + p.second;
     }
   }
+  for (const PeakDesc& P : E->peaks) {
+    const long long want = (4LL * P.nst + P.nwpart) / (8 * ENERGY_THREADS);
+    E->eslices = std::max(E->eslices, (int)std::min<long long>(want, ENERGY_SLICES));
+  }
   if ((r = E->alloc(&E->d_peaks, npeaks))) return r;
   if ((r = E->alloc(&E->d_clocks, npeaks))) return r;
   if ((r = E->alloc(&E->d_stats, npeaks))) return r;
@@ -568,10 +586,12 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   if ((r = E->alloc(&E->sstart, E->nsst))) return r;
   if ((r = E->alloc(&E->ovf_n, npeaks))) return r;
   if ((r = E->alloc(&E->ovf_in, E->nst))) return r;
+  if ((r = E->alloc(&E->new_count, E->nst))) return r;
   if ((r = E->alloc(&E->epart, 4 * E->nst))) return r;
   if ((r = E->alloc(&E->wpart, E->nmodeblk * (PM_THREADS / 32)))) return r;
   if ((r = E->alloc(&E->eslice, (size_t)npeaks * ENERGY_SLICES * 5))) return r;
   if ((r = E->alloc(&E->ecount, npeaks))) return r;
+  if ((r = E->alloc(&E->pushed_a, npeaks))) return r;
   if ((r = E->alloc(&E->sort_gate, 1))) return r;
   if ((r = E->alloc(&E->layout_gate, 1))) return r;
   if ((r = E->alloc(&E->refresh_gate, 1))) return r;
@@ -580,11 +600,11 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemcpy(E->d_peaks, E->peaks.data(), sizeof(PeakDesc) * npeaks, cudaMemcpyHostToDevice));
   CU(cudaMemcpy(E->d_st_base, st_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   {
-    std::vector<unsigned short> stp((size_t)E->nst);
+    std::vector<int2> ref((size_t)E->nst);
     for (int i = 0; i < npeaks; ++i)
-      for (long long t = st_base[i]; t < st_base[i + 1]; ++t) stp[(size_t)t] = (unsigned short)i;
-    if ((r = E->alloc(&E->d_st_peak, E->nst))) return r;
-    CU(cudaMemcpy(E->d_st_peak, stp.data(), sizeof(unsigned short) * E->nst, cudaMemcpyHostToDevice));
+      for (long long t = st_base[i]; t < st_base[i + 1]; ++t) ref[(size_t)t] = make_int2(i, (int)(t - st_base[i]));
+    if ((r = E->alloc(&E->d_st_ref, E->nst))) return r;
+    CU(cudaMemcpy(E->d_st_ref, ref.data(), sizeof(int2) * E->nst, cudaMemcpyHostToDevice));
   }
   CU(cudaMemcpy(E->d_p_base, p_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(E->d_mode_base, mode_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
@@ -596,6 +616,8 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   }
   CU(cudaMemcpy(E->d_clocks, clocks.data(), sizeof(PeakClock) * npeaks, cudaMemcpyHostToDevice));
   CU(cudaMemset(E->d_stats, 0, sizeof(PeakStats) * npeaks));
+  if ((r = E->alloc(&E->d_plan, npeaks))) return r;
+  CU(cudaMemset(E->d_plan, 0, sizeof(PeakPlan) * npeaks));
   for (int b = 0; b < 2; ++b) {
     CU(cudaMemset(E->bpos[b], 0, sizeof(int4) * E->rtot));
     CU(cudaMemset(E->bmom[b], 0, sizeof(float4) * E->rtot));
@@ -606,6 +628,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemset(E->lmom, 0, sizeof(float4) * E->ntot));
   CU(cudaMemset(E->ovf_n, 0, sizeof(u32) * npeaks));
   CU(cudaMemset(E->ovf_in, 0, sizeof(u32) * E->nst));
+  CU(cudaMemset(E->new_count, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->layout_gate, 0, sizeof(u32)));
   CU(cudaMemset(E->epart, 0, sizeof(double2) * 4 * E->nst));
   CU(cudaMemset(E->wpart, 0, sizeof(double) * E->nmodeblk * (PM_THREADS / 32)));
@@ -830,22 +853,16 @@ int pm_get_counts(pm_engine* e, int peak, double* counts) {
   int r;
   if ((r = e->read_clock(peak, &c))) return r;
   if (!c.has_delta) return -2002;
-  std::vector<PeakClock> all(e->npeaks);
-  CU(cudaMemcpy(all.data(), e->d_clocks, sizeof(PeakClock) * e->npeaks, cudaMemcpyDeviceToHost));
-  std::vector<PeakClock> tmp = all;
-  for (int i = 0; i < e->npeaks; ++i) tmp[i].dep = i == peak ? 1 : 0;
-  CU(cudaMemcpy(e->d_clocks, tmp.data(), sizeof(PeakClock) * e->npeaks, cudaMemcpyHostToDevice));
   PeakStats st;
   CU(cudaMemcpy(&st, e->d_stats + peak, sizeof(PeakStats), cudaMemcpyDeviceToHost));
   st.max_fix = 0;
   st.mass_defect = 0;
   CU(cudaMemcpy(e->d_stats + peak, &st, sizeof(PeakStats), cudaMemcpyHostToDevice));
   // Same kernels with the extra float64 output; delta is rewritten with identical values.
-  launch_deposit(e->args(), e->nst, e->smem_dep, counts, e->stream);
-  launch_fixup(e->args(), e->nst, counts, e->stream);
+  launch_deposit(e->args(), e->nst, e->smem_dep, counts, peak, e->stream);
+  launch_fixup(e->args(), e->nst, counts, peak, e->stream);
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(e->stream));
-  CU(cudaMemcpy(e->d_clocks, all.data(), sizeof(PeakClock) * e->npeaks, cudaMemcpyHostToDevice));
   return 0;
 }
 

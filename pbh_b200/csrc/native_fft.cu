@@ -220,7 +220,7 @@ __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;\n"
 // Whether the peak of an engine slot deposited this step (only then have its density and, after
 // the solve, its forces changed).
 __device__ __forceinline__ bool slot_active(const StepArgs& A, const int* slot_peak, int slot) {
-  return A.clocks[slot_peak[slot]].dep != 0;
+  return (A.plan[slot_peak[slot]].flags & PLAN_DEP) != 0;
 }
 
 // Pass Z forward: fields in[f][x][y][z] -> planes out[f][kz][x][y].  A CTA takes L consecutive
@@ -230,17 +230,18 @@ template <int N>
 __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_z_r2c(const float* __restrict__ in, float2* __restrict__ out,
                                                        StepArgs A, const int* slot_peak) {
   using G = ZGeo<N>;
-  if (slot_peak && !slot_active(A, slot_peak, blockIdx.y)) return;
   __shared__ float2 tw[G::M + 1], tl[16 * G::T];
   __shared__ __align__(16) float2 xb[G::L * G::X];
   load_ztw<false, N>(tw, tl);
+  pdl_wait();
+  if (slot_peak && !slot_active(A, slot_peak, blockIdx.y)) return;
   const int t = threadIdx.x % G::T, l = threadIdx.x / G::T;
   const long long g0 = (long long)blockIdx.x * G::L;  // first line (x N + y) of this CTA
   const int f = blockIdx.y;
   const float2* src = reinterpret_cast<const float2*>(in + (long long)f * G::N3 + (g0 + l) * N);
   float2 v[16], u[16];
 #pragma unroll
-  for (int n1 = 0; n1 < 16; ++n1) v[n1] = __ldg(src + G::T * n1 + t);  // (r[2n], r[2n+1]), n = T n1 + t
+  for (int n1 = 0; n1 < 16; ++n1) v[n1] = __ldcg(src + G::T * n1 + t);  // (r[2n], r[2n+1]), n = T n1 + t
   __syncthreads();  // tables
   float2* row = xb + l * G::X;
   line_fft<false, G::T>(v, u, row, tl, t);
@@ -286,13 +287,14 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_z_c2r(const f
   __shared__ __align__(16) float2 xb[G::TILE];  // the kz-major tile, later the exchange rows
   const long long g0 = (long long)blockIdx.x * G::L;
   const int f = blockIdx.y;
+  load_ztw<true, N>(tw, tl);
+  pdl_wait();
   if (slot_peak && !slot_active(A, slot_peak, f / 3)) return;
   const float2* src = in + (long long)f * G::NH * G::N2 + g0;
   for (int e = threadIdx.x; e < G::NH * G::L / 2; e += G::CTA) {  // two complex values (16 bytes) per copy
     const int k = e / (G::L / 2), ll = 2 * (e - k * (G::L / 2));
     cpa16(xb + k * G::C + ll, src + (long long)k * G::N2 + ll);
   }
-  load_ztw<true, N>(tw, tl);
   const bool zgrad = slot_peak && f % 3 == 2;
   float kf = 0.f;
   const float* gtab = nullptr;
@@ -392,6 +394,7 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_rows(const fl
   __shared__ float2 tl[16 * T];
   __shared__ __align__(16) float2 buf[G::B * G::RS];
   load_ptw<N>(tl);
+  pdl_wait();
   const int rb = blockIdx.x % G::R, pl = blockIdx.x / G::R;
   const int t = threadIdx.x % T, r = threadIdx.x / T;
   const long long o = (long long)pl * G::N2 + (long long)(G::B * rb + r) * N;
@@ -413,6 +416,7 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_cols(float2* 
   __shared__ float2 tl[16 * T];
   __shared__ __align__(16) float2 buf[16 * T * B];
   load_ptw<N>(tl);
+  pdl_wait();
   const int cb = blockIdx.x % G::R, pl = blockIdx.x / G::R;
   const int j = threadIdx.x % B, t = threadIdx.x / B;
   float2* plane = io + (long long)pl * G::N2 + B * cb + j;
@@ -442,8 +446,9 @@ __global__ void __launch_bounds__(cta<N>(), 768 / cta<N>())
   float2* const tl = buf + 16 * T * B + 16 * G::CTA;
   const int idx = blockIdx.x % R, pl = gridDim.x / R - 1 - blockIdx.x / R;
   const int slot = pl / G::NH, kz = pl - slot * G::NH, pk = slot_peak[slot];
-  if (!A.clocks[pk].dep) return;
   load_ptw<N>(tl);
+  pdl_wait();
+  if (!(A.plan[pk].flags & PLAN_DEP)) return;
   const int tid = threadIdx.x, j = tid % B, t = tid / B, ky = B * idx + j;
   float2* const col = spec + (long long)pl * G::N2 + ky;
   float2 v[16], u[16];
@@ -514,8 +519,9 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>())
   __shared__ __align__(16) float2 buf[G::B * G::RS];
   const int comp = blockIdx.x % 3, q = blockIdx.x / 3, rb = q % R, pl = q / R;
   const int slot = pl / G::NH, kz = pl - slot * G::NH, pk = slot_peak[slot];
-  if (!A.clocks[pk].dep) return;
   load_ptw<N>(tl);
+  pdl_wait();
+  if (!(A.plan[pk].flags & PLAN_DEP)) return;
   const int t = threadIdx.x % T, r = threadIdx.x / T, o = (B * rb + r) * N;
   float2* const dst = gspec + ((long long)(3 * slot + comp) * G::NH + kz) * G::N2 + o;
   const float2* const src = comp == 0 ? dst : spec + (long long)pl * G::N2 + o;
@@ -540,9 +546,9 @@ int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
   using Z = ZGeo<N>;
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
-  k_fft_z_r2c<N><<<dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s>>>(x, spec, StepArgs{}, nullptr);
-  k_fft_rows<N, false><<<blocks, G::CTA, 0, s>>>(spec, spec);
-  k_fft_cols<N, false><<<blocks, G::CTA, 0, s>>>(spec);
+  pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s, x, spec, StepArgs{}, nullptr);
+  pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
+  pdl_launch(k_fft_cols<N, false>, dim3(blocks), G::CTA, 0, s, spec);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -553,11 +559,11 @@ int solve_n(const float* delta, float2* spec, float2* gspec, float* force, const
   using Z = ZGeo<N>;
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nslots * G::NH);
-  k_fft_z_r2c<N><<<dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s>>>(delta, spec, A, slot_peak);
-  k_fft_rows<N, false><<<blocks, G::CTA, 0, s>>>(spec, spec);
-  k_solve_cols<N><<<blocks, G::CTA, G::COLS_SMEM, s>>>(spec, gspec, A, slot_peak);
-  k_solve_rows<N><<<3 * blocks, G::CTA, 0, s>>>(spec, gspec, A, slot_peak);
-  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s>>>(gspec, force, A, slot_peak);
+  pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s, delta, spec, A, slot_peak);
+  pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
+  pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
+  pdl_launch(k_solve_rows<N>, dim3(3 * blocks), G::CTA, 0, s, spec, gspec, A, slot_peak);
+  pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s, gspec, force, A, slot_peak);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -567,9 +573,9 @@ int c2r_n(const float2* spec, float2* work, float* out, int nfields, cudaStream_
   using Z = ZGeo<N>;
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
-  k_fft_rows<N, true><<<blocks, G::CTA, 0, s>>>(spec, work);
-  k_fft_cols<N, true><<<blocks, G::CTA, 0, s>>>(work);
-  k_fft_z_c2r<N><<<dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s>>>(work, out, StepArgs{}, nullptr);
+  pdl_launch(k_fft_rows<N, true>, dim3(blocks), G::CTA, 0, s, spec, work);
+  pdl_launch(k_fft_cols<N, true>, dim3(blocks), G::CTA, 0, s, work);
+  pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s, work, out, StepArgs{}, nullptr);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -578,6 +584,8 @@ int c2r_n(const float2* spec, float2* work, float* out, int nfields, cudaStream_
 
 bool fft_native_size(int N) { return N == 64 || N == 128 || N == 256 || N == 512; }
 bool fft_solve_size(int N) { return N == 32 || fft_native_size(N); }
+// Potential-energy partials of a solve: one per warp of k_solve_cols, N / 16 threads per column.
+long long fft_solve_partials(int N) { return (long long)(N / 2 + 1) * N * (N / 16) / 32; }
 
 // Per-device set-up: the twiddle table and the shared-memory limits.  Call with the device current.
 int fft_native_init() {

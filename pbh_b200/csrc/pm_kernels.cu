@@ -7,11 +7,6 @@
 
 #include "pm_kernels.cuh"
 
-// Sweeps of particle positions a deposit thread keeps in flight (loads issued ahead of use).
-#ifndef PM_DEP_DEPTH
-#define PM_DEP_DEPTH 1
-#endif
-
 namespace {
 
 constexpr double kTwoPi = 6.283185307179586476925286766559;
@@ -31,6 +26,12 @@ __device__ __forceinline__ void cp_async4(unsigned dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Asks L2 for `n` 16-byte elements from p on (one thread; nothing waits for it).
+__device__ __forceinline__ void prefetch_l2(const void* p, int n) {
+  if (n > 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(n * 16) : "memory");
+}
 
 __device__ __forceinline__ u32 lanemask_lt() {
   u32 m;
@@ -74,15 +75,41 @@ __device__ __forceinline__ u32 bin_count(const BinLayout& L, const BinFill& F) {
 
 // Locate the peak and the peak-local index of this CTA (uniform across the block).
 struct TileRef {
-  int pk;
-  long long t;
+  int pk, t;
 };
 
-__device__ __forceinline__ TileRef find_tile(const long long* base, const unsigned short* st_peak) {
-  TileRef r;
-  r.pk = st_peak[blockIdx.x];  // the same for every thread of the CTA
-  r.t = (long long)blockIdx.x - base[r.pk];
-  return r;
+__device__ __forceinline__ TileRef find_tile(const int2* st_ref) {
+  const int2 v = __ldg(st_ref + blockIdx.x);  // the same for every thread of the CTA
+  return TileRef{v.x, v.y};
+}
+
+// The digest of a clock (see PeakPlan).
+__device__ __forceinline__ PeakPlan plan_of(const PeakClock& c, const PeakDesc& P) {
+  PeakPlan p{};
+  const bool run = c.state == PS_RUN, push = run || c.state == PS_FINALIZE;
+  p.flags = (push ? PLAN_PUSH : 0u) | (run ? PLAN_RUN : 0u) | (c.sbuf ? PLAN_SBUF : 0u) | (c.lgen ? PLAN_LGEN : 0u) |
+            (c.dep ? PLAN_DEP : 0u);
+  p.a = c.a;
+  if (push) {
+    // H(a) = H_I a^(-3/2): the kick 0.5 da / (a H) and the drift da / (a^3 H) at the middle
+    // (pm3d.py:122-124).
+    const double a = c.a, da = c.da, amid = a + 0.5 * da;
+    p.kA = (float)c.kpend;
+    p.kB = run ? (float)(0.5 / PM_H_I * da * sqrt(a)) : 0.f;
+    p.D = run ? (float)(da / (PM_H_I * amid * sqrt(amid) * P.dx)) : 0.f;
+    p.gscale = c.a_grid == a ? 1.0f : (float)(c.a_grid / a);
+  }
+  return p;
+}
+__device__ __forceinline__ PeakPlan load_plan(const StepArgs& A, int pk) {
+  union {
+    int4 v[2];
+    PeakPlan p;
+  } u;
+  const int4* src = reinterpret_cast<const int4*>(A.plan + pk);
+  u.v[0] = __ldcg(src);
+  u.v[1] = __ldcg(src + 1);
+  return u.p;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -95,194 +122,51 @@ __device__ __forceinline__ TileRef find_tile(const long long* base, const unsign
 // the destination's `moved` count, placed after the destination's count before the step (which
 // no stayer rank reaches).  An arrival that finds no room, which the spare capacity makes rare,
 // goes to the peak's overflow area and the peak relayouts this step.
-struct PushCoef {
-  float kA, kB, D, gscale;
-  int run;
-};
-
-// Where one push CTA reads and writes.
-struct PushCtx {
-  int sx, sy, sz;        // this super-tile
-  long long gS;          // its global index
-  u32 base, cap;         // its bin
-  const BinLayout* lay;  // bin layouts (global super-tile index)
-  const BinFill* fcur;   // fills of the buffer read
-  BinFill* fnxt;         // fills of the buffer written
-  int4* opos;            // the buffer written
-  float4* omom;
-};
-
-template <int T>
-__device__ __forceinline__ void push_one(const StepArgs& A, const PeakDesc& P, int pk, const float* __restrict__ s_f,
-                                         const PushCoef& K, const PushCtx& X, int4 ps, float4 m, u32* s_stay,
-                                         bool& bad, bool& lost, double4& acc_e) {
-  constexpr int RS = patch_rs(T), PS = patch_ps(T), CS = patch_size(T);
-  const int N = P.N, l2 = P.log2N;
-  const int ix = (ps.x >> (2 * l2)) & (N - 1), iy = (ps.x >> l2) & (N - 1), iz = ps.x & (N - 1);
-  const int lx = ix - X.sx * T, ly = iy - X.sy * T, lz = iz - X.sz * T;
-  // A particle outside this super-tile (bins and state disagree) is flagged and moved on
-  // unchanged to the bin its cell names; nothing indexes outside the patch.
-  const bool inside = ps.x >= 0 && ps.x < N * N * N && (unsigned)lx < (unsigned)T && (unsigned)ly < (unsigned)T &&
-                      (unsigned)lz < (unsigned)T;
-  bad |= !inside;
-  float fx = __int_as_float(ps.y), fy = __int_as_float(ps.z), fz = __int_as_float(ps.w);
-  float ax = 0.f, ay = 0.f, az = 0.f;
-  if (inside) {
-    const float gx = 1.0f - fx, gy = 1.0f - fy, gz = 1.0f - fz;
-    const int o = lx * PS + ly * RS + lz;
-#define PM_CORNER(w, d)                       \
-  {                                           \
-    const float w_ = (w);                     \
-    ax = fmaf(w_, s_f[o + (d)], ax);          \
-    ay = fmaf(w_, s_f[CS + o + (d)], ay);     \
-    az = fmaf(w_, s_f[2 * CS + o + (d)], az); \
+// Where a particle that leaves its super-tile goes: a slot of the bin of its new cell's super-tile
+// (after that bin's count before the step, which no stayer rank reaches), else the peak's
+// overflow area; returns false when even that is full (the bins were corrupted).
+template <int T, int SB>
+__device__ __forceinline__ bool push_move(const StepArgs& A, const PeakDesc& P, int pk, const BinLayout* lay, int4 np,
+                                          float4 nm) {
+  const int l2 = P.log2N, m = P.N - 1;
+  constexpr int s = T == 4 ? 2 : T == 8 ? 3 : 4;
+  const long long gD =
+      P.st_base + pm_morton3((u32)(np.x >> (2 * l2)) >> s, (u32)((np.x >> l2) & m) >> s, (u32)(np.x & m) >> s);
+  const BinLayout L = lay[gD];
+  const u32 cnt = bin_count(L, A.fill[SB][gD]);
+  const u32 r = atomicAdd(&A.fill[SB ^ 1][gD].moved, 1u);
+  if (r < L.cap - cnt) {
+    const u32 dst = L.base + cnt + r;
+    (SB ? A.pos0 : A.pos1)[dst] = np;
+    (SB ? A.mom0 : A.mom1)[dst] = nm;
+    return true;
   }
-    const float w00 = gx * gy, w01 = gx * fy, w10 = fx * gy, w11 = fx * fy;
-    PM_CORNER(w00 * gz, 0)
-    PM_CORNER(w00 * fz, 1)
-    PM_CORNER(w01 * gz, RS)
-    PM_CORNER(w01 * fz, RS + 1)
-    PM_CORNER(w10 * gz, PS)
-    PM_CORNER(w10 * fz, PS + 1)
-    PM_CORNER(w11 * gz, PS + RS)
-    PM_CORNER(w11 * fz, PS + RS + 1)
-#undef PM_CORNER
-    ax *= K.gscale;
-    ay *= K.gscale;
-    az *= K.gscale;
-  }
-  float px = m.x + K.kA * ax, py = m.y + K.kA * ay, pz = m.z + K.kA * az;
-  // Momentum synchronised with the positions (after the closing kick): energy and momentum sums.
-  {
-    double4 t = acc_e;
-    const double dx = px, dy = py, dz = pz;
-    t.x += dx;
-    t.y += dy;
-    t.z += dz;
-    t.w += dx * dx + dy * dy + dz * dz;
-    acc_e = t;
-  }
-  int nx = ix, ny = iy, nz = iz;
-  const bool finite = isfinite(px) && isfinite(py) && isfinite(pz);
-  if (K.run && finite && inside) {  // a non-finite particle stays where it is (the peak is flagged below)
-    px += K.kB * ax;
-    py += K.kB * ay;
-    pz += K.kB * az;
-#define PM_DRIFT(f, p, i)       \
-  {                             \
-    float fn = f + K.D * p;     \
-    float c = floorf(fn);       \
-    fn -= c;                    \
-    if (fn >= 1.0f) {           \
-      fn -= 1.0f;               \
-      c += 1.0f;                \
-    }                           \
-    f = fn;                     \
-    i = (i + (int)c) & (N - 1); \
-  }
-    PM_DRIFT(fx, px, nx)
-    PM_DRIFT(fy, py, ny)
-    PM_DRIFT(fz, pz, nz)
-#undef PM_DRIFT
-  }
-  bad |= !(finite && isfinite(px) && isfinite(py) && isfinite(pz));
-  const int cell = (nx << (2 * l2)) | (ny << l2) | nz;
-  const int4 np = make_int4(cell, __float_as_int(fx), __float_as_int(fy), __float_as_int(fz));
-  const float4 nm = make_float4(px, py, pz, m.w);
-  const int tx = nx >> P.log2TS, ty = ny >> P.log2TS, tz = nz >> P.log2TS;
-  const bool stay = tx == X.sx && ty == X.sy && tz == X.sz;
-  const u32 sm = __ballot_sync(__activemask(), stay);
-  long long dst = -1, gD = X.gS;
-  if (stay) {
-    const int leader = __ffs(sm) - 1;
-    u32 r0 = 0;
-    if ((int)(threadIdx.x & 31) == leader) r0 = atomicAdd(s_stay, (u32)__popc(sm));
-    r0 = __shfl_sync(sm, r0, leader);
-    const u32 r = r0 + (u32)__popc(sm & lanemask_lt());
-    if (r < X.cap) dst = (long long)X.base + r;  // always: the stayers are at most the bin's count
-  } else {
-    gD = P.st_base + pm_morton3(tx, ty, tz);
-    const BinLayout L = X.lay[gD];
-    const u32 cnt = bin_count(L, X.fcur[gD]);
-    const u32 r = atomicAdd(&X.fnxt[gD].moved, 1u);
-    if (r < L.cap - cnt) dst = (long long)L.base + cnt + r;
-  }
-  if (dst >= 0) {
-    X.opos[dst] = np;
-    X.omom[dst] = nm;
-  } else {
-    const u32 o = atomicAdd(&A.ovf_n[pk], 1u);
-    if (o < (u32)P.n) {
-      A.lpos[P.p_off + o] = np;
-      A.lmom[P.p_off + o] = nm;
-      atomicAdd(&A.ovf_in[gD], 1u);
-    } else {
-      lost = true;  // more overflows than particles: the bins were corrupted
-    }
-  }
+  const u32 o = atomicAdd(&A.ovf_n[pk], 1u);
+  if (o >= (u32)P.n) return false;
+  A.lpos[P.p_off + o] = np;
+  A.lmom[P.p_off + o] = nm;
+  atomicAdd(&A.ovf_in[gD], 1u);
+  return true;
 }
 
-template <int T>
-__device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P, const PeakClock& C, int pk, u32 st,
-                                           float* s_f, u32* s_stay, const PushCoef& K) {
+// SB: the bin buffer read (its arrays are then kernel parameters, not per-thread selects).
+template <int T, int SB>
+__device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P, int pk, u32 st, float* s_f, u32* s_stay,
+                                           const PeakPlan& K, const BinLayout& L, const BinFill& F) {
   constexpr int T1 = T + 1, RS = patch_rs(T), PS = patch_ps(T), CS = patch_size(T);
   constexpr int CH = T / 4 + 1;  // per patch row: T/4 copies of 16 bytes, then the (wrapped) last node
-  const int N = P.N;
-  PushCtx X;
-  X.sx = pm_compact3(st >> 2);
-  X.sy = pm_compact3(st >> 1);
-  X.sz = pm_compact3(st);
-  X.gS = P.st_base + st;
-  X.lay = blay(A, C.lgen);
-  X.fcur = bfill(A, C.sbuf);
-  X.fnxt = bfill(A, C.sbuf ^ 1);
-  X.opos = bpos(A, C.sbuf ^ 1);
-  X.omom = bmom(A, C.sbuf ^ 1);
-  const BinLayout L = X.lay[X.gS];
-  X.base = L.base;
-  X.cap = L.cap;
-  const BinRuns R = bin_runs(L, X.fcur[X.gS]);
+  const int N = P.N, l2 = P.log2N;
+  const int sx = pm_compact3(st >> 2), sy = pm_compact3(st >> 1), sz = pm_compact3(st);
+  const long long gS = P.st_base + st;
+  const BinLayout* const lay = blay(A, K.flags & PLAN_LGEN);
+  const BinRuns R = bin_runs(L, F);
   const int n = R.total();
   const long long N3 = (long long)N * N * N;
-  if (n > 0) {
-    // Asynchronous copies of the patch rows (every row start is 16-byte aligned on both sides:
-    // z0 = sz*T is a multiple of 4 and the grids are 256-byte aligned).
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(s_f);
-    const int z0 = X.sz * T, zl = (X.sz * T + T) & (N - 1);
-    // Thread t copies piece t % CH of patch rows t / CH, t / CH + RSTEP, ... (the row number
-    // advanced incrementally: RSTEP rows are DX planes and DY rows further on).
-    constexpr int NTH = PUSH_THREADS - PUSH_THREADS % CH, RSTEP = NTH / CH, DX = RSTEP / T1, DY = RSTEP % T1;
-    if (threadIdx.x < NTH) {
-      const int part = threadIdx.x % CH, r0 = threadIdx.x / CH;
-      int comp = r0 / (T1 * T1), lx = (r0 / T1) % T1, ly = r0 % T1;
-      for (int row = r0; row < 3 * T1 * T1; row += RSTEP) {
-        const int gx = (X.sx * T + lx) & (N - 1), gy = (X.sy * T + ly) & (N - 1);
-        const float* src = P.force + comp * N3 + ((long long)gx * N + gy) * N;
-        const unsigned dst = sbase + 4u * (unsigned)(comp * CS + lx * PS + ly * RS + part * 4);
-        if (part < T / 4) cp_async16(dst, src + z0 + part * 4);
-        else cp_async4(dst, src + zl);
-        ly += DY;
-        if (ly >= T1) {
-          ly -= T1;
-          ++lx;
-        }
-        lx += DX;
-        while (lx >= T1) {
-          lx -= T1;
-          ++comp;
-        }
-      }
-    }
-    cp_async_wait_all();
-  }
-  __syncthreads();
-  bool bad = false, lost = false;
-  double4 acc_e = make_double4(0.0, 0.0, 0.0, 0.0);  // this thread's momentum and p^2 sums
-  // One particle per thread per sweep, the next two sweeps' particles in flight meanwhile;
-  // 32-bit indices inside the bin's two runs: particle k sits at [k] in the first run, at
-  // [k + d1] in the second.
-  const int4* __restrict__ pp = bpos(A, C.sbuf) + R.b0;
-  const float4* __restrict__ mp = bmom(A, C.sbuf) + R.b0;
+  // One particle per thread per sweep, the next two sweeps' particles in flight meanwhile (the
+  // first two already while the patch is staged); 32-bit indices inside the bin's two runs:
+  // particle k sits at [k] in the first run, at [k + d1] in the second.
+  const int4* __restrict__ pp = (SB ? A.pos1 : A.pos0) + R.b0;
+  const float4* __restrict__ mp = (SB ? A.mom1 : A.mom0) + R.b0;
   const int n0 = R.n0, d1 = (int)(R.b1 - R.b0);
   int k = threadIdx.x;
   int4 pa = make_int4(0, 0, 0, 0), pb = pa;
@@ -297,9 +181,48 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
     pb = pp[j];
     mb = mp[j];
   }
-  for (; k < n; k += PUSH_THREADS) {
-    const int4 p0 = pa;
-    const float4 m0 = ma;
+  if (n > 0) {
+    // Asynchronous copies of the patch rows (every row start is 16-byte aligned on both sides:
+    // z0 = sz*T is a multiple of 4 and the grids are 256-byte aligned).
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(s_f);
+    const int z0 = sz * T, zl = (sz * T + T) & (N - 1);
+    // Thread t copies piece t % CH of the patch rows t / CH, t / CH + RSTEP, ..., of all three grids
+    // at once (one address computation for three copies).
+    constexpr int NTH = PUSH_THREADS - PUSH_THREADS % CH, RSTEP = NTH / CH;
+    if (threadIdx.x < NTH) {
+      const int part = threadIdx.x % CH;
+      const float *f0 = P.force + (part < T / 4 ? z0 + 4 * part : zl), *f1 = f0 + N3, *f2 = f1 + N3;
+      const unsigned d0 = sbase + 16u * (unsigned)part;
+      for (int row = threadIdx.x / CH; row < T1 * T1; row += RSTEP) {
+        const int lx = row / T1, ly = row - lx * T1;
+        const u32 off = ((u32)((sx * T + lx) & (N - 1)) << (2 * l2)) + ((u32)((sy * T + ly) & (N - 1)) << l2);
+        const unsigned dst = d0 + 4u * (unsigned)(lx * PS + ly * RS);
+        if (part < T / 4) {
+          cp_async16(dst, f0 + off);
+          cp_async16(dst + 4u * CS, f1 + off);
+          cp_async16(dst + 8u * CS, f2 + off);
+        } else {
+          cp_async4(dst, f0 + off);
+          cp_async4(dst + 4u * CS, f1 + off);
+          cp_async4(dst + 8u * CS, f2 + off);
+        }
+      }
+    }
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  // A cell index belongs to this super-tile iff its bits outside the local ones equal the
+  // super-tile's: one mask and one compare (negative or out-of-mesh values never match).
+  const int local = ((T - 1) << (2 * l2)) | ((T - 1) << l2) | (T - 1);
+  const int tile_bits = ((sx * T) << (2 * l2)) | ((sy * T) << l2) | (sz * T);
+  const int mz = N - 1, my = mz << l2, mx = my << l2;  // the fields of a cell index
+  const u32 lt = lanemask_lt();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool bad = false, lost = false;
+  double ex = 0.0, ey = 0.0, ez = 0.0, ep = 0.0;  // this thread's momentum and p^2 sums
+  for (; k - lane < n; k += PUSH_THREADS) {  // uniform across a warp, so that its votes see all lanes
+    int4 ps = pa;
+    float4 m = ma;
     pa = pb;
     ma = mb;
     const int k2 = k + 2 * PUSH_THREADS;
@@ -308,288 +231,161 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
       pb = pp[j];
       mb = mp[j];
     }
-    push_one<T>(A, P, pk, s_f, K, X, p0, m0, s_stay, bad, lost, acc_e);
+    const bool valid = k < n;
+    const int c = ps.x;
+    // A particle outside this super-tile (bins and state disagree) is flagged and moved on
+    // unchanged to the bin its cell names; nothing indexes outside the patch.
+    const bool inside = (c & ~local) == tile_bits;
+    bool stay = valid && inside;
+    if (stay) {
+      const float fx = __int_as_float(ps.y), fy = __int_as_float(ps.z), fz = __int_as_float(ps.w);
+      const float gx = 1.0f - fx, gy = 1.0f - fy, gz = 1.0f - fz;
+      const int o = ((c >> (2 * l2)) & (T - 1)) * PS + ((c >> l2) & (T - 1)) * RS + (c & (T - 1));
+      float ax = 0.f, ay = 0.f, az = 0.f;
+#define PM_CORNER(w, d)                       \
+  {                                           \
+    const float w_ = (w);                     \
+    ax = fmaf(w_, s_f[o + (d)], ax);          \
+    ay = fmaf(w_, s_f[CS + o + (d)], ay);     \
+    az = fmaf(w_, s_f[2 * CS + o + (d)], az); \
   }
-  const bool any_bad = __syncthreads_or(bad), any_lost = __syncthreads_or(lost);
-  if (threadIdx.x == 0) {
-    if (any_bad) atomicOr(&A.stats[pk].status, 1u);
-    if (any_lost) atomicOr(&A.stats[pk].status, 4u);
-    // This bin's fill in the buffer written: its stayers, and where its arrivals start.
-    X.fnxt[X.gS].stay = *s_stay;
-    X.fnxt[X.gS].gap = (u32)n;
+      const float w00 = gx * gy, w01 = gx * fy, w10 = fx * gy, w11 = fx * fy;
+      PM_CORNER(w00 * gz, 0)
+      PM_CORNER(w00 * fz, 1)
+      PM_CORNER(w01 * gz, RS)
+      PM_CORNER(w01 * fz, RS + 1)
+      PM_CORNER(w10 * gz, PS)
+      PM_CORNER(w10 * fz, PS + 1)
+      PM_CORNER(w11 * gz, PS + RS)
+      PM_CORNER(w11 * fz, PS + RS + 1)
+#undef PM_CORNER
+      ax *= K.gscale;
+      ay *= K.gscale;
+      az *= K.gscale;
+      float px = m.x + K.kA * ax, py = m.y + K.kA * ay, pz = m.z + K.kA * az;
+      // Momentum synchronised with the positions (after the closing kick): energy and momentum sums.
+      {
+        const double dx = px, dy = py, dz = pz;
+        ex += dx;
+        ey += dy;
+        ez += dz;
+        ep += dx * dx + dy * dy + dz * dz;
+      }
+      const bool finite = fabsf(px) < INFINITY && fabsf(py) < INFINITY && fabsf(pz) < INFINITY;
+      if ((K.flags & PLAN_RUN) && finite) {  // a non-finite particle stays where it is (the peak is flagged)
+        px += K.kB * ax;
+        py += K.kB * ay;
+        pz += K.kB * az;
+        int cx, cy, cz;  // cells crossed
+#define PM_DRIFT(f, p, i, out)    \
+  {                               \
+    float fn = f + K.D * p;       \
+    float fl = floorf(fn);        \
+    fn -= fl;                     \
+    if (fn >= 1.0f) {             \
+      fn -= 1.0f;                 \
+      fl += 1.0f;                 \
+    }                             \
+    out = __float_as_int(fn);     \
+    i = (int)fl;                  \
+  }
+        PM_DRIFT(fx, px, cx, ps.y)
+        PM_DRIFT(fy, py, cy, ps.z)
+        PM_DRIFT(fz, pz, cz, ps.w)
+#undef PM_DRIFT
+        // Each field of the cell index advanced modulo N in place (carries fall outside its mask).
+        ps.x = ((c + (int)((u32)cx << (2 * l2))) & mx) | ((c + (int)((u32)cy << l2)) & my) | ((c + cz) & mz);
+        stay = (ps.x & ~local) == tile_bits;
+        bad |= !(fabsf(px) < INFINITY && fabsf(py) < INFINITY && fabsf(pz) < INFINITY);
+      }
+      bad |= !finite;
+      m.x = px;
+      m.y = py;
+      m.z = pz;
+    }
+    const u32 sm = __ballot_sync(0xffffffffu, stay);
+    u32 r = 0;
+    if (lane == 0) r = atomicAdd(s_stay, (u32)__popc(sm));
+    r = L.base + __shfl_sync(0xffffffffu, r, 0) + (u32)__popc(sm & lt);
+    if (stay) {
+      if (r < L.base + L.cap) {  // always: the stayers are at most the bin's count
+        (SB ? A.pos0 : A.pos1)[r] = ps;
+        (SB ? A.mom0 : A.mom1)[r] = m;
+      } else {
+        lost = true;
+      }
+    } else if (valid) {
+      bad |= !inside;
+      if (!inside && !(c >= 0 && c < N3)) ps.x = tile_bits;  // a cell outside the mesh names no bin: this one
+      lost |= !push_move<T, SB>(A, P, pk, lay, ps, m);
+    }
   }
   // Super-tile partials of the momentum and p^2 sums, in a fixed order: a plain FP64 tree over
   // the 32 lanes of a warp (about 5e-16 of the sum of magnitudes; compensating it cost 4 % of the
-  // push), then compensated merges across the warps here and across super-tiles in k_energy.
-  __shared__ CSum s_e[PUSH_THREADS / 32][4];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double4 ev = acc_e;
-  const double ea[4] = {ev.x, ev.y, ev.z, ev.w};
+  // push), then compensated merges across the warps here and across super-tiles in k_tick.
+  __shared__ double s_e[PUSH_THREADS / 32][4];
+  const double ea[4] = {ex, ey, ez, ep};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     double v = ea[q];
     for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-    if (lane == 0) s_e[warp][q] = CSum{v, 0.0};
+    if (lane == 0) s_e[warp][q] = v;
   }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&A.stats[pk].status, 1u);
+  if (__any_sync(0xffffffffu, lost) && lane == 0) atomicOr(&A.stats[pk].status, 4u);
   __syncthreads();
-  if (threadIdx.x < 4) {
-    CSum t = s_e[0][threadIdx.x];
-    for (int w = 1; w < PUSH_THREADS / 32; ++w) csum_merge(t, s_e[w][threadIdx.x]);
-    A.epart[(P.st_base + st) * 4 + threadIdx.x] = make_double2(t.s, t.c);
+  if (threadIdx.x == PUSH_THREADS - 1) {
+    // This bin's fill in the buffer written: its stayers, and where its arrivals start.
+    A.fill[SB ^ 1][gS].stay = *s_stay;
+    A.fill[SB ^ 1][gS].gap = (u32)n;
+  }
+  if (warp < 4) {  // one warp per sum
+    static_assert(PUSH_THREADS <= 1024, "one lane per warp of the CTA");
+    CSum t = csum_warp(CSum{lane < PUSH_THREADS / 32 ? s_e[lane][warp] : 0.0, 0.0});
+    if (lane == 0) A.epart[gS * 4 + warp] = make_double2(t.s, t.c);
   }
 }
 
-__global__ void __launch_bounds__(PUSH_THREADS, 2) k_push(StepArgs A) {
+__global__ void __launch_bounds__(PUSH_THREADS, 2) k_push(const __grid_constant__ StepArgs A) {
   extern __shared__ __align__(16) float s_f[];
-  __shared__ PushCoef s_k;
   __shared__ u32 s_stay;
-  const TileRef tr = find_tile(A.st_base, A.st_peak);
-  const PeakClock C = A.clocks[tr.pk];
-  if (C.state != PS_RUN && C.state != PS_FINALIZE) return;
+  // A CTA's work is a chain of memory round trips (its tile, its peak and bin, then its particles
+  // and force patch): as few as possible, because only two CTAs share an SM to hide them.  Both
+  // candidates of the bin's layout and fill are fetched beside the plan that selects them.
+  const TileRef tr = find_tile(A.st_ref);
+  if (threadIdx.x == 0) s_stay = 0u;
+  pdl_wait();
+  const PeakPlan K = load_plan(A, tr.pk);
+  const int4 F0 = __ldcg(reinterpret_cast<const int4*>(A.fill[0] + blockIdx.x)),
+             F1 = __ldcg(reinterpret_cast<const int4*>(A.fill[1] + blockIdx.x));
+  const int2 L0 = __ldcg(reinterpret_cast<const int2*>(A.lay[0] + blockIdx.x)),
+             L1 = __ldcg(reinterpret_cast<const int2*>(A.lay[1] + blockIdx.x));
   const PeakDesc P = A.peaks[tr.pk];
-  if (threadIdx.x == 0) {
-    const double a = C.a, da = C.da;
-    const bool run = C.state == PS_RUN;
-    const double amid = a + 0.5 * da;
-    s_k.kA = (float)C.kpend;
-    s_k.kB = run ? (float)(0.5 * da / (a * pm_hubble(a))) : 0.f;
-    s_k.D = run ? (float)(da / (amid * amid * amid * pm_hubble(amid)) / P.dx) : 0.f;
-    s_k.gscale = (float)(C.a_grid / a);
-    s_k.run = run ? 1 : 0;
-    s_stay = 0u;
-  }
-  __syncthreads();
-  const PushCoef K = s_k;
+  const int4 f = K.flags & PLAN_SBUF ? F1 : F0;
+  const int2 l = K.flags & PLAN_LGEN ? L1 : L0;
+  const BinFill F{(u32)f.x, (u32)f.y, (u32)f.z, 0u};
+  const BinLayout L{(u32)l.x, (u32)l.y};
+  if (threadIdx.x == 0 && tr.t == 0) A.pushed_a[tr.pk] = K.flags & PLAN_PUSH ? K.a : -1.0;
+  if (!(K.flags & PLAN_PUSH)) return;
   const u32 st = (u32)tr.t;
+  const bool sb = K.flags & PLAN_SBUF;
   switch (P.TS) {
-    case 4: push_super<4>(A, P, C, tr.pk, st, s_f, &s_stay, K); break;
-    case 8: push_super<8>(A, P, C, tr.pk, st, s_f, &s_stay, K); break;
-    default: push_super<16>(A, P, C, tr.pk, st, s_f, &s_stay, K); break;
+    case 4:
+      if (sb) push_super<4, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<4, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      break;
+    case 8:
+      if (sb) push_super<8, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<8, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      break;
+    default:
+      if (sb) push_super<16, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<16, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      break;
   }
 }
 
-// Clock advance (one thread per peak): applies the step that the push kernel just made,
-// selects the next step size, whether this step primes by sort, relayouts (the push overflowed
-// a bin) or re-sorts the super-tiles by cell, and which peaks re-deposit.  A running peak's
-// particles are now in the other bin buffer; one that relayouts switches to a new layout
-// generation, which the layout kernel fills in.
-__global__ void k_advance(StepArgs A) {
-  int any_sort = 0, any_layout = 0, any_refresh = 0;
-  for (int pk = threadIdx.x; pk < A.npeaks; pk += blockDim.x) {
-    PeakClock c = A.clocks[pk];
-    const PeakDesc P = A.peaks[pk];
-    int dep = 0;
-    // Collapse detection on the deposit made by the previous step, i.e. of the positions at c.a.
-    // This step's push has already moved a running peak on to c.a + c.da, so a stop takes
-    // effect after the step is booked below: the next step applies its closing kick and ends.
-    bool stop_now = false;
-    if (c.has_delta && c.delta_collapse > 0 && c.a_collapse < 0 && c.state != PS_PRIME) {
-      const double dmax = (double)A.stats[pk].max_fix / (double)PM_FIX_ONE / P.n_mean - 1.0;
-      if (dmax >= c.delta_collapse) {
-        c.a_collapse = c.a;
-        stop_now = c.stop_on_collapse && c.state == PS_RUN;
-      }
-    }
-    const bool pushed = c.state == PS_RUN || c.state == PS_FINALIZE;
-    const int ovf = pushed && A.ovf_n[pk] != 0u ? 1 : 0;
-    switch (c.state) {
-      case PS_PRIME:
-        dep = 1;
-        c.sortstep = 1;
-        c.relayout = 0;
-        c.refresh = 0;
-        c.lgen ^= 1;
-        c.kpend = 0.0;
-        c.a_grid = c.a;
-        c.has_delta = 1;
-        c.state = c.mode == SCHED_EXPLICIT ? PS_HOLD : PS_RUN;
-        break;
-      case PS_RUN: {
-        const double an = c.a + c.da;
-        c.kpend = 0.5 * c.da / (an * pm_hubble(an));
-        c.a = an;
-        c.a_grid = an;
-        c.nsteps += 1;
-        c.sortstep = 0;
-        c.refresh = P.full_every > 0 && (c.nsteps % P.full_every) == 0 ? 1 : 0;
-        dep = 1;
-        if (c.mode == SCHED_RATIO) {
-          if (c.nsteps >= c.max_steps) c.state = PS_FINALIZE;
-          else c.da = c.a * c.param;
-        } else if (c.mode == SCHED_FRAC) {
-          if (c.a >= c.a_end) c.state = PS_FINALIZE;
-          else c.da = fmin(c.param * c.a, c.a_end - c.a);
-        } else {
-          c.state = PS_HOLD;
-        }
-        if (stop_now && c.state == PS_RUN) c.state = PS_FINALIZE;
-        break;
-      }
-      case PS_FINALIZE:
-        c.kpend = 0.0;
-        c.sortstep = 0;
-        c.refresh = 0;
-        dep = 1;
-        c.state = PS_IDLE;
-        break;
-      default:
-        break;
-    }
-    if (pushed) {  // the particles are now in the buffer the push wrote
-      if (ovf) A.stats[pk].relayouts += 1u;
-      c.relayout = ovf;
-      c.sbuf ^= 1;
-      if (ovf) c.lgen ^= 1;
-    }
-    c.dep = dep;
-    A.clocks[pk] = c;
-    A.sortseg[pk].active = dep && c.sortstep;
-    any_sort |= dep && c.sortstep;
-    any_layout |= dep && (c.sortstep || c.relayout);
-    any_refresh |= dep && c.refresh;
-    if (dep) {
-      A.stats[pk].max_fix = 0;
-      A.stats[pk].mass_defect = 0;
-    }
-  }
-  any_sort = __syncthreads_or(any_sort);
-  any_layout = __syncthreads_or(any_layout);
-  any_refresh = __syncthreads_or(any_refresh);
-  if (threadIdx.x == 0) {
-    *A.sort_gate = any_sort ? 1u : 0u;
-    *A.layout_gate = any_layout ? 1u : 0u;
-    *A.refresh_gate = any_refresh ? 1u : 0u;
-  }
-}
-
-// ------------------------------------------------------------------------------------------
-// Energy and momentum of every peak that was just pushed (before the clock advances): the push
-// partials give K and sum p at the positions' a, the previous step's Green partials give W at
-// the same a (the grids were computed there).  ENERGY_SLICES CTAs per peak each reduce a slice
-// of the partials; the last one to finish (atomic ticket) merges the slices in slice order and
-// updates the statistics.  All sums are compensated, every order fixed.  The Layzer-Irvine
-// integral int K da advances by the trapezoid rule between samples.
-__global__ void __launch_bounds__(PM_THREADS) k_energy(StepArgs A) {
-  const int pk = blockIdx.y, sl = blockIdx.x;
-  const PeakClock C = A.clocks[pk];
-  if (C.state != PS_RUN && C.state != PS_FINALIZE) return;
-  const PeakDesc P = A.peaks[pk];
-  __shared__ CSum s_w[PM_THREADS / 32][5];
-  __shared__ u32 s_last;
-  CSum v[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) v[q] = CSum{0.0, 0.0};
-  const long long t0 = P.nst * sl / ENERGY_SLICES, t1 = P.nst * (sl + 1) / ENERGY_SLICES;
-  for (long long t = t0 + threadIdx.x; t < t1; t += PM_THREADS) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const double2 e = A.epart[(P.st_base + t) * 4 + q];
-      csum_merge(v[q], CSum{e.x, e.y});
-    }
-  }
-  // Green partials: one per warp of each Green block of this peak.
-  const long long nw = (P.nmodes + PM_THREADS * GREEN_MODES - 1) / (PM_THREADS * GREEN_MODES) * (PM_THREADS / 32);
-  const long long g0 = nw * sl / ENERGY_SLICES, g1 = nw * (sl + 1) / ENERGY_SLICES;
-  const double* wp = A.wpart + P.mode_base * (PM_THREADS / 32);
-  for (long long t = g0 + threadIdx.x; t < g1; t += PM_THREADS) csum_add(v[4], wp[t]);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    const CSum r = csum_warp(v[q]);
-    if (lane == 0) s_w[warp][q] = r;
-  }
-  __syncthreads();
-  double2* slice = A.eslice + ((long long)pk * ENERGY_SLICES) * 5;
-  if (threadIdx.x < 5) {
-    CSum t = s_w[0][threadIdx.x];
-    for (int w = 1; w < PM_THREADS / 32; ++w) csum_merge(t, s_w[w][threadIdx.x]);
-    slice[sl * 5 + threadIdx.x] = make_double2(t.s, t.c);
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&A.ecount[pk], 1u) == ENERGY_SLICES - 1 ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  __shared__ double s_tot[5];
-  if (threadIdx.x < 5) {
-    CSum t = CSum{0.0, 0.0};
-    for (int q = 0; q < ENERGY_SLICES; ++q) {
-      const double2 e = __ldcg(slice + q * 5 + threadIdx.x);
-      csum_merge(t, CSum{e.x, e.y});
-    }
-    s_tot[threadIdx.x] = t.s + t.c;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    A.ecount[pk] = 0u;
-    PeakStats& S = A.stats[pk];
-    const double a = C.a;
-    const double kin = P.m_part / (2.0 * a * a) * s_tot[3];
-    const double pot = 0.5 * (3.0 * PM_H_I * PM_H_I / (8.0 * M_PI)) * P.dx * P.dx * P.dx * s_tot[4];
-    if (S.nsamples == 0) {
-      S.li_int = 0.0;
-      S.li_e0 = a * (kin + pot);
-    } else {
-      S.li_int += 0.5 * (S.kin + kin) * (a - S.a_e);
-    }
-    S.a_e = a;
-    S.mom[0] = P.m_part * s_tot[0];
-    S.mom[1] = P.m_part * s_tot[1];
-    S.mom[2] = P.m_part * s_tot[2];
-    S.kin = kin;
-    S.pot = pot;
-    S.nsamples += 1;
-  }
-}
-
-// ------------------------------------------------------------------------------------------
-// Priming (particles loaded into the loading area): the Morton-key radix sort, the super-tile
-// starts in the sorted keys, the bin layout from the counts (k_layout), then the gather of the
-// loading area into the bins of the current buffer in sorted order.  Grid-stride loops over a
-// grid of a few CTAs per SM that return at once on the steps where no peak primes.
-__global__ void k_st_starts(StepArgs A, long long ntot) {
-  if (*A.sort_gate == 0u) return;
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < ntot; j += (long long)gridDim.x * blockDim.x) {
-    const int pk = pm_find(A.p_base, A.npeaks, j);
-    const PeakClock C = A.clocks[pk];
-    if (!(C.dep && C.sortstep)) continue;
-    const PeakDesc P = A.peaks[pk];
-    u32* ss = A.sstart + P.sst_off;
-    // Super-tile of each sorted key; a key outside the peak's key range (a failed sort) is
-    // clamped, so no start is ever written outside the peak's table.
-    const u32 kb = A.keys_sorted[j] >> P.st_shift;
-    if (kb >= (u32)P.nst) atomicOr(&A.stats[pk].status, 2u);
-    const int b = (int)min(kb, (u32)(P.nst - 1));
-    const int bprev = j == P.p_off ? -1 : (int)min(A.keys_sorted[j - 1] >> P.st_shift, (u32)(P.nst - 1));
-    for (int bb = bprev + 1; bb <= b; ++bb) ss[bb] = (u32)j;
-    if (j == P.p_off + P.n - 1)
-      for (int bb = b + 1; bb <= P.nst; ++bb) ss[bb] = (u32)(P.p_off + P.n);
-  }
-}
-
-__global__ void k_permute(StepArgs A, long long ntot) {
-  if (*A.sort_gate == 0u) return;
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < ntot; j += (long long)gridDim.x * blockDim.x) {
-    const int pk = pm_find(A.p_base, A.npeaks, j);
-    const PeakClock C = A.clocks[pk];
-    if (!(C.dep && C.sortstep)) continue;
-    const PeakDesc& P = A.peaks[pk];
-    const u32 q = A.perm[j];
-    const u32 S = min(A.keys_sorted[j] >> P.st_shift, (u32)(P.nst - 1));
-    const BinLayout L = blay(A, C.lgen)[P.st_base + S];
-    const long long r = j - (long long)A.sstart[P.sst_off + S];
-    // A failed sort (a value outside the peak, a rank outside the bin): never read or write outside.
-    if ((long long)q < P.p_off || (long long)q >= P.p_off + P.n || r < 0 || r >= (long long)L.cap) {
-      atomicOr(&A.stats[pk].status, 2u);
-      continue;
-    }
-    bpos(A, C.sbuf)[L.base + r] = A.lpos[q];
-    bmom(A, C.sbuf)[L.base + r] = A.lmom[q];
-  }
-}
-
-// Bin layout of every peak that primes or relayouts this step (one CTA per peak).  The new count
+// Bin layout of a peak that primes or relayouts this step, by one CTA of LAYOUT_THREADS.  The new count
 // of each super-tile comes from the sorted keys when priming; else it is the bin the push filled
 // plus its arrivals in the overflow area.  A bin's base capacity is count + count/8 +
 // BIN_SLACK_MIN (the peak's bin_shift and bin_min), rounded up to BIN_ALIGN.  On a relayout a
@@ -607,18 +403,14 @@ __global__ void k_permute(StepArgs A, long long ntot) {
 // proportion to the wants, and every particle is copied into the other buffer, which becomes
 // current.  The region, n + n/8 + n/8 + (BIN_SLACK_MIN + BIN_ALIGN) nst slots, covers every base
 // layout.
-// The layout goes into generation clock.lgen (the advance kernel switched to it).  The relayout
-// copies set the new fills; when priming, this kernel sets them to the counts, which the
-// permutation then provides.
-__global__ void __launch_bounds__(LAYOUT_THREADS) k_layout(StepArgs A) {
+// The layout goes into generation clock.lgen (the clock advance switched to it).  When priming,
+// the fills are set to the counts, which the permutation then provides; on a relayout the counts
+// go to new_count, and the relayout copies set the fills.
+__device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const PeakClock& C) {
   __shared__ u32 s_w[LAYOUT_THREADS / 32];
   __shared__ unsigned long long s_r[4][LAYOUT_THREADS / 32];
   __shared__ long long s_carry;
-  if (*A.layout_gate == 0u) return;
-  const int pk = blockIdx.x;
-  const PeakClock C = A.clocks[pk];
-  if (!(C.dep && (C.sortstep || C.relayout))) return;
-  const PeakDesc P = A.peaks[pk];
+  const PeakDesc& P = A.peaks[pk];
   const BinLayout* old = blay(A, C.lgen ^ 1) + P.st_base;
   BinLayout* lay = blay(A, C.lgen) + P.st_base;
   const BinFill* pushed = bfill(A, C.sbuf) + P.st_base;  // relayout: the buffer the push filled
@@ -745,6 +537,8 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) k_layout(StepArgs A) {
         cur[i] = BinFill{cnt, cnt, 0u, 0u};
         nxt[i] = BinFill{0u, 0u, 0u, 0u};
         A.ovf_in[P.st_base + i] = 0u;
+      } else {
+        A.new_count[P.st_base + i] = cnt;
       }
     }
     __syncthreads();
@@ -758,74 +552,315 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) k_layout(StepArgs A) {
       A.clocks[pk].relayout = partial ? 1 : 2;
       if (!partial) {  // the full relayout fills the other buffer, which becomes current
         A.clocks[pk].sbuf = C.sbuf ^ 1;
+        A.plan[pk].flags ^= PLAN_SBUF;
         A.stats[pk].relayouts_full += 1u;
       }
     }
   }
 }
 
-// Relayout, per super-tile.  Full (clock.relayout = 2): every bin the push filled (old layout,
-// other buffer) is copied in order to the start of its new bin in the current buffer.  Partial
-// (1): only the bins that got a new place after the last bin move there, inside the current
-// buffer.  Either way the bin's fill is then set to its new count,
-// which includes the arrivals k_relayout_ovf places next.
-__global__ void __launch_bounds__(PM_THREADS) k_relayout_copy(StepArgs A) {
-  if (*A.layout_gate == 0u) return;
-  const int pk = blockIdx.y;  // RELAYOUT_COPY_BLOCKS CTAs per peak, each looping over its bins
+// Layouts of the priming peaks (one CTA per peak; only in steps that prime).
+__global__ void __launch_bounds__(LAYOUT_THREADS) k_layout(StepArgs A) {
+  const int pk = blockIdx.x;
   const PeakClock C = A.clocks[pk];
-  if (!(C.dep && C.relayout)) return;
-  const bool full = C.relayout == 2;
-  const int src = full ? (C.sbuf ^ 1) : C.sbuf;
-  const long long st0 = A.st_base[pk], nst = A.st_base[pk + 1] - st0;
-  for (long long t = blockIdx.x; t < nst; t += gridDim.x) {
-    const long long g = st0 + t;
-    const u32 arrivals = A.ovf_in[g];
-    const BinLayout L0 = blay(A, C.lgen ^ 1)[g], L = blay(A, C.lgen)[g];
-    if (!full && L.base == L0.base) continue;  // partial relayout: this bin stays as it is (uniform)
-    const BinRuns R = bin_runs(L0, bfill(A, src)[g]);
-    const int4* ip = bpos(A, src);
-    const float4* im = bmom(A, src);
-    int4* op = bpos(A, C.sbuf) + L.base;
-    float4* om = bmom(A, C.sbuf) + L.base;
-    const int n = min(R.total(), (int)L.cap);
-    for (int k = threadIdx.x; k < n; k += PM_THREADS) {  // old and new places never overlap
-      const long long j = R.slot(k);
-      op[k] = ip[j];
-      om[k] = im[j];
+  if (C.dep && C.sortstep) layout_peak(A, pk, C);
+}
+
+// ------------------------------------------------------------------------------------------
+// After the push: each peak's energy and momentum, and its clock with (when the push overflowed a
+// bin) its new bin layout.  One launch, because every kernel of a step waits for the one before;
+// in it eslices CTAs per peak do the energies while one more does the clock.  What the energy CTAs
+// need of the clock the push has put aside (pushed_a), so the two sides share nothing.
+//
+// Energy of a peak that was just pushed: the push partials give K and sum p at the positions' a,
+// the previous step's Green partials give W at the same a (the grids were computed there).  Each
+// CTA (ENERGY_THREADS of the launch's threads; the compensated merges of more warps cost more than
+// they save) reduces a slice of the partials, about eight per thread for the engine's largest peak;
+// the last one to finish (atomic ticket) merges the slices in slice order and updates the
+// statistics.  All sums are compensated, every order fixed.  The Layzer-Irvine integral int K da
+// advances by the trapezoid rule between samples.
+__device__ __forceinline__ void energy_slice(const StepArgs& A, int pk, int sl, CSum& tot) {
+  const PeakDesc& P = A.peaks[pk];
+  __shared__ CSum s_w[ENERGY_THREADS / 32][5];
+  CSum v[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) v[q] = CSum{0.0, 0.0};
+  const long long t0 = (long long)P.nst * sl / A.eslices, t1 = (long long)P.nst * (sl + 1) / A.eslices;
+  for (long long t = t0 + threadIdx.x; t < t1; t += ENERGY_THREADS) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double2 e = A.epart[(P.st_base + t) * 4 + q];
+      csum_merge(v[q], CSum{e.x, e.y});
     }
-    __syncthreads();  // every thread has read the old fill (a partial relayout rewrites that entry)
-    if (threadIdx.x == 0) {
-      const u32 cnt = min((u32)R.total() + arrivals, L.cap);
-      bfill(A, C.sbuf)[g] = BinFill{cnt, cnt, 0u, 0u};
-    }
+  }
+  // Green partials: one per warp of the kernel that multiplies by the Green's function.
+  const long long g0 = P.nwpart * sl / A.eslices, g1 = P.nwpart * (sl + 1) / A.eslices;
+  const double* wp = A.wpart + P.mode_base * (PM_THREADS / 32);
+  for (long long t = g0 + threadIdx.x; t < g1; t += ENERGY_THREADS) csum_add(v[4], wp[t]);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const CSum r = csum_warp(v[q]);
+    if (lane == 0) s_w[warp][q] = r;
+  }
+  __syncthreads();
+  if (threadIdx.x < 5) {
+    CSum t = s_w[0][threadIdx.x];
+    for (int w = 1; w < ENERGY_THREADS / 32; ++w) csum_merge(t, s_w[w][threadIdx.x]);
+    tot = t;
   }
 }
 
-// Relayout: each particle of a relayouting peak's overflow area to the end of its new bin
-// (ovf_in counts down to zero, one rank per particle).  RELAYOUT_OVF_BLOCKS CTAs per peak walk
-// only that peak's overflow entries.
-__global__ void __launch_bounds__(PM_THREADS) k_relayout_ovf(StepArgs A) {
-  if (*A.layout_gate == 0u) return;
-  const int pk = blockIdx.y;
-  const PeakClock C = A.clocks[pk];
-  if (!(C.dep && C.relayout)) return;
+// The merged slices into the peak's statistics (one thread; s_tot: momentum (3), p^2, Green sum).
+__device__ __forceinline__ void energy_stats(const StepArgs& A, int pk, double a, const double* s_tot) {
   const PeakDesc& P = A.peaks[pk];
-  const long long novf = (long long)min(A.ovf_n[pk], (u32)P.n);
-  for (long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x; o < novf; o += (long long)gridDim.x * blockDim.x) {
-    const long long j = P.p_off + o;
-    const int4 ps = A.lpos[j];
-    const int N = P.N, l2 = P.log2N, s = P.log2TS;
-    const u32 S = pm_morton3(((ps.x >> (2 * l2)) & (N - 1)) >> s, ((ps.x >> l2) & (N - 1)) >> s, (ps.x & (N - 1)) >> s);
-    const long long g = P.st_base + S;
-    const BinLayout L = blay(A, C.lgen)[g];
-    const u32 cnt = bfill(A, C.sbuf)[g].stay;  // the new count, arrivals from the overflow area included
-    const u32 v = atomicSub(&A.ovf_in[g], 1u);
-    if (v == 0u || v > cnt || cnt > L.cap) {  // counts that disagree: never write outside the bin
-      atomicOr(&A.stats[pk].status, 4u);
+  PeakStats& S = A.stats[pk];
+  const double kin = P.m_part / (2.0 * a * a) * s_tot[3];
+  const double pot = 0.5 * (3.0 * PM_H_I * PM_H_I / (8.0 * M_PI)) * P.dx * P.dx * P.dx * s_tot[4];
+  if (S.nsamples == 0) {
+    S.li_int = 0.0;
+    S.li_e0 = a * (kin + pot);
+  } else {
+    S.li_int += 0.5 * (S.kin + kin) * (a - S.a_e);
+  }
+  S.a_e = a;
+  S.mom[0] = P.m_part * s_tot[0];
+  S.mom[1] = P.m_part * s_tot[1];
+  S.mom[2] = P.m_part * s_tot[2];
+  S.kin = kin;
+  S.pot = pot;
+  S.nsamples += 1;
+}
+
+// Clock advance of a peak (one thread): applies the step that the push just made, selects the next
+// step size, whether this step primes by sort, relayouts (the push overflowed a bin) or re-sorts
+// the super-tiles by cell, and whether the peak re-deposits.  A running peak's particles are now
+// in the other bin buffer; one that relayouts switches to a new layout generation.  The gate
+// words are raised here; the face fix-up, which runs after the kernels they gate, lowers them.
+// Returns whether the peak relayouts.
+__device__ __forceinline__ bool advance_clock(const StepArgs& A, int pk) {
+  const PeakDesc& P = A.peaks[pk];
+  PeakClock c = A.clocks[pk];
+  const u64 max_fix = A.stats[pk].max_fix;  // (fetched with the clock, not after it)
+  const u32 n_ovf = A.ovf_n[pk];
+  int dep = 0;
+  // Collapse detection on the deposit made by the previous step, i.e. of the positions at c.a.
+  // This step's push has already moved a running peak on to c.a + c.da, so a stop takes
+  // effect after the step is booked below: the next step applies its closing kick and ends.
+  bool stop_now = false;
+  if (c.has_delta && c.delta_collapse > 0 && c.a_collapse < 0 && c.state != PS_PRIME) {
+    if ((double)max_fix / (double)PM_FIX_ONE / P.n_mean - 1.0 >= c.delta_collapse) {
+      c.a_collapse = c.a;
+      stop_now = c.stop_on_collapse && c.state == PS_RUN;
+    }
+  }
+  const bool pushed = c.state == PS_RUN || c.state == PS_FINALIZE;
+  const int ovf = pushed && n_ovf != 0u ? 1 : 0;
+  switch (c.state) {
+    case PS_PRIME:
+      dep = 1;
+      c.sortstep = 1;
+      c.relayout = 0;
+      c.refresh = 0;
+      c.lgen ^= 1;
+      c.kpend = 0.0;
+      c.a_grid = c.a;
+      c.has_delta = 1;
+      c.state = c.mode == SCHED_EXPLICIT ? PS_HOLD : PS_RUN;
+      break;
+    case PS_RUN: {
+      const double an = c.a + c.da;
+      c.kpend = 0.5 / PM_H_I * c.da * sqrt(an);  // 0.5 da / (a H(a))
+      c.a = an;
+      c.a_grid = an;
+      c.nsteps += 1;
+      c.sortstep = 0;
+      c.refresh = P.full_every > 0 && (c.nsteps % P.full_every) == 0 ? 1 : 0;
+      dep = 1;
+      if (c.mode == SCHED_RATIO) {
+        if (c.nsteps >= c.max_steps) c.state = PS_FINALIZE;
+        else c.da = c.a * c.param;
+      } else if (c.mode == SCHED_FRAC) {
+        if (c.a >= c.a_end) c.state = PS_FINALIZE;
+        else c.da = fmin(c.param * c.a, c.a_end - c.a);
+      } else {
+        c.state = PS_HOLD;
+      }
+      if (stop_now && c.state == PS_RUN) c.state = PS_FINALIZE;
+      break;
+    }
+    case PS_FINALIZE:
+      c.kpend = 0.0;
+      c.sortstep = 0;
+      c.refresh = 0;
+      dep = 1;
+      c.state = PS_IDLE;
+      break;
+    default:
+      break;
+  }
+  if (pushed) {  // the particles are now in the buffer the push wrote
+    if (ovf) A.stats[pk].relayouts += 1u;
+    c.relayout = ovf;
+    c.sbuf ^= 1;
+    if (ovf) c.lgen ^= 1;
+  }
+  c.dep = dep;
+  A.clocks[pk] = c;
+  A.plan[pk] = plan_of(c, P);
+  A.sortseg[pk].active = dep && c.sortstep;
+  if (dep) {
+    A.stats[pk].max_fix = 0;
+    A.stats[pk].mass_defect = 0;
+    if (c.sortstep) atomicExch(A.sort_gate, 1u);
+    if (c.relayout) atomicExch(A.layout_gate, 1u);
+    if (c.refresh) atomicExch(A.refresh_gate, 1u);
+  }
+  return dep && c.relayout;
+}
+
+__global__ void __launch_bounds__(LAYOUT_THREADS) k_tick(StepArgs A) {
+  __shared__ u32 s_last;
+  __shared__ double s_tot[5];
+  const int pk = blockIdx.y;
+  pdl_wait();
+  if ((int)blockIdx.x == A.eslices) {  // the clock
+    if (threadIdx.x == 0) s_last = advance_clock(A, pk);
+    __syncthreads();
+    if (s_last) layout_peak(A, pk, A.clocks[pk]);
+    return;
+  }
+  const double a = A.pushed_a[pk];
+  if (a < 0.0 || threadIdx.x >= ENERGY_THREADS) return;  // not pushed
+  CSum t;  // threads 0 to 4: the sum each merges
+  energy_slice(A, pk, blockIdx.x, t);
+  if (A.eslices > 1) {
+    if (threadIdx.x < 5) {
+      A.eslice[((long long)pk * ENERGY_SLICES + blockIdx.x) * 5 + threadIdx.x] = make_double2(t.s, t.c);
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&A.ecount[pk], 1u) == (u32)A.eslices - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 5) {
+      t = CSum{0.0, 0.0};
+      for (int q = 0; q < A.eslices; ++q) {
+        const double2 e = __ldcg(A.eslice + ((long long)pk * ENERGY_SLICES + q) * 5 + threadIdx.x);
+        csum_merge(t, CSum{e.x, e.y});
+      }
+    }
+    if (threadIdx.x == 0) A.ecount[pk] = 0u;
+  }
+  if (threadIdx.x < 5) s_tot[threadIdx.x] = t.s + t.c;
+  __syncthreads();
+  if (threadIdx.x == 0) energy_stats(A, pk, a, s_tot);
+}
+
+// ------------------------------------------------------------------------------------------
+// Priming (particles loaded into the loading area): the Morton-key radix sort, the super-tile
+// starts in the sorted keys, the bin layout from the counts (k_layout), then the gather of the
+// loading area into the bins of the current buffer in sorted order.  Grid-stride loops over a
+// grid of a few CTAs per SM that return at once on the steps where no peak primes.
+__global__ void k_st_starts(StepArgs A, long long ntot) {
+  if (*A.sort_gate == 0u) return;
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < ntot; j += (long long)gridDim.x * blockDim.x) {
+    const int pk = pm_find(A.p_base, A.npeaks, j);
+    const PeakClock C = A.clocks[pk];
+    if (!(C.dep && C.sortstep)) continue;
+    const PeakDesc P = A.peaks[pk];
+    u32* ss = A.sstart + P.sst_off;
+    // Super-tile of each sorted key; a key outside the peak's key range (a failed sort) is
+    // clamped, so no start is ever written outside the peak's table.
+    const u32 kb = A.keys_sorted[j] >> P.st_shift;
+    if (kb >= (u32)P.nst) atomicOr(&A.stats[pk].status, 2u);
+    const int b = (int)min(kb, (u32)(P.nst - 1));
+    const int bprev = j == P.p_off ? -1 : (int)min(A.keys_sorted[j - 1] >> P.st_shift, (u32)(P.nst - 1));
+    for (int bb = bprev + 1; bb <= b; ++bb) ss[bb] = (u32)j;
+    if (j == P.p_off + P.n - 1)
+      for (int bb = b + 1; bb <= P.nst; ++bb) ss[bb] = (u32)(P.p_off + P.n);
+  }
+}
+
+__global__ void k_permute(StepArgs A, long long ntot) {
+  if (*A.sort_gate == 0u) return;
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < ntot; j += (long long)gridDim.x * blockDim.x) {
+    const int pk = pm_find(A.p_base, A.npeaks, j);
+    const PeakClock C = A.clocks[pk];
+    if (!(C.dep && C.sortstep)) continue;
+    const PeakDesc& P = A.peaks[pk];
+    const u32 q = A.perm[j];
+    const u32 S = min(A.keys_sorted[j] >> P.st_shift, (u32)(P.nst - 1));
+    const BinLayout L = blay(A, C.lgen)[P.st_base + S];
+    const long long r = j - (long long)A.sstart[P.sst_off + S];
+    // A failed sort (a value outside the peak, a rank outside the bin): never read or write outside.
+    if ((long long)q < P.p_off || (long long)q >= P.p_off + P.n || r < 0 || r >= (long long)L.cap) {
+      atomicOr(&A.stats[pk].status, 2u);
       continue;
     }
-    bpos(A, C.sbuf)[L.base + cnt - v] = ps;
-    bmom(A, C.sbuf)[L.base + cnt - v] = A.lmom[j];
+    bpos(A, C.sbuf)[L.base + r] = A.lpos[q];
+    bmom(A, C.sbuf)[L.base + r] = A.lmom[q];
+  }
+}
+
+// Relayout copies of the peaks whose push overflowed a bin, a grid-stride loop that returns at once
+// in the steps without one.  Full relayout (clock.relayout = 2): every bin the push filled (old
+// layout, other buffer) is copied in order to the start of its new bin in the current buffer.
+// Partial (1): only the bins that got a new place after the last bin move there, inside the
+// current buffer.  Either way the bin's fill is then set to its new count, and each particle of
+// the peak's overflow area goes to the end of its new bin (ovf_in counts down to zero, one rank
+// per particle).  The two parts write disjoint slots and read nothing the other writes, so they
+// need no order between them.
+__global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__ StepArgs A) {
+  pdl_wait();
+  if (*A.layout_gate == 0u) return;
+  for (int pk = 0; pk < A.npeaks; ++pk) {
+    const PeakClock& C = A.clocks[pk];
+    const int kind = C.dep ? C.relayout : 0, sbuf = C.sbuf, lgen = C.lgen;
+    if (!kind) continue;
+    const PeakDesc& P = A.peaks[pk];
+    const bool full = kind == 2;
+    const int src = full ? (sbuf ^ 1) : sbuf;
+    for (long long t = blockIdx.x; t < P.nst; t += gridDim.x) {
+      const long long g = P.st_base + t;
+      const BinLayout L0 = blay(A, lgen ^ 1)[g], L = blay(A, lgen)[g];
+      if (!full && L.base == L0.base) continue;  // partial relayout: this bin stays as it is (uniform)
+      const BinRuns R = bin_runs(L0, bfill(A, src)[g]);
+      const int4* ip = bpos(A, src);
+      const float4* im = bmom(A, src);
+      int4* op = bpos(A, sbuf) + L.base;
+      float4* om = bmom(A, sbuf) + L.base;
+      const int n = min(R.total(), (int)L.cap);
+      for (int k = threadIdx.x; k < n; k += PM_THREADS) {  // old and new places never overlap
+        const long long j = R.slot(k);
+        op[k] = ip[j];
+        om[k] = im[j];
+      }
+      __syncthreads();  // every thread has read the old fill (a partial relayout rewrites that entry)
+      if (threadIdx.x == 0) {
+        const u32 cnt = min(A.new_count[g], L.cap);
+        bfill(A, sbuf)[g] = BinFill{cnt, cnt, 0u, 0u};
+      }
+    }
+    const long long novf = (long long)min(A.ovf_n[pk], (u32)P.n);
+    for (long long o = (long long)blockIdx.x * PM_THREADS + threadIdx.x; o < novf;
+         o += (long long)gridDim.x * PM_THREADS) {
+      const long long j = P.p_off + o;
+      const int4 ps = A.lpos[j];
+      const int N = P.N, l2 = P.log2N, s = P.log2TS;
+      const u32 S = pm_morton3(((ps.x >> (2 * l2)) & (N - 1)) >> s, ((ps.x >> l2) & (N - 1)) >> s, (ps.x & (N - 1)) >> s);
+      const long long g = P.st_base + S;
+      const BinLayout L = blay(A, lgen)[g];
+      const u32 cnt = A.new_count[g];  // arrivals from the overflow area included
+      const u32 v = atomicSub(&A.ovf_in[g], 1u);
+      if (v == 0u || v > cnt || cnt > L.cap) {  // counts that disagree: never write outside the bin
+        atomicOr(&A.stats[pk].status, 4u);
+        continue;
+      }
+      bpos(A, sbuf)[L.base + cnt - v] = ps;
+      bmom(A, sbuf)[L.base + cnt - v] = A.lmom[j];
+    }
   }
 }
 
@@ -951,6 +986,7 @@ __device__ __forceinline__ void tile_sort(const StepArgs& A, const PeakDesc& P, 
 __global__ void __launch_bounds__(TSORT_THREADS) k_tile_sort(StepArgs A, long long nst) {
   extern __shared__ __align__(16) unsigned char s_ts[];
   __shared__ int s_pk;
+  pdl_wait();
   if (*A.refresh_gate == 0u) return;
   for (long long t = blockIdx.x; t < nst; t += gridDim.x) {
     if (threadIdx.x == 0) s_pk = pm_find(A.st_base, A.npeaks, t);
@@ -993,26 +1029,6 @@ __device__ __forceinline__ int halo_index(int lx, int ly, int lz, int T) {
   if (ly == T) return (T + 1) * (T + 1) + lx * (T + 1) + lz;
   return (T + 1) * (T + 1) + T * (T + 1) + lx * T + ly;
 }
-// Inverse of face_index.
-template <int T>
-__device__ __forceinline__ void face_coords(int f, int& lx, int& ly, int& lz) {
-  if (f < T * T) {
-    lx = 0;
-    ly = f / T;
-    lz = f % T;
-  } else if (f < T * T + (T - 1) * T) {
-    const int r = f - T * T;
-    lx = 1 + r / T;
-    ly = 0;
-    lz = r % T;
-  } else {
-    const int r = f - T * T - (T - 1) * T;
-    lx = 1 + r / (T - 1);
-    ly = 1 + r % (T - 1);
-    lz = 0;
-  }
-}
-
 // Finish the face nodes of super-tile Y (whole CTA of FIX_THREADS): each face node's own
 // partial plus the halo partials of the lower neighbours Y - o, o = (ox, oy, oz) in {0,1}^3 \ 0,
 // that reach it (node (lx + TS ox, ...) of the neighbour, which lies on its upper halo, for a
@@ -1025,42 +1041,26 @@ __device__ __forceinline__ void fixup_faces(const StepArgs& A, const PeakDesc& P
   const int N = P.N;
   const int sx = pm_compact3(Y >> 2), sy = pm_compact3(Y >> 1), sz = pm_compact3(Y);
   const long long* face = A.face + P.face_off + (long long)Y * FC;
-  // Up to KF face nodes per thread, handled together so that their loads are in flight at once:
-  // own partials, then each node's first neighbour (every face node has one), then the other
-  // neighbours of edge and corner nodes.  Integer sums: the order does not change a bit.
-  constexpr int KF = (FC + FIX_THREADS - 1) / FIX_THREADS;
-  long long S[KF];
-  int zm[KF], cx[KF], cy[KF], cz[KF];
+  // Three face nodes per thread, one of each face (x: TS x TS nodes; y: without lx = 0; z: without
+  // lx = 0 and ly = 0), so that coordinates are shifts and the neighbours that reach a node are
+  // known: always the face's own, the others only for edge and corner nodes.  All own partials and
+  // first neighbours are loaded together.  Integer sums: the order does not change a bit.
+  static_assert(TS * TS <= FIX_THREADS, "one node of each face per thread");
+  const int u = threadIdx.x / TS, v = threadIdx.x % TS;
+  const bool in = threadIdx.x < TS * TS, on[3] = {in, in && u > 0, in && u > 0 && v > 0};
+  const int cx[3] = {0, u, u}, cy[3] = {u, 0, v}, cz[3] = {v, v, 0};
+  long long S[3] = {0, 0, 0};
+  constexpr int H1 = (TS + 1) * (TS + 1), H2 = H1 + TS * (TS + 1);  // starts of the y and z planes in the halo
+  if (on[0]) S[0] = __ldcg(face + u * TS + v) + __ldcg(nb[1] + u * (TS + 1) + v);
+  if (on[1]) S[1] = __ldcg(face + TS * TS + (u - 1) * TS + v) + __ldcg(nb[2] + H1 + u * (TS + 1) + v);
+  if (on[2]) S[2] = __ldcg(face + TS * TS + (TS - 1) * TS + (u - 1) * (TS - 1) + v - 1) + __ldcg(nb[4] + H2 + u * TS + v);
+  if (on[0] && u == 0) S[0] += __ldcg(nb[2] + H1 + v) + __ldcg(nb[3] + TS * (TS + 1) + v);
+  if (on[0] && v == 0) S[0] += __ldcg(nb[4] + H2 + u) + __ldcg(nb[5] + u * (TS + 1) + TS);
+  if (on[0] && u == 0 && v == 0) S[0] += __ldcg(nb[6] + H1 + TS) + __ldcg(nb[7] + TS * (TS + 1) + TS);
+  if (on[1] && v == 0) S[1] += __ldcg(nb[4] + H2 + u * TS) + __ldcg(nb[6] + H1 + u * (TS + 1) + TS);
 #pragma unroll
-  for (int k = 0; k < KF; ++k) {
-    const int f = threadIdx.x + k * FIX_THREADS;
-    zm[k] = 0;
-    S[k] = 0;
-    cx[k] = cy[k] = cz[k] = 0;
-    if (f < FC) {
-      face_coords<TS>(f, cx[k], cy[k], cz[k]);
-      S[k] = __ldcg(face + f);
-      zm[k] = (cx[k] == 0 ? 1 : 0) | (cy[k] == 0 ? 2 : 0) | (cz[k] == 0 ? 4 : 0);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < KF; ++k) {
-    if (zm[k]) {
-      const int o = zm[k] & -zm[k];
-      S[k] += __ldcg(nb[o] + halo_index(cx[k] + TS * (o & 1), cy[k] + TS * ((o >> 1) & 1), cz[k] + TS * (o >> 2), TS));
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < KF; ++k) {
-    const int first = zm[k] & -zm[k];
-    for (int o = zm[k]; o; o = (o - 1) & zm[k]) {  // the other non-empty subsets of zm[k]
-      if (o == first) continue;
-      S[k] += __ldcg(nb[o] + halo_index(cx[k] + TS * (o & 1), cy[k] + TS * ((o >> 1) & 1), cz[k] + TS * (o >> 2), TS));
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < KF; ++k) {
-    if (threadIdx.x + k * FIX_THREADS >= FC) continue;
+  for (int k = 0; k < 3; ++k) {
+    if (!on[k]) continue;
     const long long Dv = S[k] - P.n_mean_fix;
     const long long node = ((long long)(sx * TS + cx[k]) * N + (sy * TS + cy[k])) * N + (sz * TS + cz[k]);
     P.delta[node] = (float)((double)Dv * P.inv_fix_nmean);
@@ -1085,10 +1085,12 @@ __device__ __forceinline__ int dep_addr(int node) {
   const int lx = node / (T1 * T1), r = node - lx * (T1 * T1), ly = r / T1, lz = r - ly * T1;
   return lx * patch_ps(TS) + ly * patch_rs(TS) + lz;
 }
-// A node's chunk sum from its split accumulators (high word modulo 2^32, see deposit_super).
+// A node's chunk sum S from its two accumulator words (see deposit_super): S lies within
+// [2^19 hi - DEP_BIAS, 2^19 hi - DEP_BIAS + 2^32), and its low 32 bits are lo.
+#define DEP_BIAS 32764u
+__device__ __forceinline__ u32 chunk_rest(u32 hi, u32 lo) { return lo - (hi << 19) + DEP_BIAS; }
 __device__ __forceinline__ long long chunk_sum(u32 hi, u32 lo) {
-  const long long hs = hi >= 0xFFFFE000u ? (long long)hi - (1LL << 32) : (long long)hi;
-  return hs * (1LL << 19) + (long long)lo;
+  return ((long long)hi << 19) + (long long)chunk_rest(hi, lo) - (long long)DEP_BIAS;
 }
 
 // Adds a full chunk's node sums into the fold scratch (first chunk: stores) and clears the
@@ -1104,27 +1106,96 @@ __device__ __noinline__ void fold_chunk(u64* acc64, u32* acc_hi, u32* acc_lo, bo
   }
 }
 
-// One corner weight W (a nearest integer of a product in units of 2^-38, 0 <= W < 2^39, see
-// fix_round) split for the two accumulator words: hi = W >> 19, lo = W & (2^19 - 1).  The FMA's
-// result has the bits 0x4330000000000000 + W, so hi is one funnel shift of its two words (the
-// exponent bits shift out of the 32-bit result) and lo one mask of the low word.
+// One corner weight W (the nearest integer of a product in units of 2^-38, 0 <= W < 2^39, see
+// fix_round): W >> 19, and W modulo 2^32.  The FMA's result has the bits 0x4330000000000000 + W, so
+// the first is one funnel shift of its two words (the exponent bits shift out) and the second its
+// low word as it is.
 struct Split {
   u32 hi, lo;
 };
 __device__ __forceinline__ Split fix_split(double a, double b) {
   const double r = fma(a, b, 4503599627370496.0);
   const u32 wl = (u32)__double2loint(r), wh = (u32)__double2hiint(r);
-  return Split{__funnelshift_r(wl, wh, 19), wl & 0x7FFFFu};
+  return Split{__funnelshift_r(wl, wh, 19), wl};
+}
+
+// The nodes of a super-tile itself out of the accumulators: delta of interior nodes, partials of
+// face nodes; dsum and smax: the sum of S - n_mean_fix and the largest S over the interior nodes.
+// GENERAL: 64-bit integers throughout, with the sums of folded chunks and the float64 counts.
+// Otherwise (one chunk, n_mean < 2^10) S - n_mean_fix is formed in FP64, exactly: both accumulator
+// words are brought in by bit construction (2^52 + word) and one FMA joins them, so that the
+// conversion to FP32 delta is the same as from the integer; sums of up to TS^3 such terms of one
+// chunk stay below 2^53.
+template <int TS, bool GENERAL>
+__device__ __forceinline__ void write_nodes(const u32* acc_hi, const u32* acc_lo, const u64* fold, float* delta,
+                                            double* rho64, long long* face, int N, long long nmf, double inv,
+                                            long long& dsum, long long& smax) {
+  constexpr int RS = patch_rs(TS), PS = patch_ps(TS), G4 = TS / 4, T1 = TS + 1;
+  const double c_lo = 4503599627370496.0 + (double)((long long)DEP_BIAS + nmf);  // exact below 2^53
+  long long isum = 0, imax = 0;
+  double fsum = 0.0, fmaxd = -9007199254740992.0;
+  for (int item = threadIdx.x; item < TS * TS * G4; item += DEP_THREADS) {
+    const int g = item % G4, ly = (item / G4) % TS, lx = item / (G4 * TS);
+    const int ad = lx * PS + ly * RS + 4 * g;
+    const uint4 h = *reinterpret_cast<const uint4*>(acc_hi + ad);
+    const uint4 l = *reinterpret_cast<const uint4*>(acc_lo + ad);
+    const u32 hv[4] = {h.x, h.y, h.z, h.w}, lv[4] = {l.x, l.y, l.z, l.w};
+    const bool row_face = lx == 0 || ly == 0;
+    if (row_face || g == 0) {
+      const int nf = row_face ? 4 : 1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < nf) {
+          long long S = chunk_sum(hv[k], lv[k]);
+          if (GENERAL && fold) S += (long long)fold[(lx * T1 + ly) * T1 + 4 * g + k];
+          face[face_index(lx, ly, 4 * g + k, TS)] = S;
+        }
+    }
+    if (row_face) continue;
+    float4 d;
+    float* dv = &d.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (GENERAL) {
+        long long S = chunk_sum(hv[k], lv[k]);
+        if (fold) S += (long long)fold[(lx * T1 + ly) * T1 + 4 * g + k];
+        const long long D = S - nmf;
+        dv[k] = (float)((double)D * inv);
+        if (g > 0 || k > 0) {
+          isum += D;
+          imax = S > imax ? S : imax;
+          if (rho64) rho64[((long long)lx * N + ly) * N + 4 * g + k] = (double)S * (1.0 / (double)PM_FIX_ONE);
+        }
+      } else {
+        const double hd = __hiloint2double(0x43300000, (int)hv[k]) - 4503599627370496.0;
+        const double ld = __hiloint2double(0x43300000, (int)chunk_rest(hv[k], lv[k])) - c_lo;
+        const double D = fma(hd, 524288.0, ld);
+        dv[k] = (float)(D * inv);
+        if (k > 0 || g > 0) {
+          fsum += D;
+          fmaxd = D > fmaxd ? D : fmaxd;
+        }
+      }
+    }
+    *reinterpret_cast<float4*>(delta + ((long long)lx * N + ly) * N + 4 * g) = d;
+  }
+  if (GENERAL) {
+    dsum = isum;
+    smax = imax;
+  } else {
+    dsum = (long long)fsum;
+    const long long m = (long long)fmaxd + nmf;
+    smax = m > 0 ? m : 0;
+  }
 }
 
 template <int TS, int SB>
-__device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc& P, const PeakClock& C, int pk,
-                                              u32 st, u32* smem, double* rho64) {
+__device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc& P, int pk, u32 st,
+                                              const BinLayout& L, const BinFill& F, u32* smem, double* rho64) {
   constexpr int T1 = TS + 1, NN = T1 * T1 * T1;
   constexpr int RS = patch_rs(TS), PS = patch_ps(TS), SZ = patch_size(TS);
-  constexpr int NG = TS / 4 + 1;        // 4-node groups per patch row (the last holds the upper halo node)
   constexpr int FC = TS * TS * TS - (TS - 1) * (TS - 1) * (TS - 1);
-  static_assert(RS % 4 == 0 && PS % 4 == 0 && RS >= 4 * NG, "patch rows are read 16 bytes at a time");
+  static_assert(RS % 4 == 0 && PS % 4 == 0, "patch rows are read 16 bytes at a time");
   u32* acc_hi = smem;
   u32* acc_lo = smem + SZ;
   __shared__ long long s_red[DEP_THREADS / 32];
@@ -1132,11 +1203,7 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
   const int N = P.N, l2 = P.log2N;
   const int sx = pm_compact3(st >> 2), sy = pm_compact3(st >> 1), sz = pm_compact3(st);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  static_assert((2 * SZ) % 4 == 0, "accumulators are cleared 16 bytes at a time");
-  for (int i = threadIdx.x; i < 2 * SZ / 4; i += DEP_THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
-  const long long gst = P.st_base + st;
-  const BinLayout L = blay(A, C.lgen)[gst];
-  const BinRuns R = bin_runs(L, bfill(A, SB)[gst]);
+  const BinRuns R = bin_runs(L, F);
   // A cell index belongs to this super-tile iff its bits outside the local ones equal the
   // super-tile's: one mask and one compare (negative or out-of-mesh values never match).
   const int local = ((TS - 1) << (2 * l2)) | ((TS - 1) << l2) | (TS - 1);
@@ -1147,57 +1214,56 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
   // of 16-byte entries holds the NN 8-byte sums several times over).
   static_assert((8191 / DEP_THREADS) * DEP_THREADS * sizeof(int4) >= NN * sizeof(u64), "fold scratch too small");
   bool folded = false;
-  // Split accumulators.  A weight W (at most 2^38, at least -3 for the remainder corner) goes in
-  // as hi = W >> 19 in [-1, 2^19] and lo = W & (2^19 - 1).  A node takes at most one contribution
-  // per particle of a chunk, so with CHUNK <= 8191 the low sums stay below 2^32 and the high
-  // sums lie in [-CHUNK, CHUNK * 2^19], an interval shorter than 2^32 - 8192: kept modulo 2^32
-  // in a u32, a value at or above 2^32 - 8192 is the negative one.  Both are exact.  A typical
-  // super-tile (about TS^3 particles) is a single chunk.
+  // Two accumulator words per node.  A weight W (at most 2^38) adds W >> 19 to hi and W to lo
+  // modulo 2^32; the eighth corner, whose weight is the remainder 2^38 - (the other seven), adds
+  // the hi of its own product, which the remainder differs from by less than 4.  A node takes at
+  // most one contribution per particle of a chunk of n <= 8191 particles, so hi stays below 2^32,
+  // and the node's sum S differs from 2^19 hi by more than -4 n >= -DEP_BIAS and less than
+  // n (2^19 + 4) <= 2^32 - DEP_BIAS: S is the one value in that interval whose low 32 bits are lo.
+  // Exact, and neither word needs a mask or a carry (the split into two 19-bit fields that this
+  // replaced took 14 more integer instructions per particle).  A typical super-tile (about TS^3
+  // particles) is a single chunk.
   constexpr int CH_IT = 8191 / DEP_THREADS;  // sweeps of DEP_THREADS particles per chunk
   static_assert(CH_IT >= 1 && CH_IT * DEP_THREADS <= 8191, "chunk too large for the split accumulators");
-  static_assert(PM_FIX_BITS == 38, "the split accumulators assume 38 fractional bits");
+  static_assert(PM_FIX_BITS == 38, "the two accumulator words assume 38 fractional bits");
+  static_assert(CH_IT * DEP_THREADS * 4 <= (int)DEP_BIAS, "bias of the interval");
   // 32-bit indices inside the bin's two runs (fewer integer instructions and live registers than
   // 64-bit pointers): particle k sits at pp[k] in the first run, at pp[k + d1] in the second.
   const int4* __restrict__ pp = (SB ? A.pos1 : A.pos0) + R.b0;
   const int n = R.total(), n0 = R.n0, d1 = (int)(R.b1 - R.b0);
   u64* const fold = reinterpret_cast<u64*>((SB ? A.pos0 : A.pos1) + L.base);
-  const int nit = (n + DEP_THREADS - 1) / DEP_THREADS;
-  int k = threadIdx.x;
-  constexpr int DEPTH = PM_DEP_DEPTH;
-  int4 q[DEPTH];  // the particles of the next DEPTH sweeps, loads in flight
-#pragma unroll
-  for (int d = 0; d < DEPTH; ++d) {
-    const int kk = k + d * DEP_THREADS;
-    q[d] = kk < n ? pp[kk < n0 ? kk : kk + d1] : make_int4(-1, 0, 0, 0);
+  if (threadIdx.x == 0) {
+    prefetch_l2(pp, n0);
+    prefetch_l2(pp + n0 + d1, n - n0);
   }
   bool bad = false;
-  int left = CH_IT;
-  for (int it = 0; it < nit; ++it) {
-    const int4 ps = q[0];
-    const bool valid = k < n;
-#pragma unroll
-    for (int d = 0; d + 1 < DEPTH; ++d) q[d] = q[d + 1];
-    const int kn = k + DEPTH * DEP_THREADS;
-    if (kn < n) q[DEPTH - 1] = pp[kn < n0 ? kn : kn + d1];
-    k += DEP_THREADS;
-    {
+  for (int c0 = 0; c0 < n; c0 += CH_IT * DEP_THREADS) {  // chunks; almost always one
+    if (c0) {  // fold the chunk before into `fold`
+      __syncthreads();
+      fold_chunk<TS>(fold, acc_hi, acc_lo, folded);
+      folded = true;
+      __syncthreads();
+    }
+    const int c1 = min(n, c0 + CH_IT * DEP_THREADS);
+    int k = c0 + threadIdx.x;
+    int4 next = make_int4(0, 0, 0, 0);  // the next sweep's particle, its load in flight
+    if (k < c1) next = pp[k < n0 ? k : k + d1];
+    while (k < c1) {
+      const int4 ps = next;
+      k += DEP_THREADS;
+      if (k < c1) next = pp[k < n0 ? k : k + d1];
       const int c = ps.x;
-      const bool in = valid && (c & ~local) == tile_bits;
-      bad |= valid && !in;
       const double one = (double)PM_FIX_ONE;
       const double fx = __int_as_float(ps.y), fy = __int_as_float(ps.z), fz = __int_as_float(ps.w);
       const double Fx = fx * one, Gx = one - Fx;   // exact: fx has 24 significant bits
       const double gy = 1.0 - fy, gz = 1.0 - fz;
       const double w00 = Gx * gy, w01 = Gx * fy, w10 = Fx * gy, w11 = Fx * fy;
       // Seven corners rounded to integers in units of 2^-38; the eighth takes the remainder so
-      // the particle deposits exactly 2^38 (hi/lo of 2^38 - sum, with lo in [0, 2^19)).
-      const Split c0 = fix_split(w00, gz), c1 = fix_split(w00, fz), c2 = fix_split(w01, gz), c3 = fix_split(w01, fz),
-                  c4 = fix_split(w10, gz), c5 = fix_split(w10, fz), c6 = fix_split(w11, gz);
-      const u32 shi = c0.hi + c1.hi + c2.hi + c3.hi + c4.hi + c5.hi + c6.hi;
-      const u32 slo = c0.lo + c1.lo + c2.lo + c3.lo + c4.lo + c5.lo + c6.lo;
-      const Split c7{(1u << 19) - shi - ((slo + 0x7FFFFu) >> 19), (0u - slo) & 0x7FFFFu};
-      const Split w[8] = {c0, c1, c2, c3, c4, c5, c6, c7};
-      if (in) {
+      // the particle deposits exactly 2^38 (0 modulo 2^32).
+      Split w[8] = {fix_split(w00, gz), fix_split(w00, fz), fix_split(w01, gz), fix_split(w01, fz),
+                    fix_split(w10, gz), fix_split(w10, fz), fix_split(w11, gz), fix_split(w11, fz)};
+      w[7].lo = 0u - (w[0].lo + w[1].lo + w[2].lo + w[3].lo + w[4].lo + w[5].lo + w[6].lo);
+      if ((c & ~local) == tile_bits) {
         const int nb = ((c >> (2 * l2)) & (TS - 1)) * PS + ((c >> l2) & (TS - 1)) * RS + (c & (TS - 1));
         const int off[8] = {0, 1, RS, RS + 1, PS, PS + 1, PS + RS, PS + RS + 1};
 #pragma unroll
@@ -1205,71 +1271,46 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
           atomicAdd(&acc_hi[nb + off[q]], w[q].hi);
           atomicAdd(&acc_lo[nb + off[q]], w[q].lo);
         }
+      } else {
+        bad = true;
       }
-    }
-    if (--left == 0 && it + 1 < nit) {  // chunk full and more to come: fold it into acc64
-      left = CH_IT;
-      __syncthreads();
-      fold_chunk<TS>(fold, acc_hi, acc_lo, folded);
-      folded = true;
-      __syncthreads();
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&A.stats[pk].status, 1u);
-  // Write-out of the last chunk (plus the folded ones), four nodes of a patch row at a time:
-  // interior nodes final as FP32 delta (16-byte stores; the first node of an interior row is a
-  // face node, stored here from this super-tile's own sum and completed by k_fixup), nodes on
-  // the lower faces and on the upper halo as 64-bit partials.
-  long long dsum = 0, smax = 0;
+  // Write-out of the last chunk (plus the folded ones).  First the TS^3 nodes of the super-tile,
+  // four of a row at a time: interior nodes final as FP32 delta (16-byte stores; the first node
+  // of an interior row is a face node, stored here from this super-tile's own sum and completed by
+  // k_fixup), nodes on the lower faces as 64-bit partials; then the upper halo, partials in their
+  // storage order.
   const long long gbase = ((long long)sx * TS * N + (long long)sy * TS) * N + sz * TS;
   long long* face = A.face + P.face_off + (long long)st * FC;
   long long* halo = A.halo + P.halo_off + (long long)st * P.hc;
   const long long nmf = P.n_mean_fix;
   const double inv = P.inv_fix_nmean;
-  for (int item = threadIdx.x; item < T1 * T1 * NG; item += DEP_THREADS) {
-    const int row = item / NG, g = item - row * NG;
-    const int lx = row / T1, ly = row - lx * T1;
-    const int ad = lx * PS + ly * RS + 4 * g;
-    const uint4 h = *reinterpret_cast<const uint4*>(acc_hi + ad);
-    const uint4 l = *reinterpret_cast<const uint4*>(acc_lo + ad);
-    long long S[4] = {chunk_sum(h.x, l.x), chunk_sum(h.y, l.y), chunk_sum(h.z, l.z), chunk_sum(h.w, l.w)};
-    const int nbase = row * T1 + 4 * g;  // dense node number of the group's first node
-    if (folded) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (4 * g + k <= TS) S[k] += (long long)fold[nbase + k];
+  long long dsum, smax;
+  if (folded || rho64 || nmf >= (1LL << 48))
+    write_nodes<TS, true>(acc_hi, acc_lo, folded ? fold : nullptr, P.delta + gbase, rho64 ? rho64 + gbase : nullptr,
+                          face, N, nmf, inv, dsum, smax);
+  else
+    write_nodes<TS, false>(acc_hi, acc_lo, nullptr, P.delta + gbase, nullptr, face, N, nmf, inv, dsum, smax);
+  {
+    // The three upper planes: their TS x TS parts with coordinates from shifts, then the 3 TS + 1
+    // nodes of their common edges.
+    auto put = [&](int lx, int ly, int lz) {
+      const int ad = lx * PS + ly * RS + lz;
+      long long S = chunk_sum(acc_hi[ad], acc_lo[ad]);
+      if (folded) S += (long long)fold[(lx * T1 + ly) * T1 + lz];
+      halo[halo_index(lx, ly, lz, TS)] = S;
+    };
+    for (int f = threadIdx.x; f < TS * TS; f += DEP_THREADS) {
+      const int u = f / TS, v = f % TS;
+      put(TS, u, v);
+      put(u, TS, v);
+      put(u, v, TS);
     }
-    if (lx == TS || ly == TS) {  // a row of the upper halo
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int lz = 4 * g + k;
-        if (lz <= TS) halo[halo_index(lx, ly, lz, TS)] = S[k];
-      }
-    } else if (g == NG - 1) {    // the row's upper-halo node
-      halo[halo_index(lx, ly, TS, TS)] = S[0];
-    } else if (lx == 0 || ly == 0) {  // a row of a lower face
-#pragma unroll
-      for (int k = 0; k < 4; ++k) face[face_index(lx, ly, 4 * g + k, TS)] = S[k];
-    } else {                     // interior nodes (and the row's lz = 0 face node)
-      if (g == 0) face[face_index(lx, ly, 0, TS)] = S[0];
-      float4 d;
-      float* dv = &d.x;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const long long D = S[k] - nmf;
-        dv[k] = (float)((double)D * inv);
-        if (g > 0 || k > 0) {
-          dsum += D;
-          smax = S[k] > smax ? S[k] : smax;
-        }
-      }
-      const long long gi = gbase + ((long long)lx * N + ly) * N + 4 * g;
-      *reinterpret_cast<float4*>(P.delta + gi) = d;
-      if (rho64) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (g > 0 || k > 0) rho64[gi + k] = (double)S[k] * (1.0 / (double)PM_FIX_ONE);
-      }
+    for (int f = threadIdx.x; f < 3 * TS + 1; f += DEP_THREADS) {
+      const int e = f / TS, u = f % TS;  // e = 3: the corner
+      put(e == 0 ? u : TS, e == 1 ? u : TS, e == 2 ? u : TS);
     }
   }
   for (int d = 16; d > 0; d >>= 1) {
@@ -1294,46 +1335,69 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
 }
 
 
-__global__ void __launch_bounds__(DEP_THREADS, 4) k_deposit(StepArgs A, double* rho64) {
+__global__ void __launch_bounds__(DEP_THREADS, 4)
+    k_deposit(const __grid_constant__ StepArgs A, double* rho64, int only) {
   extern __shared__ __align__(16) u32 s_dep[];
-  const TileRef tr = find_tile(A.st_base, A.st_peak);
-  const PeakClock C = A.clocks[tr.pk];
-  if (!C.dep) return;
+  const TileRef tr = find_tile(A.st_ref);
   const PeakDesc P = A.peaks[tr.pk];
+  {  // clear the accumulators
+    const int words = 2 * (P.TS == 4 ? patch_size(4) : P.TS == 8 ? patch_size(8) : patch_size(16));
+    static_assert((2 * patch_size(4)) % 4 == 0 && (2 * patch_size(8)) % 4 == 0 && (2 * patch_size(16)) % 4 == 0, "");
+    for (int i = threadIdx.x; i < words / 4; i += DEP_THREADS)
+      reinterpret_cast<uint4*>(s_dep)[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  pdl_wait();
+  // The plan and both candidates of the bin's layout and fill in one round trip (as in k_push).
+  const u32 flags = __ldcg(&A.plan[tr.pk].flags);
+  const int4 F0 = __ldcg(reinterpret_cast<const int4*>(A.fill[0] + blockIdx.x)),
+             F1 = __ldcg(reinterpret_cast<const int4*>(A.fill[1] + blockIdx.x));
+  const int2 L0 = __ldcg(reinterpret_cast<const int2*>(A.lay[0] + blockIdx.x)),
+             L1 = __ldcg(reinterpret_cast<const int2*>(A.lay[1] + blockIdx.x));
+  const bool sb = flags & PLAN_SBUF;
+  const int4 f = sb ? F1 : F0;
+  const int2 l = flags & PLAN_LGEN ? L1 : L0;
+  const BinFill F{(u32)f.x, (u32)f.y, (u32)f.z, 0u};
+  const BinLayout L{(u32)l.x, (u32)l.y};
+  if (only < 0 ? !(flags & PLAN_DEP) : tr.pk != only) return;
+  const u32 st = (u32)tr.t;
   switch (P.TS) {
     // The bin buffer as a template argument: its pointers are then kernel parameters, not a
     // per-thread select (the particle loop is register-bound).
     case 4:
-      if (C.sbuf) deposit_super<4, 1>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
-      else deposit_super<4, 0>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
+      if (sb) deposit_super<4, 1>(A, P, tr.pk, st, L, F, s_dep, rho64);
+      else deposit_super<4, 0>(A, P, tr.pk, st, L, F, s_dep, rho64);
       break;
     case 8:
-      if (C.sbuf) deposit_super<8, 1>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
-      else deposit_super<8, 0>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
+      if (sb) deposit_super<8, 1>(A, P, tr.pk, st, L, F, s_dep, rho64);
+      else deposit_super<8, 0>(A, P, tr.pk, st, L, F, s_dep, rho64);
       break;
     default:
-      if (C.sbuf) deposit_super<16, 1>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
-      else deposit_super<16, 0>(A, P, C, tr.pk, (u32)tr.t, s_dep, rho64);
+      if (sb) deposit_super<16, 1>(A, P, tr.pk, st, L, F, s_dep, rho64);
+      else deposit_super<16, 0>(A, P, tr.pk, st, L, F, s_dep, rho64);
       break;
   }
 }
 
 // Face fix-up: one CTA per super-tile whose peak deposited this step.  Small and
 // latency-bound, so many CTAs per SM.
-__global__ void __launch_bounds__(FIX_THREADS) k_fixup(StepArgs A, double* rho64) {
+__global__ void __launch_bounds__(FIX_THREADS) k_fixup(const __grid_constant__ StepArgs A, double* rho64, int only) {
   __shared__ long long s_red[FIX_THREADS / 32];
   __shared__ long long s_max[FIX_THREADS / 32];
   __shared__ const long long* s_nb[8];
-  const TileRef tr = find_tile(A.st_base, A.st_peak);
-  const PeakClock C = A.clocks[tr.pk];
-  if (!C.dep) return;
+  const TileRef tr = find_tile(A.st_ref);
+  pdl_wait();
+  const u32 flags = __ldcg(&A.plan[tr.pk].flags);
   const PeakDesc P = A.peaks[tr.pk];
+  if (only < 0 ? !(flags & PLAN_DEP) : tr.pk != only) return;
   const u32 Y = (u32)tr.t;
   if (threadIdx.x == 0) {
     // Ready for the next push, which fills the other buffer: no arrivals yet, overflow area
     // empty.  (Here rather than in the deposit, whose particle loop is register-bound.)
-    bfill(A, C.sbuf ^ 1)[P.st_base + Y].moved = 0u;
-    if (Y == 0) A.ovf_n[tr.pk] = 0u;
+    bfill(A, flags & PLAN_SBUF ? 0 : 1)[blockIdx.x].moved = 0u;
+    if (Y == 0) {
+      A.ovf_n[tr.pk] = 0u;
+      *A.sort_gate = *A.layout_gate = *A.refresh_gate = 0u;  // this step's gated kernels have run
+    }
   }
   if (threadIdx.x < 8) {
     const int o = threadIdx.x, NS = P.NS;
@@ -1442,6 +1506,7 @@ __device__ __forceinline__ double green_mode(const GreenCtx& g, long long m, flo
 __global__ void __launch_bounds__(PM_THREADS) k_green(StepArgs A) {
   __shared__ int s_pk;
   __shared__ long long s_lb;
+  pdl_wait();
   if (threadIdx.x == 0) {
     const int gi = pm_find(A.green_base, A.ngreen, (long long)blockIdx.x);
     s_pk = A.green_peak[gi];
@@ -1511,6 +1576,7 @@ __global__ void k_reset_peak(StepArgs A, int pk, double a0, int mode, double par
   else if (mode == SCHED_FRAC) c.da = fmin(param * a0, a_end - a0);
   else c.da = 0.0;
   A.clocks[pk] = c;
+  A.plan[pk] = plan_of(c, A.peaks[pk]);
   A.stats[pk].status = 0;
   A.stats[pk].nsamples = 0;
   A.stats[pk].relayouts = 0;
@@ -1525,6 +1591,12 @@ __global__ void k_release_peak(StepArgs A, int pk) {
   c.dep = 0;
   c.kpend = 0.0;
   A.clocks[pk] = c;
+  A.plan[pk] = plan_of(c, A.peaks[pk]);
+}
+
+__global__ void k_write_clock(StepArgs A, int pk, PeakClock c) {
+  A.clocks[pk] = c;
+  A.plan[pk] = plan_of(c, A.peaks[pk]);
 }
 
 // Particles (n,3) float64 in lattice order -> split state + cell keys (pm3d.py:76-79 convention).
@@ -1742,11 +1814,10 @@ static unsigned stride_grid(long long n, int t, int per_sm) {
 }
 
 void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s) {
-  k_push<<<(unsigned)nst, PUSH_THREADS, smem, s>>>(A);
+  pdl_launch(k_push, dim3((unsigned)nst), PUSH_THREADS, smem, s, A);
 }
-void launch_advance(const StepArgs& A, cudaStream_t s) { k_advance<<<1, 256, 0, s>>>(A); }
-void launch_energy(const StepArgs& A, cudaStream_t s) {
-  k_energy<<<dim3(ENERGY_SLICES, A.npeaks), PM_THREADS, 0, s>>>(A);
+void launch_tick(const StepArgs& A, cudaStream_t s) {
+  pdl_launch(k_tick, dim3(A.eslices + 1, A.npeaks), LAYOUT_THREADS, 0, s, A);
 }
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s) {
   k_permute<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A, ntot);
@@ -1755,25 +1826,27 @@ void launch_st_starts(const StepArgs& A, long long ntot, cudaStream_t s) {
   k_st_starts<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A, ntot);
 }
 void launch_tile_sort(const StepArgs& A, long long nst, cudaStream_t s) {
-  k_tile_sort<<<stride_grid(nst, 1, 1), TSORT_THREADS, pm_tile_sort_smem(), s>>>(A, nst);
+  pdl_launch(k_tile_sort, dim3(stride_grid(nst, 1, 1)), TSORT_THREADS, pm_tile_sort_smem(), s, A, nst);
 }
-void launch_layout(const StepArgs& A, long long nst, long long ntot, cudaStream_t s) {
-  k_layout<<<(unsigned)A.npeaks, LAYOUT_THREADS, 0, s>>>(A);
-  k_relayout_copy<<<dim3(RELAYOUT_COPY_BLOCKS, (unsigned)A.npeaks), PM_THREADS, 0, s>>>(A);
-  k_relayout_ovf<<<dim3(RELAYOUT_OVF_BLOCKS, (unsigned)A.npeaks), PM_THREADS, 0, s>>>(A);
+void launch_layout(const StepArgs& A, cudaStream_t s) { k_layout<<<(unsigned)A.npeaks, LAYOUT_THREADS, 0, s>>>(A); }
+void launch_relayout(const StepArgs& A, long long nst, cudaStream_t s) {
+  pdl_launch(k_relayout, dim3(stride_grid(nst, 1, RELAYOUT_CTAS_PER_SM)), PM_THREADS, 0, s, A);
 }
-void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, cudaStream_t s) {
-  k_deposit<<<(unsigned)nst, DEP_THREADS, smem, s>>>(A, rho64);
+void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, int only, cudaStream_t s) {
+  pdl_launch(k_deposit, dim3((unsigned)nst), DEP_THREADS, smem, s, A, rho64, only);
 }
-void launch_fixup(const StepArgs& A, long long nst, double* rho64, cudaStream_t s) {
-  k_fixup<<<(unsigned)nst, FIX_THREADS, 0, s>>>(A, rho64);
+void launch_fixup(const StepArgs& A, long long nst, double* rho64, int only, cudaStream_t s) {
+  pdl_launch(k_fixup, dim3((unsigned)nst), FIX_THREADS, 0, s, A, rho64, only);
 }
 void launch_green(const StepArgs& A, long long nblocks, cudaStream_t s) {
-  k_green<<<(unsigned)nblocks, PM_THREADS, 0, s>>>(A);
+  pdl_launch(k_green, dim3((unsigned)nblocks), PM_THREADS, 0, s, A);
 }
 void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double param, double a_end,
                        int max_steps, int set_thr, double delta_collapse, int stop, cudaStream_t s) {
   k_reset_peak<<<1, 1, 0, s>>>(A, pk, a0, mode, param, a_end, max_steps, set_thr, delta_collapse, stop);
+}
+void launch_write_clock(const StepArgs& A, int pk, const PeakClock& c, cudaStream_t s) {
+  k_write_clock<<<1, 1, 0, s>>>(A, pk, c);
 }
 void launch_release_peak(const StepArgs& A, int pk, cudaStream_t s) { k_release_peak<<<1, 1, 0, s>>>(A, pk); }
 void launch_set_particles(const StepArgs& A, int pk, const PeakDesc& P, const double* x, const double* p,

@@ -28,7 +28,8 @@
 #define PUSH_THREADS 512
 #define DEP_THREADS 256    // deposit CTA (4 per SM)
 #define GREEN_MODES 4      // modes per thread of the Green kernel (a block covers PM_THREADS * GREEN_MODES)
-#define ENERGY_SLICES 16   // CTAs per peak of the energy reduction
+#define ENERGY_SLICES 128  // most CTAs per peak of the energy reduction
+#define ENERGY_THREADS 256 // threads of them that work
 #define FIX_THREADS 256    // face fix-up CTA
 #define TSORT_THREADS 1024 // super-tile sort (refresh) CTA
 #define TSORT_CAP 5120     // particles of a super-tile sorted in shared memory; denser ones via global
@@ -50,8 +51,7 @@
 #define BIN_SLACK_MIN 32
 #define BIN_ALIGN 8        // bin bases and capacities are multiples of 8 slots (128 bytes)
 #define LAYOUT_THREADS 1024
-#define RELAYOUT_OVF_BLOCKS 32  // CTAs per peak placing a relayout's overflow area
-#define RELAYOUT_COPY_BLOCKS 256  // CTAs per peak moving a relayout's bins
+#define RELAYOUT_CTAS_PER_SM 4  // grid of the relayout copies
 
 // Fill of one bin in one buffer: the stayers occupy [base, base + stay), the arrivals
 // [base + gap, base + gap + min(moved, cap - gap)); gap is the bin's count before the push
@@ -69,12 +69,13 @@ struct StepArgs {
   const PeakDesc* peaks;
   PeakClock* clocks;
   PeakStats* stats;
-  SortSeg* sortseg;            // sort activity flags, written by the advance kernel
-  u32* sort_gate;              // 1 when any peak primes by sort this step (advance kernel)
-  u32* layout_gate;            // 1 when any peak primes or relayouts this step (advance kernel)
-  u32* refresh_gate;           // 1 when any peak re-sorts its super-tiles this step (advance kernel)
+  SortSeg* sortseg;            // sort activity flags, written by k_tick
+  u32* sort_gate;              // 1 when any peak primes by sort this step (k_tick)
+  u32* layout_gate;            // 1 when any peak primes or relayouts this step (k_tick)
+  u32* refresh_gate;           // 1 when any peak re-sorts its super-tiles this step (k_tick)
   const long long* st_base;    // [npeaks + 1] prefix of super-tiles
-  const unsigned short* st_peak;  // [super-tile] its peak (one load instead of a search)
+  const int2* st_ref;          // [super-tile] {its peak, its index in the peak} (one load instead of a search)
+  PeakPlan* plan;              // [peak] digest of the clock (see PeakPlan)
   const long long* p_base;     // [npeaks + 1] prefix of particles
   const long long* mode_base;  // [npeaks + 1] prefix of Green blocks
   const long long* green_base; // [ngreen + 1] prefix of Green blocks over the peaks k_green serves
@@ -91,6 +92,7 @@ struct StepArgs {
   BinFill* fill[2];            // [super-tile] bin fills of buffers 0 and 1
   u32* ovf_n;                  // [peak] particles in the overflow area (push), reset by the deposit
   u32* ovf_in;                 // [super-tile] overflowed particles whose destination it is
+  u32* new_count;              // [super-tile] particles after a relayout
   u32* keys_push;              // Morton keys written by set_particles / reload (priming sort input)
   const u32* keys_sorted;      // sort output keys
   const u32* perm;             // sort output permutation
@@ -101,6 +103,8 @@ struct StepArgs {
   double* wpart;               // [Green block][warp] partials of sum_k w_k |delta_k|^2 G_k
   double2* eslice;             // [peak][ENERGY_SLICES][5] slice partials of the energy kernel
   u32* ecount;                 // [peak] energy slices finished this step (0 between steps)
+  int eslices;                 // energy CTAs per peak
+  double* pushed_a;            // [peak] expansion factor the push started from, -1 when it did not push
   int* sort_err;               // [peak] the priming sort's bounded look-back gave up (sort plan)
 };
 
@@ -119,21 +123,22 @@ size_t pm_deposit_smem(int TSmax);
 size_t pm_push_smem(int TSmax);
 
 void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s);
-void launch_advance(const StepArgs& A, cudaStream_t s);
-void launch_energy(const StepArgs& A, cudaStream_t s);
+void launch_tick(const StepArgs& A, cudaStream_t s);
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_st_starts(const StepArgs& A, long long ntot, cudaStream_t s);
-// Bin layouts of the priming and relayout peaks, then the relayout's copies (gated launches).
-void launch_layout(const StepArgs& A, long long nst, long long ntot, cudaStream_t s);
+void launch_layout(const StepArgs& A, cudaStream_t s);                     // priming peaks
+void launch_relayout(const StepArgs& A, long long nst, cudaStream_t s);    // gated
 void launch_tile_sort(const StepArgs& A, long long nst, cudaStream_t s);
-void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, cudaStream_t s);
-void launch_fixup(const StepArgs& A, long long nst, double* rho64, cudaStream_t s);
+// only >= 0: deposit that peak alone, whether or not its clock asks for it.
+void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, int only, cudaStream_t s);
+void launch_fixup(const StepArgs& A, long long nst, double* rho64, int only, cudaStream_t s);
 void launch_green(const StepArgs& A, long long nblocks, cudaStream_t s);
 
 // The native Poisson solve of 32^3 to 512^3 meshes and plain transforms of 64^3 to 512^3
 // (native_fft.cu).  fft_native_init: once per device before use.
 bool fft_native_size(int N);
 bool fft_solve_size(int N);
+long long fft_solve_partials(int N);
 int fft_native_init();
 int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
                      const int* slot_peak, int nslots, cudaStream_t s);
@@ -142,6 +147,8 @@ int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, flo
 // cleared; set_thr = 1 also sets the collapse threshold and its stop flag (else they are kept).
 void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double param, double a_end,
                        int max_steps, int set_thr, double delta_collapse, int stop, cudaStream_t s);
+// write_clock: the host's clock for a peak, on the stream.
+void launch_write_clock(const StepArgs& A, int pk, const PeakClock& c, cudaStream_t s);
 // release: the peak goes idle (no pending kick, no grids), on the stream, without a host round trip.
 void launch_release_peak(const StepArgs& A, int pk, cudaStream_t s);
 void launch_set_particles(const StepArgs& A, int pk, const PeakDesc& P, const double* x, const double* p,
