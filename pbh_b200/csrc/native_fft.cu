@@ -18,7 +18,11 @@
 // every exchange hit distinct shared-memory banks within each half-warp (for the 64^3 Z pass,
 // at most two-way).
 //
-// The engine's Poisson solve (delta -> three force grids) is five launches:
+// The engine's Poisson solve (delta -> three force grids).  The inverse along x comes first, so the
+// x transform, the Green multiply and the inverse x transform of a column need no pass over
+// memory between them; and because the y and z gradients multiply by factors that do not depend on
+// kx, only two fields leave that pass (A = -i G delta_k and B = g(kx) A; the y and z components are
+// g(ky) A and g(kz) A, multiplied where A is next read) instead of three.  256^3 and 512^3:
 //   k_fft_z_r2c   a real FFT along z of CTA/T consecutive (x, y) lines per CTA (T = N/32): a complex
 //                 FFT of the N/2 packed (even, odd) pairs, then the split into N/2+1 outputs,
 //                 written transposed into the kz planes
@@ -26,15 +30,16 @@
 //   k_solve_cols  per column of a plane: forward X, the Green multiply, inverse X of two fields
 //   k_solve_rows  inverse Y of the three components
 //   k_fft_z_c2r   the real inverse along z of the three components, written as force rows
-// The inverse along x comes first, so the x transform, the Green multiply and the inverse x
-// transform of a column need no pass over memory between them; and because the y and z
-// gradients multiply by factors that do not depend on kx, only two fields leave that pass
-// (A = -i G delta_k and B = g(kx) A; the y and z components are g(ky) A and g(kz) A, multiplied
-// where A is next read) instead of three.  Per cell the passes move 8 + 8 + 12 + 20 + 24 = 72 bytes;
-// the six passes this replaced (Y before X on the way back) moved 88 and did the multiply once per
-// component: 296 -> 244 us at 256^3, 2431 -> 2062 at 512^3, 72 -> 55 at 128^3 (events around the
-// whole solve), with the same errors against float64.  HBM bounds the row and Z passes (5.1-6.9
-// TB/s of these bytes at 256^3); the column pass (55 us for 202 MB) waits on its exchanges.
+// Up to 128^3 the y-z slab of one x fits an SM:
+//   k_slab_fwd    Z and Y of a slab
+//   k_solve_cols  as above
+//   k_slab_inv    inverse Y and Z of a slab, one component
+// Per cell the five passes move 8 + 8 + 12 + 20 + 24 = 72 bytes, the three 8 + 12 + 20 = 40; the six
+// passes they replace (Y before X on the way back) moved 88 and did the multiply once per
+// component.  Whole solve by events, six passes, five, three: 296, 244, - us at 256^3; 2431, 2062, -
+// at 512^3; 72, 47, 43 at 128^3; 42, 25, 22 at 64^3 (eight of them: -, 55, 46).  Errors against
+// float64 are the same.  HBM bounds the row and Z passes (5.1-6.9 TB/s of these bytes at 256^3);
+// the column pass (55 us for 202 MB) waits on its exchanges.
 // Chaining the plane passes in one persistent kernel, plane by plane so that L2 holds a plane from
 // pass to pass, was slower (350 us at 256^3: its item claims, waits and fences cost more than
 // the HBM traffic they save).
@@ -150,8 +155,9 @@ __device__ __forceinline__ int line_slot(int k1, int t) {
 // x[T n1 + t] on entry and u[p] = X[line_k<T>(t, p)] on exit.  row: the line's exchange row in
 // shared memory (16 T values); tl: W_L^{t k1} at [k1 * T + t] (the forward ones, conjugated here
 // for the inverse).  The threads of a line are
-// consecutive lanes of one warp (T = 32: the whole warp).  Ends after the exchange has been read:
-// the caller must barrier before it writes the row again.
+// consecutive lanes of one warp (T = 32: the whole warp), so the exchange needs no CTA barrier; the
+// rows must not overlap.  Ends after the exchange has been read: the caller synchronizes the warp
+// before it writes the row again.
 template <bool INV>
 __device__ __forceinline__ float2 twc(float2 w) { return INV ? cconj(w) : w; }
 
@@ -163,7 +169,7 @@ __device__ __forceinline__ void line_fft(float2 (&v)[16], float2 (&u)[16], float
     const int k1 = brev(p, 4);
     row[line_slot<T>(k1, t)] = k1 ? cmul(v[p], twc<INV>(tl[k1 * T + t])) : v[p];
   }
-  __syncthreads();
+  __syncwarp();  // the T threads of a line are lanes of one warp
   if constexpr (T <= 16) {
     // this thread's k1 = t + T s, s < 16 / T: one T-point DFT each
 #pragma unroll
@@ -245,7 +251,7 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_z_r2c(const f
   __syncthreads();  // tables
   float2* row = xb + l * G::X;
   line_fft<false, G::T>(v, u, row, tl, t);
-  __syncthreads();
+  __syncwarp();
   // Z_k into the line's row in natural order, swizzled so that the column reads below are
   // conflict-free: Z_k at row[k ^ sw(l)].
   const int sw = G::sw(l);
@@ -541,6 +547,149 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>())
   for (int p = 0; p < 16; ++p) dst[line_k<T>(t, p)] = u[p];
 }
 
+// ------------------------------------------------------------------------------------------
+// Meshes up to 128^3: the y and z transforms of one x slab in one kernel, the slab (NH x N complex,
+// 70 KB at 128^3) in shared memory between them.  Three launches a solve instead of five, and per
+// cell 8 + 12 + 20 bytes instead of 72.  A larger slab does not fit an SM.
+template <int N>
+struct SGeo {
+  static constexpr int M = N / 2, NH = M + 1, TZ = M / 16, TY = N / 16;
+  static constexpr int THREADS = (NH * TY + 31) / 32 * 32;  // one thread per 16 elements of a (kz) line
+  static_assert(N * TZ <= THREADS, "a thread per 16 pairs of a z line");
+  static constexpr int X = M + TZ;   // row stride (float2) of the z lines
+  static constexpr int C = N + TY;   // row stride of the kz lines
+  static constexpr int BUF = NH * C > N * X ? NH * C : N * X;
+  static constexpr size_t SMEM = sizeof(float2) * (BUF + 16 * TZ + 16 * TY + M + 1);
+  static constexpr int MINB = N == 128 ? 2 : 4;  // CTAs per SM
+  // The inverse runs at 64 registers; two CTAs of 128^3 then have 512 threads each, and its one line
+  // too many takes a second round.
+  static constexpr int ITHREADS = N == 128 ? 512 : THREADS;
+  static constexpr long long N2 = (long long)N * N;
+};
+template <bool INV, int N, int THREADS>
+__device__ __forceinline__ void load_slab_tw(float2* tz, float2* ty, float2* tw) {
+  using G = SGeo<N>;
+  for (int i = threadIdx.x; i < 16 * G::TZ; i += THREADS) tz[i] = tw_global<false, G::M>((i / G::TZ) * (i % G::TZ));
+  for (int i = threadIdx.x; i < 16 * G::TY; i += THREADS) ty[i] = tw_global<false, N>((i / G::TY) * (i % G::TY));
+  for (int i = threadIdx.x; i <= G::M; i += THREADS) tw[i] = tw_global<INV, N>(i);
+}
+
+// Forward: densities in[slot][x][y][z] -> spectra out[slot][kz][x][ky].  grid (N, nslots).
+template <int N>
+__global__ void __launch_bounds__(SGeo<N>::THREADS, SGeo<N>::MINB)
+    k_slab_fwd(const float* in, float2* out, const __grid_constant__ StepArgs A, const int* slot_peak) {
+  using G = SGeo<N>;
+  extern __shared__ __align__(16) float2 s_slab[];
+  float2 *const xb = s_slab, *const tz = xb + G::BUF, *const ty = tz + 16 * G::TZ, *const tw = ty + 16 * G::TY;
+  load_slab_tw<false, N, G::THREADS>(tz, ty, tw);
+  const int x = blockIdx.x, slot = blockIdx.y;
+  pdl_wait();
+  if (!slot_active(A, slot_peak, slot)) return;
+  float2 v[16], u[16];
+  const int tid = threadIdx.x;
+  const bool zt = tid < N * G::TZ;  // whole warps
+  const int t = tid % G::TZ, y = tid / G::TZ;
+  if (zt) {
+    const float2* src = reinterpret_cast<const float2*>(in + ((long long)slot * N + x) * G::N2 + y * N);
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = __ldcg(src + G::TZ * n1 + t);
+  }
+  __syncthreads();  // tables
+  if (zt) {
+    float2* const row = xb + y * G::X;
+    line_fft<false, G::TZ>(v, u, row, tz, t);
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) row[line_k<G::TZ>(t, p)] = u[p];
+  }
+  __syncthreads();
+  // Line kz: X_k = E_k + W_N^k O_k of every row, E = (Z_k + conj Z_{M-k})/2, O = -i (Z_k - conj Z_{M-k})/2
+  // (threads beyond the last line repeat it)
+  const int k = min(tid / G::TY, G::M), ty_ = tid % G::TY;
+  const float2 wk = tw[k];
+#pragma unroll
+  for (int n1 = 0; n1 < 16; ++n1) {
+    const float2* zr = xb + (G::TY * n1 + ty_) * G::X;
+    const float2 zk = zr[k & (G::M - 1)], zm = cconj(zr[(G::M - k) & (G::M - 1)]);
+    const float2 E = cscale(cadd(zk, zm), 0.5f), O = cscale(mul_w4<false>(csub(zk, zm)), 0.5f);
+    v[n1] = cadd(E, cmul(wk, O));
+  }
+  __syncthreads();  // the z lines are read; their memory becomes the exchange rows
+  line_fft<false, G::TY>(v, u, xb + k * G::C, ty, ty_);
+  if (tid / G::TY > G::M) return;
+  float2* dst = out + ((long long)slot * G::NH + k) * G::N2 + x * N;
+#pragma unroll
+  for (int p = 0; p < 16; ++p) dst[line_k<G::TY>(ty_, p)] = u[p];
+}
+
+// Inverse of one component: the x component from B (gspec's first field), y and z from A (spec) times
+// their gradient factors -> force grids out[slot][comp][x][y][z].  The three components of a slab
+// are adjacent in the grid, so that A is read from HBM once.  grid (3 N, nslots).
+template <int N>
+__global__ void __launch_bounds__(SGeo<N>::ITHREADS, SGeo<N>::MINB)
+    k_slab_inv(const float2* spec, const float2* gspec, float* out, const __grid_constant__ StepArgs A,
+               const int* slot_peak) {
+  using G = SGeo<N>;
+  extern __shared__ __align__(16) float2 s_slab[];
+  float2 *const xb = s_slab, *const tz = xb + G::BUF, *const ty = tz + 16 * G::TZ, *const tw = ty + 16 * G::TY;
+  load_slab_tw<true, N, G::ITHREADS>(tz, ty, tw);
+  const int comp = blockIdx.x % 3, x = blockIdx.x / 3, slot = blockIdx.y;
+  const int tid = threadIdx.x, ty_ = tid % G::TY;
+  const PeakDesc& P = A.peaks[slot_peak[slot]];
+  const float kf = (float)(2.0 * M_PI / P.L);
+  const float* const gtab = P.gtab;
+  pdl_wait();
+  if (!slot_active(A, slot_peak, slot)) return;
+  __syncthreads();  // tables
+  float2 v[16], u[16];
+  const float2* src = (comp == 0 ? gspec + (long long)3 * slot * G::NH * G::N2 : spec + (long long)slot * G::NH * G::N2) + x * N;
+  // Whole warps take part; threads beyond the last line repeat it.
+#pragma unroll 1
+  for (int l0 = (tid & ~31) / G::TY; l0 <= G::M; l0 += G::ITHREADS / G::TY) {
+    const int k = min(l0 + (tid & 31) / G::TY, G::M);
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = src[k * (int)G::N2 + G::TY * n1 + ty_];
+    if (comp == 1) {
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = cscale(v[n1], gfac<N>(G::TY * n1 + ty_, kf, gtab));
+    } else if (comp == 2) {
+      const float gz = gtab ? __ldg(gtab + k) : kf * (float)k;
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = cscale(v[n1], gz);
+    }
+    float2* const line = xb + k * G::C;
+    line_fft<true, G::TY>(v, u, line, ty, ty_);
+    __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 16; ++p) line[line_k<G::TY>(ty_, p)] = u[p];
+  }
+  __syncthreads();
+  // Row y: Z_n = E_n + i O_n with E = X_n + conj X_{M-n}, O = (X_n - conj X_{M-n}) W_N^{-n}; only the
+  // real parts of X_0 and X_M count (see k_fft_z_c2r).
+  const bool zt = tid < N * G::TZ;  // whole warps
+  const int t = tid % G::TZ, y = tid / G::TZ;
+  if (zt) {
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) {
+      const int n = G::TZ * n1 + t;
+      float2 xk = xb[n * G::C + y], xm = cconj(xb[(G::M - n) * G::C + y]);
+      if (n == 0) {
+        xk.y = 0.f;
+        xm.y = 0.f;
+      }
+      const float2 O = cmul(csub(xk, xm), tw[n]);
+      v[n1] = cadd(cadd(xk, xm), make_float2(-O.y, O.x));
+    }
+  }
+  __syncthreads();  // the kz lines are read; their memory becomes the exchange rows
+  if (zt) {
+    line_fft<true, G::TZ>(v, u, xb + y * G::X, tz, t);
+    float2* dst = reinterpret_cast<float2*>(out + ((long long)(3 * slot + comp) * N + x) * G::N2 + y * N);
+#pragma unroll
+    for (int p = 0; p < 16; ++p) dst[line_k<G::TZ>(t, p)] = u[p];  // (r[2n], r[2n+1])
+  }
+}
+
 template <int N>
 int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
   using Z = ZGeo<N>;
@@ -556,14 +705,21 @@ int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
 template <int N>
 int solve_n(const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A, const int* slot_peak,
             int nslots, cudaStream_t s) {
-  using Z = ZGeo<N>;
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nslots * G::NH);
-  pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s, delta, spec, A, slot_peak);
-  pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
-  pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
-  pdl_launch(k_solve_rows<N>, dim3(3 * blocks), G::CTA, 0, s, spec, gspec, A, slot_peak);
-  pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s, gspec, force, A, slot_peak);
+  if constexpr (N <= 128) {
+    using S = SGeo<N>;
+    pdl_launch(k_slab_fwd<N>, dim3(N, nslots), S::THREADS, S::SMEM, s, delta, spec, A, slot_peak);
+    pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
+    pdl_launch(k_slab_inv<N>, dim3(3 * N, nslots), S::ITHREADS, S::SMEM, s, spec, gspec, force, A, slot_peak);
+  } else {
+    using Z = ZGeo<N>;
+    pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s, delta, spec, A, slot_peak);
+    pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
+    pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
+    pdl_launch(k_solve_rows<N>, dim3(3 * blocks), G::CTA, 0, s, spec, gspec, A, slot_peak);
+    pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s, gspec, force, A, slot_peak);
+  }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -603,6 +759,8 @@ int fft_native_init() {
   smem(k_solve_cols<128>, PGeo<128>::COLS_SMEM);
   smem(k_solve_cols<256>, PGeo<256>::COLS_SMEM);
   smem(k_solve_cols<512>, PGeo<512>::COLS_SMEM);
+  smem(k_slab_fwd<128>, SGeo<128>::SMEM);
+  smem(k_slab_inv<128>, SGeo<128>::SMEM);
   return e == cudaSuccess ? 0 : -(int)e;
 }
 
