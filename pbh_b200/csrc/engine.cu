@@ -373,6 +373,18 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   int TSmax = 1, max_bits = 0;
   const int full_every = (E->flags >> 8) & 0xFF;  // 0: never (the default; measured not to pay)
   std::vector<long long> st_base(npeaks + 1), p_base(npeaks + 1), mode_base(npeaks + 1);
+  // Super-tile side of the peaks that leave it open: 16 cells (the whole mesh below that), or 8 when
+  // the engine would then have fewer super-tiles, and so CTAs in the push and the deposit, than the
+  // GPU has SMs.  (One 32^3 peak: 45 us a step with 16, 31 with 8; one 64^3 peak 49 and 41; one
+  // 128^3 peak, 512 super-tiles of 16, 114 and 146.)
+  int sms = 0;
+  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E->device));
+  long long nst16 = 0;
+  for (int i = 0; i < npeaks; ++i) {
+    const long long side = cfg[i].tile > 0 ? std::max(1, cfg[i].N / cfg[i].tile) : std::max(1, cfg[i].N / 16);
+    nst16 += side * side * side;
+  }
+  const int tile_auto = nst16 < sms ? 8 : 16;
   for (int i = 0; i < npeaks; ++i) {
     const pm_peak_cfg& c = cfg[i];
     const int l2 = ilog2(c.N);
@@ -380,8 +392,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
     const long long npart = c.n > 0 ? c.n : (long long)c.Np * c.Np * c.Np;
     if (c.Np < 1 || npart >= (1LL << 31)) return -2002;
     if (!(c.L > 0)) return -2003;
-    // Super-tile side: 16^3 cells (the whole mesh below that); 4 and 8 are also built.
-    const int TS = c.tile > 0 ? c.tile : std::min(16, c.N);
+    const int TS = c.tile > 0 ? c.tile : std::min(tile_auto, c.N);
     if (ilog2(TS) < 2 || TS > 16 || TS > c.N) return -2004;
     PeakDesc& P = E->peaks[i];
     P = PeakDesc{};

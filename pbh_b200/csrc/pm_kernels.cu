@@ -78,8 +78,8 @@ struct TileRef {
   int pk, t;
 };
 
-__device__ __forceinline__ TileRef find_tile(const int2* st_ref) {
-  const int2 v = __ldg(st_ref + blockIdx.x);  // the same for every thread of the CTA
+__device__ __forceinline__ TileRef find_tile(const int2* st_ref, int tile) {
+  const int2 v = __ldg(st_ref + tile);  // the same for every thread of the CTA
   return TileRef{v.x, v.y};
 }
 
@@ -150,7 +150,7 @@ __device__ __forceinline__ bool push_move(const StepArgs& A, const PeakDesc& P, 
 }
 
 // SB: the bin buffer read (its arrays are then kernel parameters, not per-thread selects).
-template <int T, int SB>
+template <int T, int SB, int PT>
 __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P, int pk, u32 st, float* s_f, u32* s_stay,
                                            const PeakPlan& K, const BinLayout& L, const BinFill& F) {
   constexpr int T1 = T + 1, RS = patch_rs(T), PS = patch_ps(T), CS = patch_size(T);
@@ -176,8 +176,8 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
     pa = pp[j];
     ma = mp[j];
   }
-  if (k + PUSH_THREADS < n) {
-    const int j = k + PUSH_THREADS < n0 ? k + PUSH_THREADS : k + PUSH_THREADS + d1;
+  if (k + PT < n) {
+    const int j = k + PT < n0 ? k + PT : k + PT + d1;
     pb = pp[j];
     mb = mp[j];
   }
@@ -188,7 +188,7 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
     const int z0 = sz * T, zl = (sz * T + T) & (N - 1);
     // Thread t copies piece t % CH of the patch rows t / CH, t / CH + RSTEP, ..., of all three grids
     // at once (one address computation for three copies).
-    constexpr int NTH = PUSH_THREADS - PUSH_THREADS % CH, RSTEP = NTH / CH;
+    constexpr int NTH = PT - PT % CH, RSTEP = NTH / CH;
     if (threadIdx.x < NTH) {
       const int part = threadIdx.x % CH;
       const float *f0 = P.force + (part < T / 4 ? z0 + 4 * part : zl), *f1 = f0 + N3, *f2 = f1 + N3;
@@ -220,12 +220,12 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bool bad = false, lost = false;
   double ex = 0.0, ey = 0.0, ez = 0.0, ep = 0.0;  // this thread's momentum and p^2 sums
-  for (; k - lane < n; k += PUSH_THREADS) {  // uniform across a warp, so that its votes see all lanes
+  for (; k - lane < n; k += PT) {  // uniform across a warp, so that its votes see all lanes
     int4 ps = pa;
     float4 m = ma;
     pa = pb;
     ma = mb;
-    const int k2 = k + 2 * PUSH_THREADS;
+    const int k2 = k + 2 * PT;
     if (k2 < n) {
       const int j = k2 < n0 ? k2 : k2 + d1;
       pb = pp[j];
@@ -323,7 +323,7 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
   // Super-tile partials of the momentum and p^2 sums, in a fixed order: a plain FP64 tree over
   // the 32 lanes of a warp (about 5e-16 of the sum of magnitudes; compensating it cost 4 % of the
   // push), then compensated merges across the warps here and across super-tiles in k_tick.
-  __shared__ double s_e[PUSH_THREADS / 32][4];
+  __shared__ double s_e[PT / 32][4];
   const double ea[4] = {ex, ey, ez, ep};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -334,25 +334,28 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&A.stats[pk].status, 1u);
   if (__any_sync(0xffffffffu, lost) && lane == 0) atomicOr(&A.stats[pk].status, 4u);
   __syncthreads();
-  if (threadIdx.x == PUSH_THREADS - 1) {
+  if (threadIdx.x == PT - 1) {
     // This bin's fill in the buffer written: its stayers, and where its arrivals start.
     A.fill[SB ^ 1][gS].stay = *s_stay;
     A.fill[SB ^ 1][gS].gap = (u32)n;
   }
   if (warp < 4) {  // one warp per sum
-    static_assert(PUSH_THREADS <= 1024, "one lane per warp of the CTA");
-    CSum t = csum_warp(CSum{lane < PUSH_THREADS / 32 ? s_e[lane][warp] : 0.0, 0.0});
+    static_assert(PT >= 128 && PT <= 1024, "four warps for the sums, one lane per warp of the CTA");
+    CSum t = csum_warp(CSum{lane < PT / 32 ? s_e[lane][warp] : 0.0, 0.0});
     if (lane == 0) A.epart[gS * 4 + warp] = make_double2(t.s, t.c);
   }
 }
 
-__global__ void __launch_bounds__(PUSH_THREADS, 2) k_push(const __grid_constant__ StepArgs A) {
+// PT threads per CTA: PUSH_THREADS, or PUSH_THREADS_SMALL when no super-tile is larger than 8^3 cells
+// (512 particles are then four sweeps, whose loads overlap, instead of one).
+template <int PT>
+__global__ void __launch_bounds__(PT, 1024 / PT) k_push(const __grid_constant__ StepArgs A) {
   extern __shared__ __align__(16) float s_f[];
   __shared__ u32 s_stay;
   // A CTA's work is a chain of memory round trips (its tile, its peak and bin, then its particles
   // and force patch): as few as possible, because only two CTAs share an SM to hide them.  Both
   // candidates of the bin's layout and fill are fetched beside the plan that selects them.
-  const TileRef tr = find_tile(A.st_ref);
+  const TileRef tr = find_tile(A.st_ref, blockIdx.x);
   if (threadIdx.x == 0) s_stay = 0u;
   pdl_wait();
   const PeakPlan K = load_plan(A, tr.pk);
@@ -371,16 +374,17 @@ __global__ void __launch_bounds__(PUSH_THREADS, 2) k_push(const __grid_constant_
   const bool sb = K.flags & PLAN_SBUF;
   switch (P.TS) {
     case 4:
-      if (sb) push_super<4, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
-      else push_super<4, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      if (sb) push_super<4, 1, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<4, 0, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       break;
     case 8:
-      if (sb) push_super<8, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
-      else push_super<8, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      if (sb) push_super<8, 1, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<8, 0, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       break;
     default:
-      if (sb) push_super<16, 1>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
-      else push_super<16, 0>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      if (PT == PUSH_THREADS_SMALL) break;
+      if (sb) push_super<16, 1, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
+      else push_super<16, 0, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       break;
   }
 }
@@ -567,18 +571,14 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) k_layout(StepArgs A) {
 }
 
 // ------------------------------------------------------------------------------------------
-// After the push: each peak's energy and momentum, and its clock with (when the push overflowed a
-// bin) its new bin layout.  One launch, because every kernel of a step waits for the one before;
-// in it eslices CTAs per peak do the energies while one more does the clock.  What the energy CTAs
-// need of the clock the push has put aside (pushed_a), so the two sides share nothing.
-//
-// Energy of a peak that was just pushed: the push partials give K and sum p at the positions' a,
-// the previous step's Green partials give W at the same a (the grids were computed there).  Each
-// CTA (ENERGY_THREADS of the launch's threads; the compensated merges of more warps cost more than
-// they save) reduces a slice of the partials, about eight per thread for the engine's largest peak;
-// the last one to finish (atomic ticket) merges the slices in slice order and updates the
-// statistics.  All sums are compensated, every order fixed.  The Layzer-Irvine integral int K da
-// advances by the trapezoid rule between samples.
+// Energy and momentum of a peak that was just pushed: the push partials give K and sum p at the
+// positions' a, the previous step's Green partials give W at the same a (the grids were computed
+// there).  The deposit's launch carries these CTAs beside its own, because nothing in the step
+// waits for the result; what they need of the clock the push has put aside (pushed_a), since the
+// clock has moved on by then.  Each CTA reduces a slice of the partials (about eight per thread for
+// the engine's largest peak); the last one to finish (atomic ticket) merges the slices in slice
+// order and updates the statistics.  All sums are compensated, every order fixed.  The
+// Layzer-Irvine integral int K da advances by the trapezoid rule between samples.
 __device__ __forceinline__ void energy_slice(const StepArgs& A, int pk, int sl, CSum& tot) {
   const PeakDesc& P = A.peaks[pk];
   __shared__ CSum s_w[ENERGY_THREADS / 32][5];
@@ -630,6 +630,37 @@ __device__ __forceinline__ void energy_stats(const StepArgs& A, int pk, double a
   S.kin = kin;
   S.pot = pot;
   S.nsamples += 1;
+}
+
+__device__ __noinline__ void energy_cta(const StepArgs& A, int pk, int sl) {
+  __shared__ u32 s_last;
+  __shared__ double s_tot[5];
+  const double a = A.pushed_a[pk];
+  if (a < 0.0) return;  // not pushed
+  CSum t;  // threads 0 to 4: the sum each merges
+  energy_slice(A, pk, sl, t);
+  if (A.eslices > 1) {
+    if (threadIdx.x < 5) {
+      A.eslice[((long long)pk * ENERGY_SLICES + sl) * 5 + threadIdx.x] = make_double2(t.s, t.c);
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&A.ecount[pk], 1u) == (u32)A.eslices - 1 ? 1u : 0u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < 5) {
+      t = CSum{0.0, 0.0};
+      for (int q = 0; q < A.eslices; ++q) {
+        const double2 e = __ldcg(A.eslice + ((long long)pk * ENERGY_SLICES + q) * 5 + threadIdx.x);
+        csum_merge(t, CSum{e.x, e.y});
+      }
+    }
+    if (threadIdx.x == 0) A.ecount[pk] = 0u;
+  }
+  if (threadIdx.x < 5) s_tot[threadIdx.x] = t.s + t.c;
+  __syncthreads();
+  if (threadIdx.x == 0) energy_stats(A, pk, a, s_tot);
 }
 
 // Clock advance of a peak (one thread): applies the step that the push just made, selects the next
@@ -719,43 +750,14 @@ __device__ __forceinline__ bool advance_clock(const StepArgs& A, int pk) {
   return dep && c.relayout;
 }
 
-__global__ void __launch_bounds__(LAYOUT_THREADS) k_tick(StepArgs A) {
-  __shared__ u32 s_last;
-  __shared__ double s_tot[5];
-  const int pk = blockIdx.y;
+// One CTA per peak: its clock, then (when the push overflowed a bin) its new bin layout.
+__global__ void __launch_bounds__(LAYOUT_THREADS) k_tick(const __grid_constant__ StepArgs A) {
+  __shared__ int s_relayout;
+  const int pk = blockIdx.x;
   pdl_wait();
-  if ((int)blockIdx.x == A.eslices) {  // the clock
-    if (threadIdx.x == 0) s_last = advance_clock(A, pk);
-    __syncthreads();
-    if (s_last) layout_peak(A, pk, A.clocks[pk]);
-    return;
-  }
-  const double a = A.pushed_a[pk];
-  if (a < 0.0 || threadIdx.x >= ENERGY_THREADS) return;  // not pushed
-  CSum t;  // threads 0 to 4: the sum each merges
-  energy_slice(A, pk, blockIdx.x, t);
-  if (A.eslices > 1) {
-    if (threadIdx.x < 5) {
-      A.eslice[((long long)pk * ENERGY_SLICES + blockIdx.x) * 5 + threadIdx.x] = make_double2(t.s, t.c);
-      __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&A.ecount[pk], 1u) == (u32)A.eslices - 1 ? 1u : 0u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x < 5) {
-      t = CSum{0.0, 0.0};
-      for (int q = 0; q < A.eslices; ++q) {
-        const double2 e = __ldcg(A.eslice + ((long long)pk * ENERGY_SLICES + q) * 5 + threadIdx.x);
-        csum_merge(t, CSum{e.x, e.y});
-      }
-    }
-    if (threadIdx.x == 0) A.ecount[pk] = 0u;
-  }
-  if (threadIdx.x < 5) s_tot[threadIdx.x] = t.s + t.c;
+  if (threadIdx.x == 0) s_relayout = advance_clock(A, pk);
   __syncthreads();
-  if (threadIdx.x == 0) energy_stats(A, pk, a, s_tot);
+  if (s_relayout) layout_peak(A, pk, A.clocks[pk]);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1336,9 +1338,15 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
 
 
 __global__ void __launch_bounds__(DEP_THREADS, 4)
-    k_deposit(const __grid_constant__ StepArgs A, double* rho64, int only) {
+    k_deposit(const __grid_constant__ StepArgs A, double* rho64, int only, int necta) {
   extern __shared__ __align__(16) u32 s_dep[];
-  const TileRef tr = find_tile(A.st_ref);
+  if ((int)blockIdx.x < necta) {  // the energies' CTAs (in front, so that they start at once)
+    pdl_wait();
+    energy_cta(A, (int)blockIdx.x / A.eslices, (int)blockIdx.x % A.eslices);
+    return;
+  }
+  const int tile = (int)blockIdx.x - necta;
+  const TileRef tr = find_tile(A.st_ref, tile);
   const PeakDesc P = A.peaks[tr.pk];
   {  // clear the accumulators
     const int words = 2 * (P.TS == 4 ? patch_size(4) : P.TS == 8 ? patch_size(8) : patch_size(16));
@@ -1349,10 +1357,10 @@ __global__ void __launch_bounds__(DEP_THREADS, 4)
   pdl_wait();
   // The plan and both candidates of the bin's layout and fill in one round trip (as in k_push).
   const u32 flags = __ldcg(&A.plan[tr.pk].flags);
-  const int4 F0 = __ldcg(reinterpret_cast<const int4*>(A.fill[0] + blockIdx.x)),
-             F1 = __ldcg(reinterpret_cast<const int4*>(A.fill[1] + blockIdx.x));
-  const int2 L0 = __ldcg(reinterpret_cast<const int2*>(A.lay[0] + blockIdx.x)),
-             L1 = __ldcg(reinterpret_cast<const int2*>(A.lay[1] + blockIdx.x));
+  const int4 F0 = __ldcg(reinterpret_cast<const int4*>(A.fill[0] + tile)),
+             F1 = __ldcg(reinterpret_cast<const int4*>(A.fill[1] + tile));
+  const int2 L0 = __ldcg(reinterpret_cast<const int2*>(A.lay[0] + tile)),
+             L1 = __ldcg(reinterpret_cast<const int2*>(A.lay[1] + tile));
   const bool sb = flags & PLAN_SBUF;
   const int4 f = sb ? F1 : F0;
   const int2 l = flags & PLAN_LGEN ? L1 : L0;
@@ -1384,7 +1392,7 @@ __global__ void __launch_bounds__(FIX_THREADS) k_fixup(const __grid_constant__ S
   __shared__ long long s_red[FIX_THREADS / 32];
   __shared__ long long s_max[FIX_THREADS / 32];
   __shared__ const long long* s_nb[8];
-  const TileRef tr = find_tile(A.st_ref);
+  const TileRef tr = find_tile(A.st_ref, blockIdx.x);
   pdl_wait();
   const u32 flags = __ldcg(&A.plan[tr.pk].flags);
   const PeakDesc P = A.peaks[tr.pk];
@@ -1792,7 +1800,8 @@ size_t pm_tile_sort_smem() {
 }
 
 int pm_kernels_init() {
-  cudaError_t e = cudaFuncSetAttribute(k_push, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaError_t e =
+      cudaFuncSetAttribute(k_push<PUSH_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pm_tile_sort_smem());
@@ -1814,10 +1823,11 @@ static unsigned stride_grid(long long n, int t, int per_sm) {
 }
 
 void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s) {
-  pdl_launch(k_push, dim3((unsigned)nst), PUSH_THREADS, smem, s, A);
+  if (smem <= pm_push_smem(8)) pdl_launch(k_push<PUSH_THREADS_SMALL>, dim3((unsigned)nst), PUSH_THREADS_SMALL, smem, s, A);
+  else pdl_launch(k_push<PUSH_THREADS>, dim3((unsigned)nst), PUSH_THREADS, smem, s, A);
 }
 void launch_tick(const StepArgs& A, cudaStream_t s) {
-  pdl_launch(k_tick, dim3(A.eslices + 1, A.npeaks), LAYOUT_THREADS, 0, s, A);
+  pdl_launch(k_tick, dim3(A.npeaks), LAYOUT_THREADS, 0, s, A);
 }
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s) {
   k_permute<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A, ntot);
@@ -1833,7 +1843,8 @@ void launch_relayout(const StepArgs& A, long long nst, cudaStream_t s) {
   pdl_launch(k_relayout, dim3(stride_grid(nst, 1, RELAYOUT_CTAS_PER_SM)), PM_THREADS, 0, s, A);
 }
 void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, int only, cudaStream_t s) {
-  pdl_launch(k_deposit, dim3((unsigned)nst), DEP_THREADS, smem, s, A, rho64, only);
+  const int necta = only < 0 ? A.npeaks * A.eslices : 0;
+  pdl_launch(k_deposit, dim3((unsigned)(nst + necta)), DEP_THREADS, smem, s, A, rho64, only, necta);
 }
 void launch_fixup(const StepArgs& A, long long nst, double* rho64, int only, cudaStream_t s) {
   pdl_launch(k_fixup, dim3((unsigned)nst), FIX_THREADS, 0, s, A, rho64, only);

@@ -26,10 +26,11 @@
 
 #define PM_THREADS 256
 #define PUSH_THREADS 512
+#define PUSH_THREADS_SMALL 128
 #define DEP_THREADS 256    // deposit CTA (4 per SM)
 #define GREEN_MODES 4      // modes per thread of the Green kernel (a block covers PM_THREADS * GREEN_MODES)
 #define ENERGY_SLICES 128  // most CTAs per peak of the energy reduction
-#define ENERGY_THREADS 256 // threads of them that work
+#define ENERGY_THREADS DEP_THREADS  // they ride in the deposit's launch
 #define FIX_THREADS 256    // face fix-up CTA
 #define TSORT_THREADS 1024 // super-tile sort (refresh) CTA
 #define TSORT_CAP 5120     // particles of a super-tile sorted in shared memory; denser ones via global
