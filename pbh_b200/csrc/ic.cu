@@ -4,6 +4,7 @@
 // displacements of the quiet-start lattice.
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -48,45 +49,60 @@ __device__ double spline_eval(const double* __restrict__ xs, const double* __res
   return ((c[i] * t + c[m + i]) * t + c[2 * m + i]) * t + c[3 * m + i];
 }
 
-// Field on the centred cell grid x = (i + 1/2) dx - L/2 (pm3d.py:42-46).
-__global__ void k_field(int N, double L, int kind, double amp, double a0, double a1, double a2,
-                        const double* __restrict__ xs, const double* __restrict__ c, int m, double* __restrict__ out) {
+// The curvature field amp * profile(min(r, x_m)) on the centred cell grid x = (i + 1/2) dx - L/2
+// (pm3d.py:42-46); the noise (if any) is copied behind it on the way, so that one batched
+// transform takes both.
+__global__ void k_field(int N, double L, double amp, double a0, double a1, double a2, const double* __restrict__ xs,
+                        const double* __restrict__ c, int m, const double* __restrict__ noise,
+                        double* __restrict__ out) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long N3 = (long long)N * N * N;
   if (g >= N3) return;
-  const int iz = (int)(g % N), iy = (int)((g / N) % N), ix = (int)(g / ((long long)N * N));
+  const int l2 = 31 - __clz(N), iz = (int)(g & (N - 1)), iy = (int)((g >> l2) & (N - 1)), ix = (int)(g >> (2 * l2));
   const double dx = L / N;
   const double X = (ix + 0.5) * dx - L / 2, Y = (iy + 0.5) * dx - L / 2, Z = (iz + 0.5) * dx - L / 2;
-  if (kind == 0) {
-    const double r = sqrt((X / a0) * (X / a0) + (Y / a1) * (Y / a1) + (Z / a2) * (Z / a2));
-    out[g] = amp * spline_eval(xs, c, m, fmin(r, xs[m]));
-  } else {
-    out[g] = amp * exp(-(X * X / (2 * a0 * a0) + Y * Y / (2 * a1 * a1) + Z * Z / (2 * a2 * a2)));
-  }
+  const double r = sqrt((X / a0) * (X / a0) + (Y / a1) * (Y / a1) + (Z / a2) * (Z / a2));
+  if (noise) out[N3 + g] = noise[g];
+  out[g] = amp * spline_eval(xs, c, m, fmin(r, xs[m]));
 }
 
-// Noise spectrum shaping.  kind 0: band-limited P flat in ln k (pm3d.py:49-54);
-// kind 1: sqrt(P) = 1/k, P(0) = 0 (benchmark recipe).
-__global__ void k_shape(cufftDoubleComplex* __restrict__ s, int N, double L, int kind, double tail_rms, double k1,
-                        double k2) {
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int Nh = N / 2 + 1;
-  const long long M = (long long)N * N * Nh;
-  if (m >= M) return;
-  const int kz = (int)(m % Nh), iy = (int)((m / Nh) % N), ix = (int)(m / ((long long)Nh * N));
-  const double kf = kTwoPi / L;
-  const double kx = kline(ix, N, kf), ky = kline(iy, N, kf), kzv = kf * kz;
-  const double kk = m == 0 ? 0.0 : sqrt(kx * kx + ky * ky + kzv * kzv);
-  double f;
-  if (kind == 0) {
-    const bool band = kk >= k1 && kk <= k2;
-    const double P = band ? 2 * kPi * kPi * tail_rms * tail_rms / (fmax(kk, 1e-30) * fmax(kk, 1e-30) * fmax(kk, 1e-30) * log(k2 / k1)) : 0.0;
-    f = sqrt(P * (double)N * N * N / (L * L * L));
-  } else {
-    f = m == 0 ? 0.0 : 1.0 / kk;
+// The Gaussian peak exp(-sum x_i^2 / 2 R_i^2) is a product over the axes, and so is its transform:
+// out[axis][k] = sum_j exp(-x_j^2 / 2 R^2) W_N^(j k), one warp per value, instead of a field and a
+// 3D transform (143 + 150 us at 256^3).
+__global__ void __launch_bounds__(kThreads) k_gauss_lines(int N, double L, double r0, double r1, double r2,
+                                                          double2* __restrict__ out) {
+  const int w = (blockIdx.x * kThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= 3 * N) return;
+  const int axis = w / N, k = w - axis * N;
+  const double R = axis == 0 ? r0 : axis == 1 ? r1 : r2, dx = L / N;
+  double re = 0.0, im = 0.0;
+  for (int j = lane; j < N; j += 32) {
+    const double X = (j + 0.5) * dx - L / 2;
+    const double f = exp(-(X * X) / (2 * R * R));
+    double sn, cs;
+    sincospi(2.0 * (double)((j * k) & (N - 1)) / (double)N, &sn, &cs);
+    re += f * cs;
+    im -= f * sn;
   }
-  s[m].x *= f;
-  s[m].y *= f;
+  for (int d = 16; d > 0; d >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, d);
+    im += __shfl_xor_sync(0xffffffffu, im, d);
+  }
+  if (lane == 0) out[w] = make_double2(re, im);
+}
+
+// Noise spectrum shape at |k| = kk.  kind 0: band-limited P flat in ln k (pm3d.py:49-54); kind 1:
+// sqrt(P) = 1/k, P(0) = 0 (benchmark recipe).
+struct Shape {
+  int kind;
+  double N3, L, tail_rms, k1, k2;
+};
+__device__ __forceinline__ double shape_at(const Shape& h, double kk, bool zero) {
+  if (h.kind) return zero ? 0.0 : 1.0 / kk;
+  if (!(kk >= h.k1 && kk <= h.k2)) return 0.0;
+  const double km = fmax(kk, 1e-30);
+  const double P = 2 * kPi * kPi * h.tail_rms * h.tail_rms / (km * km * km * log(h.k2 / h.k1));
+  return sqrt(P * h.N3 / (h.L * h.L * h.L));
 }
 
 // Counter-based normal deviates for seeded noise generated on the device: Philox4x32-10
@@ -132,21 +148,8 @@ __global__ void k_philox_normal(double* __restrict__ out, long long n, unsigned 
     if (4 * q + k < n) out[4 * q + k] = z[k];
 }
 
-// y += a x with a = 1 (kind 0: make_ic's tail noise is already at its amplitude) or
-// a = noise_frac * amp / rms (kind 1: the recipe's noise scaled to noise_frac of the peak), rms
-// read from stat[1] on the device.
-__global__ void k_axpy_spec(cufftDoubleComplex* __restrict__ y, const cufftDoubleComplex* __restrict__ x,
-                            const double* __restrict__ stat, int kind, double noise_frac, double amp, long long M) {
-  const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  const double a = kind == 0 ? 1.0 : noise_frac * amp / stat[1];
-  y[m].x += a * x[m].x;
-  y[m].y += a * x[m].y;
-}
-
-// delta_k (kind 0: 0.4 k^2 zeta_k / H_i^2, pm3d.py:59), zero mode removed; then the four
-// spectra inverted at once: delta_lin = irfftn(dk) (pm3d.py:70) and psi_c = -irfftn(i k_c phi),
-// phi = -dk/k^2 (pm3d.py:61-62).  Each spectrum carries numpy's 1/N^3 and, in the kz = 0 and
+// One mode of delta_k (kind 0: 0.4 k^2 zeta_k / H_i^2, pm3d.py:59), zero mode removed, and of the
+// three displacements (see k_spectra).  Each spectrum carries numpy's 1/N^3 and, in the kz = 0 and
 // kz = N/2 planes, its Hermitian part (numpy's irfftn uses only that part there).
 __device__ __forceinline__ void four_spectra(const cufftDoubleComplex z, int kind, double kx, double ky, double kz,
                                             long long m, double* re, double* im) {
@@ -168,130 +171,229 @@ __device__ __forceinline__ void four_spectra(const cufftDoubleComplex z, int kin
   }
 }
 
-__global__ void k_disp_spectra(const cufftDoubleComplex* __restrict__ s, int N, double L, int kind,
-                               cufftDoubleComplex* __restrict__ out) {
+// Everything about the linear density spectrum before the potential: the peak's (gl: the Gaussian
+// lines; spec: a transformed field) plus the shaped noise (ns), times its amplitude a.
+struct Modes {
+  int N, l2, kind;
+  double kf, amp, a;
+  const double2* gl;
+  const cufftDoubleComplex *spec, *ns;
+  Shape shape;
+};
+__device__ __forceinline__ cufftDoubleComplex mode_at(const Modes& g, int ix, int iy, int kz, double kx, double ky,
+                                                      double kzv) {
+  const int N = g.N, Nh = N / 2 + 1;
+  const long long m = ((long long)ix * N + iy) * Nh + kz;
+  cufftDoubleComplex z;
+  if (g.kind) {
+    const double2 a = g.gl[ix], b = g.gl[N + iy], c = g.gl[2 * N + kz];
+    const double2 ab = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    z.x = g.amp * (ab.x * c.x - ab.y * c.y);
+    z.y = g.amp * (ab.x * c.y + ab.y * c.x);
+  } else {
+    z = g.spec[m];
+  }
+  if (g.ns) {
+    const double f = g.a * shape_at(g.shape, sqrt(kx * kx + ky * ky + kzv * kzv), m == 0);
+    const cufftDoubleComplex n = g.ns[m];
+    z.x += f * n.x;
+    z.y += f * n.y;
+  }
+  return z;
+}
+
+// The nf spectra inverted at once: psi_c = -irfftn(i k_c phi) with phi = -dk / k^2 (pm3d.py:61-62),
+// and (nf = 4) delta_lin = irfftn(dk) (pm3d.py:70).  noise_frac and stat (kind 1): the noise is scaled
+// to noise_frac of the peak by its own rms, which is on the device.
+__global__ void __launch_bounds__(kThreads) k_spectra(Modes g, double noise_frac, const double* __restrict__ stat, int nf,
+                                                      cufftDoubleComplex* __restrict__ out) {
   const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int Nh = N / 2 + 1;
+  const int N = g.N, Nh = N / 2 + 1;
   const long long M = (long long)N * N * Nh;
   if (m >= M) return;
-  const int kz = (int)(m % Nh), iy = (int)((m / Nh) % N), ix = (int)(m / ((long long)Nh * N));
-  const double kf = kTwoPi / L;
-  const double kx = kline(ix, N, kf), ky = kline(iy, N, kf), kzv = kf * kz;
+  g.a = g.kind ? noise_frac * g.amp / stat[0] : 1.0;
+  const u32 row = (u32)m / (u32)Nh;  // M < 2^32: a mesh of 2048^3 does not fit the GPU
+  const int kz = (int)(m - (long long)row * Nh), iy = (int)(row & (N - 1)), ix = (int)(row >> g.l2);
+  const double kx = kline(ix, N, g.kf), ky = kline(iy, N, g.kf), kzv = g.kf * kz;
   double re[4], im[4];
-  four_spectra(s[m], kind, kx, ky, kzv, m, re, im);
+  four_spectra(mode_at(g, ix, iy, kz, kx, ky, kzv), g.kind, kx, ky, kzv, m, re, im);
   if (kz == 0 || kz == N / 2) {
     const int px = (-ix) & (N - 1), py = (-iy) & (N - 1);
-    const long long mp = ((long long)px * N + py) * Nh + kz;
+    const double qx = kline(px, N, g.kf), qy = kline(py, N, g.kf);
     double rp[4], ip[4];
-    four_spectra(s[mp], kind, kline(px, N, kf), kline(py, N, kf), kzv, mp, rp, ip);
+    four_spectra(mode_at(g, px, py, kz, qx, qy, kzv), g.kind, qx, qy, kzv, ((long long)px * N + py) * Nh + kz, rp, ip);
     for (int c = 0; c < 4; ++c) {
       re[c] = 0.5 * (re[c] + rp[c]);
       im[c] = 0.5 * (im[c] - ip[c]);
     }
   }
-  const double inv = 1.0 / ((double)N * N * N);
-  for (int c = 0; c < 4; ++c) {
-    out[c * M + m].x = re[c] * inv;
-    out[c * M + m].y = im[c] * inv;
+  const double inv = 1.0 / g.shape.N3;
+  for (int c = 1; c < 4; ++c) {
+    out[(c - 1) * M + m].x = re[c] * inv;
+    out[(c - 1) * M + m].y = im[c] * inv;
+  }
+  if (nf == 4) {
+    out[3 * M + m].x = re[0] * inv;
+    out[3 * M + m].y = im[0] * inv;
   }
 }
 
-// Lattice (pm3d.py:64-65), CIC displacement at (Q + L/2) % L (pm3d.py:66), x and p
-// (pm3d.py:67-68).  Python's float % is x - L*floor(x/L).
+// Rms of the shaped noise on the grid (numpy's std) from its spectrum (Parseval; the mean is the
+// zero mode, left out; the half spectrum counts 0 < kz < N/2 twice), instead of transforming it
+// back and reading the grid twice.  Partials per block, summed in a fixed order by the last one.
+__global__ void __launch_bounds__(kThreads) k_noise_rms(Modes g, double* __restrict__ part, u32* __restrict__ count,
+                                                        double* __restrict__ stat) {
+  __shared__ double sh[kThreads / 32];
+  __shared__ bool last;
+  const int N = g.N, Nh = N / 2 + 1;
+  const long long M = (long long)N * N * Nh;
+  double s = 0.0;
+  for (long long m = (long long)blockIdx.x * kThreads + threadIdx.x; m < M; m += (long long)gridDim.x * kThreads) {
+    if (m == 0) continue;
+    const u32 row = (u32)m / (u32)Nh;  // M < 2^32: a mesh of 2048^3 does not fit the GPU
+    const int kz = (int)(m - (long long)row * Nh);
+    const double kx = kline((int)(row >> g.l2), N, g.kf), ky = kline((int)(row & (N - 1)), N, g.kf), kzv = g.kf * kz;
+    const double f = shape_at(g.shape, sqrt(kx * kx + ky * ky + kzv * kzv), false);
+    const cufftDoubleComplex n = g.ns[m];
+    const double p = (f * n.x) * (f * n.x) + (f * n.y) * (f * n.y);
+    s += kz == 0 || kz == N / 2 ? p : 2.0 * p;
+  }
+  auto block_sum = [&](double v) {
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) t += sh[w];
+    __syncthreads();
+    return t;
+  };
+  const double t = block_sum(s);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double q = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads) q += __ldcg(part + b);
+  q = block_sum(q);
+  if (threadIdx.x == 0) {
+    *count = 0u;
+    stat[0] = sqrt(q) / g.shape.N3;
+  }
+}
+
+// Python's float modulo, x - L floor(x/L), for x / L in [-1, 2) without the general remainder (the
+// same bits: both subtractions are exact there).
 __device__ __forceinline__ double pymod(double x, double L) {
+  if (x >= 0.0 && x < L) return x;
+  if (x >= L && x < 2 * L) return x - L;
+  if (x < 0.0 && x >= -L) return x + L;
   double r = fmod(x, L);
   if (r != 0.0 && ((r < 0) != (L < 0))) r += L;
   return r;
 }
 
-__global__ void k_lattice(int N, int Np, double L, const double* __restrict__ psi, double* __restrict__ x,
-                          double* __restrict__ p) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long n = (long long)Np * Np * Np;
-  if (i >= n) return;
-  const int jz = (int)(i % Np), jy = (int)((i / Np) % Np), jx = (int)(i / ((long long)Np * Np));
+// One axis of the lattice: coordinate Q_j (pm3d.py:64-65), and the two mesh nodes and CIC weights at
+// (Q_j + L/2) % L (pm3d.py:66).  A lattice point that lies on a node up to rounding (any Np that
+// divides N into odd parts, Np = N above all) is put on it, so that the far node is not read.
+struct LatticeAxis {
+  double q, w0, w1;
+  int i0, i1;
+};
+__global__ void k_lattice_axis(int N, int Np, double L, LatticeAxis* __restrict__ out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= Np) return;
   const double dq = L / Np, dx = L / N;
-  const double Q[3] = {(jx + 0.5) * dq - L / 2, (jy + 0.5) * dq - L / 2, (jz + 0.5) * dq - L / 2};
-  long long i0[3], i1[3];
-  double f[3];
-  for (int d = 0; d < 3; ++d) {
-    const double at = pymod(Q[d] + L / 2, L);
-    const double g = at / dx - 0.5;
-    const double fl = floor(g);
-    const long long c = (long long)fl;
-    f[d] = g - fl;
-    i0[d] = ((c % N) + N) % N;
-    i1[d] = (((c + 1) % N) + N) % N;
-  }
-  const long long N3 = (long long)N * N * N;
-  double disp[3] = {0.0, 0.0, 0.0};
-  for (int c = 0; c < 8; ++c) {
-    const int cx = c >> 2, cy = (c >> 1) & 1, cz = c & 1;
-    const long long o = ((cx ? i1[0] : i0[0]) * N + (cy ? i1[1] : i0[1])) * N + (cz ? i1[2] : i0[2]);
-    const double w = (cx ? f[0] : 1.0 - f[0]) * (cy ? f[1] : 1.0 - f[1]) * (cz ? f[2] : 1.0 - f[2]);
-    for (int d = 0; d < 3; ++d) disp[d] += psi[(1 + d) * N3 + o] * w;
-  }
-  for (int d = 0; d < 3; ++d) {
-    x[3 * i + d] = pymod(Q[d] + disp[d] + L / 2, L);
-    p[3 * i + d] = PM_H_I * disp[d];
-  }
+  LatticeAxis a;
+  a.q = (j + 0.5) * dq - L / 2;
+  const double g = pymod(a.q + L / 2, L) / dx - 0.5, near = rint(g);
+  const bool on = fabs(g - near) <= 4e-16 * N;
+  const double fl = on ? near : floor(g);
+  const long long c = (long long)fl;
+  a.w1 = on ? 0.0 : g - fl;
+  a.w0 = 1.0 - a.w1;
+  a.i0 = (int)(((c % N) + N) % N);
+  a.i1 = (int)(((c + 1) % N + N) % N);
+  out[j] = a;
 }
 
-// Block partial sums of x and (x - mean)^2 for numpy's std (mean first, then the spread).
-// Block partials of sum v (squares = 0) or of sum (v - stat[0])^2 (squares = 1).
-__global__ void k_partial(const double* __restrict__ v, long long n, const double* __restrict__ stat, int squares,
-                          double* __restrict__ part) {
-  __shared__ double sh[kThreads];
-  const double mean = squares ? stat[0] : 0.0;
-  double s = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double d = squares ? v[i] - mean : v[i];
-    s += squares ? d * d : d;
+// Lattice and CIC displacement (pm3d.py:64-68): x and p of every particle.  A block takes kThreads
+// consecutive particles, and their coordinates from the axis table (no division or remainder per
+// particle); their 24-byte rows leave through shared memory, 8 bytes per lane in order.
+__global__ void __launch_bounds__(kThreads) k_lattice(int N, int Np, double L, const LatticeAxis* __restrict__ ax,
+                                                      const double* __restrict__ psi, double* __restrict__ x,
+                                                      double* __restrict__ p) {
+  __shared__ double sx[3 * kThreads], sp[3 * kThreads];
+  const long long n = (long long)Np * Np * Np, b0 = (long long)blockIdx.x * kThreads;
+  const long long i = b0 + threadIdx.x;
+  if (i < n) {
+    const u32 row = n < (1LL << 32) ? (u32)i / (u32)Np : (u32)(i / Np);  // jx Np + jy
+    const u32 jx = row / (u32)Np;
+    const LatticeAxis A[3] = {ax[jx], ax[row - jx * (u32)Np], ax[(u32)(i - (long long)row * Np)]};
+    const long long N3 = (long long)N * N * N;
+    double disp[3] = {0.0, 0.0, 0.0};
+    for (int c = 0; c < 8; ++c) {
+      const double w = (c & 4 ? A[0].w1 : A[0].w0) * (c & 2 ? A[1].w1 : A[1].w0) * (c & 1 ? A[2].w1 : A[2].w0);
+      if (w == 0.0) continue;
+      const long long o = ((long long)(c & 4 ? A[0].i1 : A[0].i0) * N + (c & 2 ? A[1].i1 : A[1].i0)) * N + (c & 1 ? A[2].i1 : A[2].i0);
+      for (int d = 0; d < 3; ++d) disp[d] += psi[d * N3 + o] * w;
+    }
+    for (int d = 0; d < 3; ++d) {
+      sx[3 * threadIdx.x + d] = pymod(A[d].q + disp[d] + L / 2, L);
+      sp[3 * threadIdx.x + d] = PM_H_I * disp[d];
+    }
   }
-  sh[threadIdx.x] = s;
   __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
+  const long long m = min((long long)kThreads, n - b0) * 3;
+  for (int k = threadIdx.x; k < m; k += kThreads) {
+    x[3 * b0 + k] = sx[k];
+    p[3 * b0 + k] = sp[k];
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// The partials summed in block order by one thread: stat[0] = mean (squares = 0), or stat[1] =
-// rms / N3 of the unnormalised inverse transform (squares = 1), the noise field's rms.
-__global__ void k_reduce_partials(const double* __restrict__ part, int nb, long long n, long long N3, int squares,
-                                  double* __restrict__ stat) {
-  double t = 0.0;
-  for (int b = 0; b < nb; ++b) t += part[b];
-  if (!squares) stat[0] = t / (double)n;
-  else stat[1] = sqrt(t / (double)n) / (double)N3;
-}
-
-constexpr int kStdBlocks = 1024;
-
-// Standard deviation of v (two passes, fixed order) into stat[1], divided by N3; on stream s.
-void grid_std(const double* v, long long n, long long N3, double* part, double* stat, cudaStream_t s) {
-  k_partial<<<kStdBlocks, kThreads, 0, s>>>(v, n, stat, 0, part);
-  k_reduce_partials<<<1, 1, 0, s>>>(part, kStdBlocks, n, N3, 0, stat);
-  k_partial<<<kStdBlocks, kThreads, 0, s>>>(v, n, stat, 1, part);
-  k_reduce_partials<<<1, 1, 0, s>>>(part, kStdBlocks, n, N3, 1, stat);
-}
+constexpr int kRmsBlocks = 592;
 
 unsigned nblk(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-// Device buffers and FP64 cuFFT plans of pm_make_ic, kept per (device, N) after first use so
+// Device buffers and FP64 cuFFT plans of pm_make_ic, kept per (device, N, path) after first use so
 // that repeated calls (a request loop) neither allocate nor plan again.
 struct ICWork {
-  double *field = nullptr, *real4 = nullptr, *tmp_real = nullptr, *noise = nullptr;
-  cufftDoubleComplex *spec = nullptr, *nspec = nullptr, *spec4 = nullptr, *tmp_spec = nullptr;
-  double* part = nullptr;  // kStdBlocks partials, then stat[2] (mean, noise rms)
-  cufftHandle d2z = 0, z2d = 0, z2d4 = 0;
+  double* field = nullptr;               // [2][N^3] peak field, noise
+  cufftDoubleComplex* spec = nullptr;    // [2][M] their spectra
+  cufftDoubleComplex* spec4 = nullptr;   // [4][M] displacements, delta_lin
+  double* real4 = nullptr;               // [4][N^3]
+  double2* lines = nullptr;              // [3][N] Gaussian lines
+  double* part = nullptr;                // kRmsBlocks partials, then stat[1] (noise rms)
+  u32* count = nullptr;
+  LatticeAxis* axis = nullptr;           // [axis_n]
+  int axis_n = 0;
+  double* spline = nullptr;              // [spline_n] knots, coefficients
+  int spline_n = 0;
+  cufftHandle d2z = 0, d2z2 = 0, z2d3 = 0, z2d4 = 0;
   bool ok = false;
+  std::mutex busy;                       // held through a synchronous call
 };
 std::mutex g_ic_mu;
 // Keyed by (device, N, path): the synchronous pm_make_ic and the stream-ordered
 // pm_make_ic_async keep separate work areas, so the two never share buffers in flight.
 std::map<std::tuple<int, int, int>, ICWork> g_ic;
+
+void ic_free(ICWork& w) {
+  cudaFree(w.field);
+  cudaFree(w.spec);
+  cudaFree(w.spec4);
+  cudaFree(w.real4);
+  cudaFree(w.lines);
+  cudaFree(w.part);
+  cudaFree(w.count);
+  cudaFree(w.axis);
+  cudaFree(w.spline);
+  for (cufftHandle h : {w.d2z, w.d2z2, w.z2d3, w.z2d4})
+    if (h) cufftDestroy(h);
+}
 
 int ic_work(int device, int N, int path, ICWork** out) {
   std::lock_guard<std::mutex> lock(g_ic_mu);
@@ -300,21 +402,22 @@ int ic_work(int device, int N, int path, ICWork** out) {
     const long long N3 = (long long)N * N * N, M = (long long)N * N * (N / 2 + 1);
     int rc = 0;
     int n3[3] = {N, N, N};
-    CU(cudaMalloc(&w.field, sizeof(double) * N3));
-    CU(cudaMalloc(&w.real4, sizeof(double) * 4 * N3));
-    CU(cudaMalloc(&w.tmp_real, sizeof(double) * N3));
-    CU(cudaMalloc(&w.noise, sizeof(double) * N3));
-    CU(cudaMalloc(&w.spec, sizeof(cufftDoubleComplex) * M));
-    CU(cudaMalloc(&w.nspec, sizeof(cufftDoubleComplex) * M));
+    CU(cudaMalloc(&w.field, sizeof(double) * 2 * N3));
+    CU(cudaMalloc(&w.spec, sizeof(cufftDoubleComplex) * 2 * M));
     CU(cudaMalloc(&w.spec4, sizeof(cufftDoubleComplex) * 4 * M));
-    CU(cudaMalloc(&w.tmp_spec, sizeof(cufftDoubleComplex) * M));
-    CU(cudaMalloc(&w.part, sizeof(double) * (kStdBlocks + 2)));
+    CU(cudaMalloc(&w.real4, sizeof(double) * 4 * N3));
+    CU(cudaMalloc(&w.lines, sizeof(double2) * 3 * N));
+    CU(cudaMalloc(&w.part, sizeof(double) * (kRmsBlocks + 1)));
+    CU(cudaMalloc(&w.count, sizeof(u32)));
+    CU(cudaMemset(w.count, 0, sizeof(u32)));
     CF(cufftPlan3d(&w.d2z, N, N, N, CUFFT_D2Z));
-    CF(cufftPlan3d(&w.z2d, N, N, N, CUFFT_Z2D));
+    CF(cufftPlanMany(&w.d2z2, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, 2));
+    CF(cufftPlanMany(&w.z2d3, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 3));
     CF(cufftPlanMany(&w.z2d4, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 4));
     w.ok = true;
   done:
     if (rc) {
+      ic_free(w);
       g_ic.erase({device, N, path});
       return rc;
     }
@@ -323,27 +426,27 @@ int ic_work(int device, int N, int path, ICWork** out) {
   return 0;
 }
 
+// Grows a kept buffer to n elements; the stream is drained first, since earlier work on it may
+// still read the old one.
+template <class T>
+cudaError_t grow(T** buf, int* have, int n, cudaStream_t s) {
+  if (*have >= n) return cudaSuccess;
+  cudaError_t e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && *buf) e = cudaFree(*buf);
+  *buf = nullptr;
+  *have = 0;
+  if (e == cudaSuccess) e = cudaMalloc((void**)buf, sizeof(T) * (size_t)n);
+  if (e == cudaSuccess) *have = n;
+  return e;
+}
+
 }  // namespace
 
 extern "C" int pm_ic_release_cache(void) {
   std::lock_guard<std::mutex> lock(g_ic_mu);
   for (auto& kv : g_ic) {
-    ICWork& w = kv.second;
     cudaSetDevice(std::get<0>(kv.first));
-    cudaFree(w.field);
-    cudaFree(w.real4);
-    cudaFree(w.tmp_real);
-    cudaFree(w.noise);
-    cudaFree(w.spec);
-    cudaFree(w.nspec);
-    cudaFree(w.spec4);
-    cudaFree(w.tmp_spec);
-    cudaFree(w.part);
-    if (w.ok) {
-      cufftDestroy(w.d2z);
-      cufftDestroy(w.z2d);
-      cufftDestroy(w.z2d4);
-    }
+    ic_free(kv.second);
   }
   g_ic.clear();
   return 0;
@@ -360,46 +463,69 @@ int check_params(const pm_ic_params* prm, const double* x_out, const double* p_o
   return 0;
 }
 
-// The IC pipeline on stream s with work area w (spline arrays xs, cs on the device for kind 0).
-// The noise rms is left in w->part[kStdBlocks + 1].
-int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* delta_lin_out, const double* xs,
-               const double* cs, ICWork* w, cudaStream_t s) {
-  const int N = prm->N, Np = prm->Np;
+// Bounded by the float64 transforms (cuFFT, 4 back and at most 2 forward: 1.05 of the 1.43 ms of a
+// 256^3 call) and, below 64^3, by its launches (nine).  Before the lines, the Parseval sum, the
+// fused spectra and the axis table (a field transform, an inverse transform with two grid
+// reductions for the rms, four passes over the spectra, 64-bit remainders per particle):
+// 2.51 ms at 256^3 with noise and delta_lin, 270 -> 147 us for a 64^3 curvature profile.
+//
+// The IC pipeline on stream s with work area w (kind 0: w->spline holds the spline).  The noise rms
+// is left in w->part[kRmsBlocks].
+int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* delta_lin_out, ICWork* w, cudaStream_t s) {
+  const int N = prm->N, Np = prm->Np, nf = delta_lin_out ? 4 : 3;
   const long long N3 = (long long)N * N * N, M = (long long)N * N * (N / 2 + 1);
   const double L = prm->L;
   int rc = 0;
-  double* stat = w->part + kStdBlocks;
+  double* stat = w->part + kRmsBlocks;
   const bool want_noise = (prm->kind == 0 && prm->tail_rms > 0) || (prm->kind == 1 && prm->noise_frac > 0);
   const bool noisy = want_noise && (prm->noise || prm->noise_seed);
-  CF(cufftSetStream(w->d2z, s));
-  CF(cufftSetStream(w->z2d, s));
-  CF(cufftSetStream(w->z2d4, s));
-  CU(cudaMemsetAsync(stat, 0, sizeof(double) * 2, s));
-  k_field<<<nblk(N3), kThreads, 0, s>>>(N, L, prm->kind, prm->amp, prm->axes[0], prm->axes[1], prm->axes[2], xs, cs,
-                                        prm->kind == 0 ? prm->spline_m : 0, w->field);
-  CU(cudaGetLastError());
-  CF(cufftExecD2Z(w->d2z, w->field, w->spec));
-  if (noisy) {
-    if (!prm->noise) {  // seeded device noise
-      k_philox_normal<<<nblk((N3 + 3) / 4), kThreads, 0, s>>>(w->noise, N3, prm->noise_seed);
-      CU(cudaGetLastError());
-    }
-    CF(cufftExecD2Z(w->d2z, prm->noise ? (double*)prm->noise : w->noise, w->nspec));
-    k_shape<<<nblk(M), kThreads, 0, s>>>(w->nspec, N, L, prm->kind, prm->tail_rms, prm->k1, prm->k2);
-    CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(w->tmp_spec, w->nspec, sizeof(cufftDoubleComplex) * M, cudaMemcpyDeviceToDevice, s));
-    CF(cufftExecZ2D(w->z2d, w->tmp_spec, w->tmp_real));  // unnormalised inverse; numpy divides by N^3
-    grid_std(w->tmp_real, N3, N3, w->part, stat, s);
-    k_axpy_spec<<<nblk(M), kThreads, 0, s>>>(w->spec, w->nspec, stat, prm->kind, prm->noise_frac, prm->amp, M);
+  const cufftHandle inverse = nf == 4 ? w->z2d4 : w->z2d3;
+  Modes g{};
+  g.N = N;
+  while ((1 << g.l2) < N) ++g.l2;
+  g.kind = prm->kind;
+  g.kf = kTwoPi / L;
+  g.amp = prm->amp;
+  g.gl = w->lines;
+  g.spec = w->spec;
+  g.ns = noisy ? w->spec + M : nullptr;
+  g.shape = Shape{prm->kind, (double)N3, L, prm->tail_rms, prm->k1, prm->k2};
+  CU(grow(&w->axis, &w->axis_n, Np, s));
+  k_lattice_axis<<<nblk(Np), kThreads, 0, s>>>(N, Np, L, w->axis);
+  if (noisy && !prm->noise) {  // seeded device noise
+    k_philox_normal<<<nblk((N3 + 3) / 4), kThreads, 0, s>>>(w->field + N3, N3, prm->noise_seed);
     CU(cudaGetLastError());
   }
-  k_disp_spectra<<<nblk(M), kThreads, 0, s>>>(w->spec, N, L, prm->kind, w->spec4);
+  if (prm->kind == 0) {
+    const int m = prm->spline_m;
+    k_field<<<nblk(N3), kThreads, 0, s>>>(N, L, prm->amp, prm->axes[0], prm->axes[1], prm->axes[2], w->spline,
+                                          w->spline + m + 1, m, noisy ? prm->noise : nullptr, w->field);
+    CU(cudaGetLastError());
+    const cufftHandle forward = noisy ? w->d2z2 : w->d2z;
+    CF(cufftSetStream(forward, s));
+    CF(cufftExecD2Z(forward, w->field, w->spec));
+  } else {
+    k_gauss_lines<<<nblk(3LL * N * 32), kThreads, 0, s>>>(N, L, prm->axes[0], prm->axes[1], prm->axes[2], w->lines);
+    CU(cudaGetLastError());
+    if (noisy) {
+      CF(cufftSetStream(w->d2z, s));
+      CF(cufftExecD2Z(w->d2z, prm->noise ? (double*)prm->noise : w->field + N3, w->spec + M));
+    }
+  }
+  if (noisy) {
+    k_noise_rms<<<(unsigned)std::min<long long>(kRmsBlocks, nblk(M)), kThreads, 0, s>>>(g, w->part, w->count, stat);
+    CU(cudaGetLastError());
+  } else {
+    CU(cudaMemsetAsync(stat, 0, sizeof(double), s));
+  }
+  k_spectra<<<nblk(M), kThreads, 0, s>>>(g, prm->noise_frac, stat, nf, w->spec4);
   CU(cudaGetLastError());
-  CF(cufftExecZ2D(w->z2d4, w->spec4, w->real4));
-  k_lattice<<<nblk((long long)Np * Np * Np), kThreads, 0, s>>>(N, Np, L, w->real4, x_out, p_out);
+  CF(cufftSetStream(inverse, s));
+  CF(cufftExecZ2D(inverse, w->spec4, w->real4));
+  k_lattice<<<nblk((long long)Np * Np * Np), kThreads, 0, s>>>(N, Np, L, w->axis, w->real4, x_out, p_out);
   CU(cudaGetLastError());
   if (delta_lin_out)
-    CU(cudaMemcpyAsync(delta_lin_out, w->real4, sizeof(double) * N3, cudaMemcpyDeviceToDevice, s));
+    CU(cudaMemcpyAsync(delta_lin_out, w->real4 + 3 * N3, sizeof(double) * N3, cudaMemcpyDeviceToDevice, s));
 done:
   return rc;
 }
@@ -410,27 +536,25 @@ extern "C" int pm_make_ic(const pm_ic_params* prm, double* x_out, double* p_out,
                           double* noise_rms_out) {
   if (int r = check_params(prm, x_out, p_out)) return r;
   int rc = 0, device = 0;
-  double *xs = nullptr, *cs = nullptr;
-  double stat[2] = {0.0, 0.0};
+  double rms = 0.0;
   ICWork* w = nullptr;
+  std::unique_lock<std::mutex> hold;
   CU(cudaGetDevice(&device));
   rc = ic_work(device, prm->N, 0, &w);
   if (rc) return rc;
+  hold = std::unique_lock<std::mutex>(w->busy);
   if (prm->kind == 0) {
     const int m = prm->spline_m;
-    CU(cudaMalloc(&xs, sizeof(double) * (m + 1)));
-    CU(cudaMalloc(&cs, sizeof(double) * 4 * m));
-    CU(cudaMemcpy(xs, prm->spline_x, sizeof(double) * (m + 1), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(cs, prm->spline_c, sizeof(double) * 4 * m, cudaMemcpyHostToDevice));
+    CU(grow(&w->spline, &w->spline_n, 5 * m + 1, 0));
+    CU(cudaMemcpyAsync(w->spline, prm->spline_x, sizeof(double) * (m + 1), cudaMemcpyHostToDevice, 0));
+    CU(cudaMemcpyAsync(w->spline + m + 1, prm->spline_c, sizeof(double) * 4 * m, cudaMemcpyHostToDevice, 0));
   }
-  rc = make_ic_on(prm, x_out, p_out, delta_lin_out, xs, cs, w, 0);
+  rc = make_ic_on(prm, x_out, p_out, delta_lin_out, w, 0);
   if (rc) goto done;
-  CU(cudaMemcpy(stat, w->part + kStdBlocks, sizeof(stat), cudaMemcpyDeviceToHost));
+  CU(cudaMemcpyAsync(&rms, w->part + kRmsBlocks, sizeof(rms), cudaMemcpyDeviceToHost, 0));
   CU(cudaDeviceSynchronize());
-  if (noise_rms_out) *noise_rms_out = stat[1];
+  if (noise_rms_out) *noise_rms_out = rms;
 done:
-  cudaFree(xs);
-  cudaFree(cs);
   return rc;
 }
 
@@ -442,5 +566,5 @@ extern "C" int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* 
   if (e != cudaSuccess) return -(int)e;
   ICWork* w = nullptr;
   if (int r = ic_work(device, prm->N, 1, &w)) return r;
-  return make_ic_on(prm, x_out, p_out, nullptr, nullptr, nullptr, w, (cudaStream_t)stream);
+  return make_ic_on(prm, x_out, p_out, nullptr, w, (cudaStream_t)stream);
 }
