@@ -53,7 +53,7 @@ struct PeakDesc {
   int native_fft;          // 1: the native solve makes the forces (no cuFFT, no k_green)
   int bin_shift, bin_min;  // bin capacity: count + (count >> bin_shift) + bin_min, rounded up to BIN_ALIGN
   int bin_grow;            // relayout: room for this many more steps of a bin's growth (region allowing)
-  int pad_bg;
+  int np4;                 // Np / 4 of an Np^3 lattice with Np a multiple of 4, else 0
   double L, dx, smooth, n_mean, m_part;
   long long n_mean_fix;    // round(n_mean * 2^38)
   double inv_fix_nmean;    // 2^-38 / n_mean

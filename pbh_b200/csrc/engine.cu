@@ -85,6 +85,7 @@ struct pm_engine {
   u32* ovf_n = nullptr;                        // [peak] overflow-area particles
   u32* ovf_in = nullptr;                       // [super-tile] overflowed arrivals
   u32* new_count = nullptr;                    // [super-tile] count after a relayout
+  u32* load_count = nullptr;                   // [super-tile] loaded particles
   u32* keys[2] = {nullptr, nullptr};
   u32* vals[2] = {nullptr, nullptr};
   u32* sstart = nullptr;
@@ -101,10 +102,11 @@ struct pm_engine {
   long long* halo = nullptr;
   SortPlan sort{};       // Morton-key sort used by priming
   int sort_result = 0;   // which (keys, vals) pair holds the sorted output
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // replayed step without / with the priming sort
-  bool prime_pending = false;  // a peak was (re)loaded: the next step must include the priming sort
+  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};  // replayed step: plain, priming, priming by sort
+  bool prime_pending = false;  // a peak was (re)loaded: the next step must place its particles
   std::vector<char> occupied;  // host view: slots holding a run (dynamic mode FFT extents)
   long long bytes = 0;
+  bool sort_hook = false;      // pm_debug_sort_stall is set
   int* sort_dbg = nullptr;     // device {spin limit, silent tile} of the sort plan (test hook)
   // Host snapshots of the clocks and statistics (pm_snapshot): two pinned buffers, each with the
   // event recorded after its copy.
@@ -115,6 +117,9 @@ struct pm_engine {
     cudaEvent_t done = nullptr;
     bool queued = false;
   } snap[2];
+
+  // Priming by the radix sort: with a refresh period, or while the sort's test hook is set.
+  bool primes_sorted() const { return ((flags >> 8) & 0xFF) != 0 || sort_hook; }
 
   StepArgs args() const {
     StepArgs A{};
@@ -150,6 +155,8 @@ struct pm_engine {
     A.ovf_n = ovf_n;
     A.ovf_in = ovf_in;
     A.new_count = new_count;
+    A.load_count = load_count;
+    A.sorted = primes_sorted() ? 1 : 0;
     A.keys_push = keys[0];
     A.keys_sorted = keys[sort_result];
     A.perm = vals[sort_result];
@@ -222,13 +229,17 @@ struct pm_engine {
     launch_tick(A, stream);
     CU(mark());
     int r = 0;
-    if (with_sort) {  // only steps that prime a peak: no sort launches at all in the steady state
-      if ((r = sort_run<u32>(&sort, keys[0], vals[0], keys[1], vals[1], true, true, stream))) return r;
-      launch_st_starts(A, ntot, stream);
-    }
-    if (with_sort) {
-      launch_layout(A, stream);
-      launch_permute(A, ntot, stream);
+    if (with_sort) {  // only steps that prime a peak: none of these launches in the steady state
+      if (A.sorted) {
+        if ((r = sort_run<u32>(&sort, keys[0], vals[0], keys[1], vals[1], true, true, stream))) return r;
+        launch_st_starts(A, ntot, stream);
+        launch_layout(A, stream);
+        launch_permute(A, ntot, stream);
+      } else {
+        launch_load_count(A, ntot, stream);
+        launch_layout(A, stream);
+        launch_load_place(A, ntot, stream);
+      }
     }
     launch_relayout(A, nst, stream);  // gated: only when a push overflowed a bin
     CU(mark());
@@ -259,7 +270,7 @@ struct pm_engine {
     const bool with_sort = prime_pending;
     prime_pending = false;
     if ((flags & 2) && !(flags & 4)) {
-      cudaGraphExec_t& g = graph[with_sort ? 1 : 0];
+      cudaGraphExec_t& g = graph[!with_sort ? 0 : primes_sorted() ? 2 : 1];
       if (!g) {
         cudaGraph_t cg = nullptr;
         CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -320,7 +331,7 @@ struct pm_engine {
     cudaFree(sort_dbg);
     void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_ref, d_plan, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
                     wpart, eslice, ecount, pushed_a, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
-                    fill[0], fill[1], ovf_n, ovf_in, new_count, keys[0], keys[1], vals[0], vals[1], sstart,
+                    fill[0], fill[1], ovf_n, ovf_in, new_count, load_count, keys[0], keys[1], vals[0], vals[1], sstart,
                     sort_gate, layout_gate, refresh_gate, face, halo};
     for (void* b : bufs) cudaFree(b);
     if (stream) cudaStreamDestroy(stream);
@@ -415,6 +426,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
     P.bin_shift = tight ? 32 : BIN_SLACK_SHIFT;
     P.bin_min = tight ? 0 : BIN_SLACK_MIN;
     P.bin_grow = tight ? 0 : BIN_GROW_STEPS;
+    P.np4 = npart == (long long)c.Np * c.Np * c.Np && c.Np % 4 == 0 ? c.Np / 4 : 0;
     P.L = c.L;
     P.dx = c.L / c.N;
     P.smooth = c.smooth;
@@ -598,6 +610,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   if ((r = E->alloc(&E->ovf_n, npeaks))) return r;
   if ((r = E->alloc(&E->ovf_in, E->nst))) return r;
   if ((r = E->alloc(&E->new_count, E->nst))) return r;
+  if ((r = E->alloc(&E->load_count, E->nst))) return r;
   if ((r = E->alloc(&E->epart, 4 * E->nst))) return r;
   if ((r = E->alloc(&E->wpart, E->nmodeblk * (PM_THREADS / 32)))) return r;
   if ((r = E->alloc(&E->eslice, (size_t)npeaks * ENERGY_SLICES * 5))) return r;
@@ -640,6 +653,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemset(E->ovf_n, 0, sizeof(u32) * npeaks));
   CU(cudaMemset(E->ovf_in, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->new_count, 0, sizeof(u32) * E->nst));
+  CU(cudaMemset(E->load_count, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->layout_gate, 0, sizeof(u32)));
   CU(cudaMemset(E->epart, 0, sizeof(double2) * 4 * E->nst));
   CU(cudaMemset(E->wpart, 0, sizeof(double) * E->nmodeblk * (PM_THREADS / 32)));
@@ -963,6 +977,7 @@ int pm_debug_sort_stall(pm_engine* e, int peak, int spin_limit) {
     v[0] = spin_limit;
     v[1] = (int)tile;
   }
+  e->sort_hook = v[1] >= 0;
   CU(cudaMemcpyAsync(e->sort_dbg, v, sizeof(v), cudaMemcpyHostToDevice, e->stream));
   CU(cudaStreamSynchronize(e->stream));
   return 0;

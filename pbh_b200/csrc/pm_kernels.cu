@@ -428,7 +428,7 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
     want = 0u;
     u32 need = 0u;
     if (C.sortstep) {
-      cnt = ss[i + 1] >= ss[i] ? ss[i + 1] - ss[i] : 0u;
+      cnt = !A.sorted ? A.load_count[P.st_base + i] : ss[i + 1] >= ss[i] ? ss[i + 1] - ss[i] : 0u;
     } else {
       const u32 prev = min(pushed[i].gap, old[i].cap);  // the bin's count before the push
       cnt = bin_count(old[i], pushed[i]) + ovf_in[i];
@@ -541,6 +541,8 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
         cur[i] = BinFill{cnt, cnt, 0u, 0u};
         nxt[i] = BinFill{0u, 0u, 0u, 0u};
         A.ovf_in[P.st_base + i] = 0u;
+        A.load_count[P.st_base + i] = 0u;  // ready for the next load
+        A.new_count[P.st_base + i] = 0u;   // k_load_place counts it up
       } else {
         A.new_count[P.st_base + i] = cnt;
       }
@@ -761,10 +763,94 @@ __global__ void __launch_bounds__(LAYOUT_THREADS) k_tick(const __grid_constant__
 }
 
 // ------------------------------------------------------------------------------------------
-// Priming (particles loaded into the loading area): the Morton-key radix sort, the super-tile
-// starts in the sorted keys, the bin layout from the counts (k_layout), then the gather of the
-// loading area into the bins of the current buffer in sorted order.  Grid-stride loops over a
-// grid of a few CTAs per SM that return at once on the steps where no peak primes.
+// Priming (particles loaded into the loading area): counts per super-tile (k_load_count), the bin
+// layout from them (k_layout), then every particle to the next free slot of its bin of the
+// current buffer (k_load_place).  Nothing needs an order inside a bin, so 4 + 64 bytes per particle
+// do.  A warp takes a 2 x 4 x 4 block of the lattice (load_index), whose nodes the patch strides of
+// the push and the deposit put in distinct shared-memory banks; in the lattice's own order the
+// push was 3.5 % slower afterwards.  At 256^3 the step that primes took 1617 us with the full radix
+// sort of the cell keys, 737 with this; at 512^3 15.3 and 5.7 ms.
+// An engine with a refresh period, whose bins are to be in cell order, primes by that sort
+// instead: the Morton-key radix sort, the super-tile starts in the sorted keys, the layout, then
+// the gather of the loading area into the bins in sorted order (so does one whose sort test hook
+// is set).  All are grid-stride loops that return at once on the steps where no peak primes.
+
+// Calls f(pk) for the peaks with pick(clock), in order, by a whole CTA of PM_THREADS: the clocks are
+// read PM_THREADS at a time instead of one after the other.
+template <class Pick, class F>
+__device__ __forceinline__ void for_peaks(const StepArgs& A, Pick pick, F f) {
+  __shared__ u32 s_mask[PM_THREADS / 32];
+  for (int base = 0; base < A.npeaks; base += PM_THREADS) {
+    const int i = base + threadIdx.x;
+    const u32 m = __ballot_sync(0xffffffffu, i < A.npeaks && pick(A.clocks[i]));
+    if ((threadIdx.x & 31) == 0) s_mask[threadIdx.x >> 5] = m;
+    __syncthreads();
+    for (int w = 0; w < PM_THREADS / 32; ++w)
+      for (u32 b = s_mask[w]; b; b &= b - 1) f(base + 32 * w + __ffs(b) - 1);
+    __syncthreads();
+  }
+}
+
+// Place in the loading area of a warp's lane: the warp-th 2 x 4 x 4 block of an Np^3 lattice (Np a
+// multiple of 4), else the warp-th 32 particles.
+__device__ __forceinline__ long long load_index(const PeakDesc& P, long long warp, int lane) {
+  if (!P.np4) return warp * 32 + lane;
+  const u32 q = (u32)P.np4, w = (u32)warp, row = w / q, bz = w - row * q, bx = row / q, by = row - bx * q;
+  return ((long long)(2 * bx + (lane >> 4)) * (4 * q) + 4 * by + ((lane >> 2) & 3)) * (4 * q) + 4 * bz + (lane & 3);
+}
+
+__global__ void __launch_bounds__(PM_THREADS) k_load_count(const __grid_constant__ StepArgs A) {
+  if (*A.sort_gate == 0u) return;
+  for_peaks(A, [](const PeakClock& c) { return c.dep && c.sortstep; }, [&](int pk) {
+    const PeakDesc& P = A.peaks[pk];
+    const long long n = P.n, nw = (n + 31) / 32;
+    for (long long w = (long long)blockIdx.x * (PM_THREADS / 32) + (threadIdx.x >> 5); w < nw;
+         w += (long long)gridDim.x * (PM_THREADS / 32)) {
+      const long long j = load_index(P, w, threadIdx.x & 31);
+      const u32 S = j < n ? min(A.keys_push[P.p_off + j] >> P.st_shift, (u32)(P.nst - 1)) : 0xffffffffu;
+      const u32 peers = __match_any_sync(0xffffffffu, S);
+      if (j < n && (peers & lanemask_lt()) == 0) atomicAdd(&A.load_count[P.st_base + S], (u32)__popc(peers));
+    }
+  });
+}
+
+__global__ void __launch_bounds__(PM_THREADS) k_load_place(const __grid_constant__ StepArgs A) {
+  if (*A.sort_gate == 0u) return;
+  for_peaks(A, [](const PeakClock& c) { return c.dep && c.sortstep; }, [&](int pk) {
+    const PeakDesc& P = A.peaks[pk];
+    const int sbuf = A.clocks[pk].sbuf;
+    const BinLayout* lay = blay(A, A.clocks[pk].lgen);
+    int4* opos = bpos(A, sbuf);
+    float4* omom = bmom(A, sbuf);
+    const long long n = P.n, nw = (n + 31) / 32;
+    for (long long w = (long long)blockIdx.x * (PM_THREADS / 32) + (threadIdx.x >> 5); w < nw;
+         w += (long long)gridDim.x * (PM_THREADS / 32)) {
+      const long long j = load_index(P, w, threadIdx.x & 31);
+      const bool v = j < n;
+      const u32 S = v ? min(A.keys_push[P.p_off + j] >> P.st_shift, (u32)(P.nst - 1)) : 0xffffffffu;
+      int4 ps;
+      float4 m;
+      if (v) {
+        ps = A.lpos[P.p_off + j];
+        m = A.lmom[P.p_off + j];
+      }
+      const u32 peers = __match_any_sync(0xffffffffu, S);
+      const int leader = __ffs(peers) - 1;
+      u32 r = 0;
+      if (v && (int)(threadIdx.x & 31) == leader) r = atomicAdd(&A.new_count[P.st_base + S], (u32)__popc(peers));
+      r = __shfl_sync(0xffffffffu, r, leader) + (u32)__popc(peers & lanemask_lt());
+      if (!v) continue;
+      const BinLayout L = lay[P.st_base + S];
+      if (r >= L.cap) {  // counts that disagree: never write outside the bin
+        atomicOr(&A.stats[pk].status, 4u);
+        continue;
+      }
+      opos[L.base + r] = ps;
+      omom[L.base + r] = m;
+    }
+  });
+}
+
 __global__ void k_st_starts(StepArgs A, long long ntot) {
   if (*A.sort_gate == 0u) return;
   for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < ntot; j += (long long)gridDim.x * blockDim.x) {
@@ -817,10 +903,9 @@ __global__ void k_permute(StepArgs A, long long ntot) {
 __global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__ StepArgs A) {
   pdl_wait();
   if (*A.layout_gate == 0u) return;
-  for (int pk = 0; pk < A.npeaks; ++pk) {
+  for_peaks(A, [](const PeakClock& c) { return c.dep && c.relayout; }, [&](int pk) {
     const PeakClock& C = A.clocks[pk];
-    const int kind = C.dep ? C.relayout : 0, sbuf = C.sbuf, lgen = C.lgen;
-    if (!kind) continue;
+    const int kind = C.relayout, sbuf = C.sbuf, lgen = C.lgen;
     const PeakDesc& P = A.peaks[pk];
     const bool full = kind == 2;
     const int src = full ? (sbuf ^ 1) : sbuf;
@@ -863,7 +948,7 @@ __global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__
       bpos(A, sbuf)[L.base + cnt - v] = ps;
       bmom(A, sbuf)[L.base + cnt - v] = A.lmom[j];
     }
-  }
+  });
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1828,6 +1913,12 @@ void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s) 
 }
 void launch_tick(const StepArgs& A, cudaStream_t s) {
   pdl_launch(k_tick, dim3(A.npeaks), LAYOUT_THREADS, 0, s, A);
+}
+void launch_load_count(const StepArgs& A, long long ntot, cudaStream_t s) {
+  k_load_count<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A);
+}
+void launch_load_place(const StepArgs& A, long long ntot, cudaStream_t s) {
+  k_load_place<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A);
 }
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s) {
   k_permute<<<stride_grid(ntot, PM_THREADS, 8), PM_THREADS, 0, s>>>(A, ntot);

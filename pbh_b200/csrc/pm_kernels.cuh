@@ -93,7 +93,9 @@ struct StepArgs {
   BinFill* fill[2];            // [super-tile] bin fills of buffers 0 and 1
   u32* ovf_n;                  // [peak] particles in the overflow area (push), reset by the deposit
   u32* ovf_in;                 // [super-tile] overflowed particles whose destination it is
-  u32* new_count;              // [super-tile] particles after a relayout
+  u32* new_count;              // [super-tile] particles after a relayout; particles placed so far (priming)
+  u32* load_count;             // [super-tile] loaded particles (zero outside a priming step)
+  int sorted;                  // this step primes by the radix sort
   u32* keys_push;              // Morton keys written by set_particles / reload (priming sort input)
   const u32* keys_sorted;      // sort output keys
   const u32* perm;             // sort output permutation
@@ -125,6 +127,8 @@ size_t pm_push_smem(int TSmax);
 
 void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s);
 void launch_tick(const StepArgs& A, cudaStream_t s);
+void launch_load_count(const StepArgs& A, long long ntot, cudaStream_t s);
+void launch_load_place(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_st_starts(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_layout(const StepArgs& A, cudaStream_t s);                     // priming peaks
