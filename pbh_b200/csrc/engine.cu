@@ -103,6 +103,10 @@ struct pm_engine {
   SortPlan sort{};       // Morton-key sort used by priming
   int sort_result = 0;   // which (keys, vals) pair holds the sorted output
   cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};  // replayed step: plain, priming, priming by sort
+  // The expansion factor a peak is known to be held at (PS_HOLD with forces there), set by an
+  // explicit step that has completed and dropped by everything else that may move a clock; NaN:
+  // not known, the clock has to be read back.
+  std::vector<double> held_at;
   bool prime_pending = false;  // a peak was (re)loaded: the next step must place its particles
   std::vector<char> occupied;  // host view: slots holding a run (dynamic mode FFT extents)
   long long bytes = 0;
@@ -267,6 +271,7 @@ struct pm_engine {
   }
 
   int step() {
+    held_at.assign(held_at.size(), NAN);
     const bool with_sort = prime_pending;
     prime_pending = false;
     if ((flags & 2) && !(flags & 4)) {
@@ -287,6 +292,7 @@ struct pm_engine {
     return launch_step(with_sort);
   }
   int step_timed(cudaEvent_t* ev, double* phase_ms) {
+    held_at.assign(held_at.size(), NAN);
     const bool with_sort = prime_pending;
     prime_pending = false;
     return launch_step(with_sort, ev, phase_ms);
@@ -298,6 +304,7 @@ struct pm_engine {
     return 0;
   }
   int write_clock(int pk, const PeakClock& c) {
+    held_at[pk] = NAN;
     if (c.state == PS_PRIME) prime_pending = true;
     launch_write_clock(args(), pk, c, stream);
     CU(cudaGetLastError());
@@ -379,6 +386,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   E->npeaks = npeaks;
   E->peaks.resize(npeaks);
   E->occupied.assign(npeaks, 0);
+  E->held_at.assign(npeaks, NAN);
   std::map<int, int> class_of;
   long long poff = 0, roff = 0, stb = 0, mb = 0, sso = 0, fo = 0, ho = 0;
   int TSmax = 1, max_bits = 0;
@@ -742,6 +750,7 @@ int pm_set_particles(pm_engine* e, int peak, const double* x, const double* p, d
   if (!(a0 > 0) || mode < 0 || mode > 2) return -2001;
   CU(cudaSetDevice(e->device));
   const StepArgs A = e->args();
+  e->held_at[peak] = NAN;
   launch_reset_peak(A, peak, a0, mode, param, a_end, max_steps, 0, 0.0, 0, e->stream);
   e->prime_pending = true;
   launch_set_particles(A, peak, e->peaks[peak], x, p, e->stream);
@@ -815,30 +824,34 @@ int pm_step_explicit(pm_engine* e, int peak, double a, double da) {
   if (!e || peak < 0 || peak >= e->npeaks) return -2000;
   if (!(a > 0) || !(da > 0)) return -2001;
   CU(cudaSetDevice(e->device));
-  PeakClock c;
   int r;
-  if ((r = e->read_clock(peak, &c))) return r;
-  // Bring the peak to "forces known at a" (pm3d.py:119-120).
-  if (c.state == PS_HOLD && c.a != a) {
-    c.state = PS_FINALIZE;  // apply the pending kick with the grids it belongs to
-    if ((r = e->write_clock(peak, c)) || (r = e->step()) || (r = e->read_clock(peak, &c))) return r;
+  // A run of steps that each start where the last one ended (the driver's loop): nothing to read
+  // back, one round trip per step instead of two.
+  if (e->held_at[peak] != a) {
+    PeakClock c;
+    if ((r = e->read_clock(peak, &c))) return r;
+    // Bring the peak to "forces known at a" (pm3d.py:119-120).
+    if (c.state == PS_HOLD && c.a != a) {
+      c.state = PS_FINALIZE;  // apply the pending kick with the grids it belongs to
+      if ((r = e->write_clock(peak, c)) || (r = e->step()) || (r = e->read_clock(peak, &c))) return r;
+    }
+    if (c.state == PS_IDLE || c.state == PS_PRIME || (c.state == PS_HOLD && !c.has_delta)) {
+      // A loaded peak (PRIME) has its particles in the loading area already; any other state
+      // holds them in the grouped state, from where they are reloaded.
+      if (c.state != PS_PRIME) launch_reload(e->args(), peak, e->peaks[peak], e->stream);
+      c.a = a;
+      c.a_grid = a;
+      c.mode = SCHED_EXPLICIT;
+      c.state = PS_PRIME;
+      if ((r = e->write_clock(peak, c)) || (r = e->step()) || (r = e->read_clock(peak, &c))) return r;
+    }
+    if (c.state != PS_HOLD) return -2002;
   }
-  if (c.state == PS_IDLE || c.state == PS_PRIME || (c.state == PS_HOLD && !c.has_delta)) {
-    // A loaded peak (PRIME) has its particles in the loading area already; any other state
-    // holds them in the grouped state, from where they are reloaded for the priming sort.
-    if (c.state != PS_PRIME) launch_reload(e->args(), peak, e->peaks[peak], e->stream);
-    c.a = a;
-    c.a_grid = a;
-    c.mode = SCHED_EXPLICIT;
-    c.state = PS_PRIME;
-    if ((r = e->write_clock(peak, c)) || (r = e->step()) || (r = e->read_clock(peak, &c))) return r;
-  }
-  if (c.state != PS_HOLD) return -2002;
-  c.mode = SCHED_EXPLICIT;
-  c.da = da;
-  c.state = PS_RUN;
-  if ((r = e->write_clock(peak, c)) || (r = e->step())) return r;
+  launch_begin_step(e->args(), peak, da, e->stream);
+  if ((r = e->step())) return r;
+  CU(cudaGetLastError());
   CU(cudaStreamSynchronize(e->stream));
+  e->held_at[peak] = a + da;  // as the device's clock adds them
   return 0;
 }
 
@@ -905,6 +918,7 @@ int pm_set_collapse_threshold(pm_engine* e, int peak, double delta_collapse, int
 int pm_release(pm_engine* e, int peak) {
   if (!e || peak < 0 || peak >= e->npeaks) return -2000;
   CU(cudaSetDevice(e->device));
+  e->held_at[peak] = NAN;
   launch_release_peak(e->args(), peak, e->stream);
   CU(cudaGetLastError());
   e->occupied[peak] = 0;
@@ -918,6 +932,7 @@ int pm_load_peak(pm_engine* e, int peak, const double* x, const double* p, doubl
   CU(cudaSetDevice(e->device));
   if (wait_event) CU(cudaStreamWaitEvent(e->stream, (cudaEvent_t)wait_event, 0));
   const StepArgs A = e->args();
+  e->held_at[peak] = NAN;
   launch_reset_peak(A, peak, a0, mode, param, a_end, max_steps, 1, delta_collapse, stop, e->stream);
   launch_set_particles(A, peak, e->peaks[peak], x, p, e->stream);
   CU(cudaGetLastError());

@@ -1687,6 +1687,16 @@ __global__ void k_release_peak(StepArgs A, int pk) {
   A.plan[pk] = plan_of(c, A.peaks[pk]);
 }
 
+// A held peak's next explicit step.
+__global__ void k_begin_step(StepArgs A, int pk, double da) {
+  PeakClock c = A.clocks[pk];
+  c.mode = SCHED_EXPLICIT;
+  c.da = da;
+  c.state = PS_RUN;
+  A.clocks[pk] = c;
+  A.plan[pk] = plan_of(c, A.peaks[pk]);
+}
+
 __global__ void k_write_clock(StepArgs A, int pk, PeakClock c) {
   A.clocks[pk] = c;
   A.plan[pk] = plan_of(c, A.peaks[pk]);
@@ -1979,6 +1989,7 @@ void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double pa
                        int max_steps, int set_thr, double delta_collapse, int stop, cudaStream_t s) {
   k_reset_peak<<<1, 1, 0, s>>>(A, pk, a0, mode, param, a_end, max_steps, set_thr, delta_collapse, stop);
 }
+void launch_begin_step(const StepArgs& A, int pk, double da, cudaStream_t s) { k_begin_step<<<1, 1, 0, s>>>(A, pk, da); }
 void launch_write_clock(const StepArgs& A, int pk, const PeakClock& c, cudaStream_t s) {
   k_write_clock<<<1, 1, 0, s>>>(A, pk, c);
 }

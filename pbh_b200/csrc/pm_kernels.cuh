@@ -152,7 +152,8 @@ int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, flo
 // cleared; set_thr = 1 also sets the collapse threshold and its stop flag (else they are kept).
 void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double param, double a_end,
                        int max_steps, int set_thr, double delta_collapse, int stop, cudaStream_t s);
-// write_clock: the host's clock for a peak, on the stream.
+// begin_step: a held peak runs one explicit step of da next.  write_clock: the host's clock for a peak, on the stream.
+void launch_begin_step(const StepArgs& A, int pk, double da, cudaStream_t s);
 void launch_write_clock(const StepArgs& A, int pk, const PeakClock& c, cudaStream_t s);
 // release: the peak goes idle (no pending kick, no grids), on the stream, without a host round trip.
 void launch_release_peak(const StepArgs& A, int pk, cudaStream_t s);
