@@ -67,6 +67,7 @@ struct pm_engine {
   PeakStats* d_stats = nullptr;
   long long* d_st_base = nullptr;
   int2* d_st_ref = nullptr;             // [super-tile] {peak, index in the peak}
+  long long* d_fix_ref = nullptr;       // [super-tile][8] offsets of the face fix-up
   PeakPlan* d_plan = nullptr;           // digests of the clocks
   long long* d_p_base = nullptr;
   long long* d_mode_base = nullptr;
@@ -133,6 +134,7 @@ struct pm_engine {
     A.sortseg = sort.seg;
     A.st_base = d_st_base;
     A.st_ref = d_st_ref;
+    A.fix_ref = d_fix_ref;
     A.plan = d_plan;
     A.p_base = d_p_base;
     A.mode_base = d_mode_base;
@@ -336,7 +338,7 @@ struct pm_engine {
       if (sn.done) cudaEventDestroy(sn.done);
     }
     cudaFree(sort_dbg);
-    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_ref, d_plan, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
+    void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_ref, d_fix_ref, d_plan, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
                     wpart, eslice, ecount, pushed_a, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
                     fill[0], fill[1], ovf_n, ovf_in, new_count, load_count, keys[0], keys[1], vals[0], vals[1], sstart,
                     sort_gate, layout_gate, refresh_gate, face, halo};
@@ -633,8 +635,20 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemcpy(E->d_st_base, st_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   {
     std::vector<int2> ref((size_t)E->nst);
-    for (int i = 0; i < npeaks; ++i)
-      for (long long t = st_base[i]; t < st_base[i + 1]; ++t) ref[(size_t)t] = make_int2(i, (int)(t - st_base[i]));
+    std::vector<long long> fix(8 * (size_t)E->nst);
+    for (int i = 0; i < npeaks; ++i) {
+      const PeakDesc& P = E->peaks[i];
+      for (int t = 0; t < P.nst; ++t) {
+        const size_t g = (size_t)(st_base[i] + t);
+        ref[g] = make_int2(i | P.TS << 16, t);
+        const u32 sx = pm_compact3((u32)t >> 2), sy = pm_compact3((u32)t >> 1), sz = pm_compact3((u32)t), m = (u32)P.NS - 1;
+        fix[8 * g] = P.face_off + (long long)t * P.fc;
+        for (u32 o = 1; o < 8; ++o)
+          fix[8 * g + o] = P.halo_off + (long long)pm_morton3((sx - (o & 1)) & m, (sy - ((o >> 1) & 1)) & m, (sz - (o >> 2)) & m) * P.hc;
+      }
+    }
+    if ((r = E->alloc(&E->d_fix_ref, fix.size()))) return r;
+    CU(cudaMemcpy(E->d_fix_ref, fix.data(), sizeof(long long) * fix.size(), cudaMemcpyHostToDevice));
     if ((r = E->alloc(&E->d_st_ref, E->nst))) return r;
     CU(cudaMemcpy(E->d_st_ref, ref.data(), sizeof(int2) * E->nst, cudaMemcpyHostToDevice));
   }

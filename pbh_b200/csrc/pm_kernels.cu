@@ -75,12 +75,12 @@ __device__ __forceinline__ u32 bin_count(const BinLayout& L, const BinFill& F) {
 
 // Locate the peak and the peak-local index of this CTA (uniform across the block).
 struct TileRef {
-  int pk, t;
+  int pk, t, TS;
 };
 
 __device__ __forceinline__ TileRef find_tile(const int2* st_ref, int tile) {
   const int2 v = __ldg(st_ref + tile);  // the same for every thread of the CTA
-  return TileRef{v.x, v.y};
+  return TileRef{v.x & 0xFFFF, v.y, v.x >> 16};
 }
 
 // The digest of a clock (see PeakPlan).
@@ -1122,12 +1122,14 @@ __device__ __forceinline__ int halo_index(int lx, int ly, int lz, int T) {
 // face node with (lx, ly, lz) zero where o is one).  nb[o]: the neighbours' halo partials.
 // Adds to the caller's statistics.
 template <int TS>
-__device__ __forceinline__ void fixup_faces(const StepArgs& A, const PeakDesc& P, u32 Y, const long long* const* nb,
-                                            double* rho64, long long& dsum, long long& smax) {
-  constexpr int FC = TS * TS * TS - (TS - 1) * (TS - 1) * (TS - 1);
-  const int N = P.N;
-  const int sx = pm_compact3(Y >> 2), sy = pm_compact3(Y >> 1), sz = pm_compact3(Y);
-  const long long* face = A.face + P.face_off + (long long)Y * FC;
+__device__ __forceinline__ bool fixup_faces(const StepArgs& A, int pk, u32 Y, int only, double* rho64, long long& dsum,
+                                            long long& smax) {
+  // Where this super-tile's face partials and its lower neighbours' halo partials start: a table, so
+  // that the partials are two memory round trips away (the kernel is bound by their latency) and
+  // are on their way before the peak's plan has arrived.
+  const long long* const ref = A.fix_ref + 8LL * blockIdx.x;
+  const long long* const face = A.face + __ldg(ref);
+  auto nb = [&](int o) { return A.halo + __ldg(ref + o); };
   // Three face nodes per thread, one of each face (x: TS x TS nodes; y: without lx = 0; z: without
   // lx = 0 and ly = 0), so that coordinates are shifts and the neighbours that reach a node are
   // known: always the face's own, the others only for edge and corner nodes.  All own partials and
@@ -1138,23 +1140,41 @@ __device__ __forceinline__ void fixup_faces(const StepArgs& A, const PeakDesc& P
   const int cx[3] = {0, u, u}, cy[3] = {u, 0, v}, cz[3] = {v, v, 0};
   long long S[3] = {0, 0, 0};
   constexpr int H1 = (TS + 1) * (TS + 1), H2 = H1 + TS * (TS + 1);  // starts of the y and z planes in the halo
-  if (on[0]) S[0] = __ldcg(face + u * TS + v) + __ldcg(nb[1] + u * (TS + 1) + v);
-  if (on[1]) S[1] = __ldcg(face + TS * TS + (u - 1) * TS + v) + __ldcg(nb[2] + H1 + u * (TS + 1) + v);
-  if (on[2]) S[2] = __ldcg(face + TS * TS + (TS - 1) * TS + (u - 1) * (TS - 1) + v - 1) + __ldcg(nb[4] + H2 + u * TS + v);
-  if (on[0] && u == 0) S[0] += __ldcg(nb[2] + H1 + v) + __ldcg(nb[3] + TS * (TS + 1) + v);
-  if (on[0] && v == 0) S[0] += __ldcg(nb[4] + H2 + u) + __ldcg(nb[5] + u * (TS + 1) + TS);
-  if (on[0] && u == 0 && v == 0) S[0] += __ldcg(nb[6] + H1 + TS) + __ldcg(nb[7] + TS * (TS + 1) + TS);
-  if (on[1] && v == 0) S[1] += __ldcg(nb[4] + H2 + u * TS) + __ldcg(nb[6] + H1 + u * (TS + 1) + TS);
+  if (on[0]) S[0] = __ldcg(face + u * TS + v) + __ldcg(nb(1) + u * (TS + 1) + v);
+  if (on[1]) S[1] = __ldcg(face + TS * TS + (u - 1) * TS + v) + __ldcg(nb(2) + H1 + u * (TS + 1) + v);
+  if (on[2]) S[2] = __ldcg(face + TS * TS + (TS - 1) * TS + (u - 1) * (TS - 1) + v - 1) + __ldcg(nb(4) + H2 + u * TS + v);
+  if (on[0] && u == 0) S[0] += __ldcg(nb(2) + H1 + v) + __ldcg(nb(3) + TS * (TS + 1) + v);
+  if (on[0] && v == 0) S[0] += __ldcg(nb(4) + H2 + u) + __ldcg(nb(5) + u * (TS + 1) + TS);
+  if (on[0] && u == 0 && v == 0) S[0] += __ldcg(nb(6) + H1 + TS) + __ldcg(nb(7) + TS * (TS + 1) + TS);
+  if (on[1] && v == 0) S[1] += __ldcg(nb(4) + H2 + u * TS) + __ldcg(nb(6) + H1 + u * (TS + 1) + TS);
+  const u32 flags = __ldcg(&A.plan[pk].flags);
+  if (only < 0 ? !(flags & PLAN_DEP) : pk != only) return false;
+  if (threadIdx.x == 0) {
+    // Ready for the next push, which fills the other buffer: no arrivals yet, overflow area
+    // empty.  (Here rather than in the deposit, whose particle loop is register-bound.)
+    bfill(A, flags & PLAN_SBUF ? 0 : 1)[blockIdx.x].moved = 0u;
+    if (Y == 0) {
+      A.ovf_n[pk] = 0u;
+      *A.sort_gate = *A.layout_gate = *A.refresh_gate = 0u;  // this step's gated kernels have run
+    }
+  }
+  const PeakDesc& P = A.peaks[pk];
+  const int N = P.N;
+  const int sx = pm_compact3(Y >> 2), sy = pm_compact3(Y >> 1), sz = pm_compact3(Y);
+  const long long nmf = P.n_mean_fix;
+  const double inv = P.inv_fix_nmean;
+  float* const delta = P.delta;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (!on[k]) continue;
-    const long long Dv = S[k] - P.n_mean_fix;
+    const long long Dv = S[k] - nmf;
     const long long node = ((long long)(sx * TS + cx[k]) * N + (sy * TS + cy[k])) * N + (sz * TS + cz[k]);
-    P.delta[node] = (float)((double)Dv * P.inv_fix_nmean);
+    delta[node] = (float)((double)Dv * inv);
     if (rho64) rho64[node] = (double)S[k] * (1.0 / (double)PM_FIX_ONE);
     dsum += Dv;
     smax = S[k] > smax ? S[k] : smax;
   }
+  return true;
 }
 
 // Nearest integer to the exact product a*b for 0 <= a*b < 2^51: one FMA with 2^52 rounds the
@@ -1332,13 +1352,7 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
       __syncthreads();
     }
     const int c1 = min(n, c0 + CH_IT * DEP_THREADS);
-    int k = c0 + threadIdx.x;
-    int4 next = make_int4(0, 0, 0, 0);  // the next sweep's particle, its load in flight
-    if (k < c1) next = pp[k < n0 ? k : k + d1];
-    while (k < c1) {
-      const int4 ps = next;
-      k += DEP_THREADS;
-      if (k < c1) next = pp[k < n0 ? k : k + d1];
+    auto add = [&](const int4& ps) {
       const int c = ps.x;
       const double one = (double)PM_FIX_ONE;
       const double fx = __int_as_float(ps.y), fy = __int_as_float(ps.z), fz = __int_as_float(ps.w);
@@ -1361,6 +1375,22 @@ __device__ __forceinline__ void deposit_super(const StepArgs& A, const PeakDesc&
       } else {
         bad = true;
       }
+    };
+    // Two sweeps per round, the next two sweeps' loads in flight meanwhile, and two rounds unrolled:
+    // one sweep per round took 192 instructions per particle and 134 us at 256^3, this 160 and 123.
+    int k = c0 + threadIdx.x;
+    int4 na = make_int4(0, 0, 0, 0), nb = na;
+    if (k < c1) na = pp[k < n0 ? k : k + d1];
+    if (k + DEP_THREADS < c1) nb = pp[k + DEP_THREADS < n0 ? k + DEP_THREADS : k + DEP_THREADS + d1];
+#pragma unroll 2
+    while (k < c1) {
+      const int4 pa = na, pb = nb;
+      const bool two = k + DEP_THREADS < c1;
+      k += 2 * DEP_THREADS;
+      if (k < c1) na = pp[k < n0 ? k : k + d1];
+      if (k + DEP_THREADS < c1) nb = pp[k + DEP_THREADS < n0 ? k + DEP_THREADS : k + DEP_THREADS + d1];
+      add(pa);
+      if (two) add(pb);
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&A.stats[pk].status, 1u);
@@ -1434,7 +1464,7 @@ __global__ void __launch_bounds__(DEP_THREADS, 4)
   const TileRef tr = find_tile(A.st_ref, tile);
   const PeakDesc P = A.peaks[tr.pk];
   {  // clear the accumulators
-    const int words = 2 * (P.TS == 4 ? patch_size(4) : P.TS == 8 ? patch_size(8) : patch_size(16));
+    const int words = 2 * (tr.TS == 4 ? patch_size(4) : tr.TS == 8 ? patch_size(8) : patch_size(16));
     static_assert((2 * patch_size(4)) % 4 == 0 && (2 * patch_size(8)) % 4 == 0 && (2 * patch_size(16)) % 4 == 0, "");
     for (int i = threadIdx.x; i < words / 4; i += DEP_THREADS)
       reinterpret_cast<uint4*>(s_dep)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -1476,35 +1506,13 @@ __global__ void __launch_bounds__(DEP_THREADS, 4)
 __global__ void __launch_bounds__(FIX_THREADS) k_fixup(const __grid_constant__ StepArgs A, double* rho64, int only) {
   __shared__ long long s_red[FIX_THREADS / 32];
   __shared__ long long s_max[FIX_THREADS / 32];
-  __shared__ const long long* s_nb[8];
   const TileRef tr = find_tile(A.st_ref, blockIdx.x);
   pdl_wait();
-  const u32 flags = __ldcg(&A.plan[tr.pk].flags);
-  const PeakDesc P = A.peaks[tr.pk];
-  if (only < 0 ? !(flags & PLAN_DEP) : tr.pk != only) return;
-  const u32 Y = (u32)tr.t;
-  if (threadIdx.x == 0) {
-    // Ready for the next push, which fills the other buffer: no arrivals yet, overflow area
-    // empty.  (Here rather than in the deposit, whose particle loop is register-bound.)
-    bfill(A, flags & PLAN_SBUF ? 0 : 1)[blockIdx.x].moved = 0u;
-    if (Y == 0) {
-      A.ovf_n[tr.pk] = 0u;
-      *A.sort_gate = *A.layout_gate = *A.refresh_gate = 0u;  // this step's gated kernels have run
-    }
-  }
-  if (threadIdx.x < 8) {
-    const int o = threadIdx.x, NS = P.NS;
-    const u32 sn = pm_morton3((pm_compact3(Y >> 2) - (o & 1)) & (NS - 1), (pm_compact3(Y >> 1) - ((o >> 1) & 1)) & (NS - 1),
-                              (pm_compact3(Y) - (o >> 2)) & (NS - 1));
-    s_nb[o] = A.halo + P.halo_off + (long long)sn * P.hc;
-  }
-  __syncthreads();
   long long dsum = 0, smax = 0;
-  switch (P.TS) {
-    case 4: fixup_faces<4>(A, P, Y, s_nb, rho64, dsum, smax); break;
-    case 8: fixup_faces<8>(A, P, Y, s_nb, rho64, dsum, smax); break;
-    default: fixup_faces<16>(A, P, Y, s_nb, rho64, dsum, smax); break;
-  }
+  const bool active = tr.TS == 4   ? fixup_faces<4>(A, tr.pk, (u32)tr.t, only, rho64, dsum, smax)
+                      : tr.TS == 8 ? fixup_faces<8>(A, tr.pk, (u32)tr.t, only, rho64, dsum, smax)
+                                   : fixup_faces<16>(A, tr.pk, (u32)tr.t, only, rho64, dsum, smax);
+  if (!active) return;  // the whole CTA
   for (int d = 16; d > 0; d >>= 1) {
     dsum += __shfl_xor_sync(0xffffffffu, dsum, d);
     const long long om = __shfl_xor_sync(0xffffffffu, smax, d);

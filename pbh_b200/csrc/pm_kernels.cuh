@@ -75,7 +75,9 @@ struct StepArgs {
   u32* layout_gate;            // 1 when any peak primes or relayouts this step (k_tick)
   u32* refresh_gate;           // 1 when any peak re-sorts its super-tiles this step (k_tick)
   const long long* st_base;    // [npeaks + 1] prefix of super-tiles
-  const int2* st_ref;          // [super-tile] {its peak, its index in the peak} (one load instead of a search)
+  const int2* st_ref;          // [super-tile] {its peak | side << 16, its index in the peak} (one load, no search)
+  const long long* fix_ref;    // [super-tile][8] offsets: its face partials, then the halo partials of its
+                               // lower neighbours o = 1..7 (bit 0: x - 1, bit 1: y - 1, bit 2: z - 1)
   PeakPlan* plan;              // [peak] digest of the clock (see PeakPlan)
   const long long* p_base;     // [npeaks + 1] prefix of particles
   const long long* mode_base;  // [npeaks + 1] prefix of Green blocks
