@@ -59,6 +59,7 @@ struct PeakDesc {
   double inv_fix_nmean;    // 2^-38 / n_mean
   long long p_off, n;      // particle range in the loading/overflow area (and in the sort arrays)
   long long r_off, r_size; // bin region of this peak in each of the two bin buffers
+  long long mv_off;        // offset of this peak's list of relayout pieces
   long long st_base;       // first global super-tile index of this peak
   long long sst_off;       // offset of this peak's super-tile start array (nst + 1 entries)
   long long face_off;      // offset of this peak's face partials (nst * fc)

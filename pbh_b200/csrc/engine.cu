@@ -58,6 +58,7 @@ struct pm_engine {
   int npeaks = 0;
   std::vector<PeakDesc> peaks;
   std::vector<MeshClass> classes;
+  long long nmoves = 0;  // entries of the relayout piece lists
   long long ntot = 0, nst = 0, nmodeblk = 0, nsst = 0, nfc = 0, nhc = 0;
   int TSmax = 0;
   size_t smem_dep = 0, smem_push = 0;
@@ -86,6 +87,8 @@ struct pm_engine {
   u32* ovf_n = nullptr;                        // [peak] overflow-area particles
   u32* ovf_in = nullptr;                       // [super-tile] overflowed arrivals
   u32* new_count = nullptr;                    // [super-tile] count after a relayout
+  uint4* moves = nullptr;                      // relayout pieces
+  u32* n_moves = nullptr;                      // [peak] their number
   u32* load_count = nullptr;                   // [super-tile] loaded particles
   u32* keys[2] = {nullptr, nullptr};
   u32* vals[2] = {nullptr, nullptr};
@@ -162,6 +165,8 @@ struct pm_engine {
     A.ovf_in = ovf_in;
     A.new_count = new_count;
     A.load_count = load_count;
+    A.moves = moves;
+    A.n_moves = n_moves;
     A.sorted = primes_sorted() ? 1 : 0;
     A.keys_push = keys[0];
     A.keys_sorted = keys[sort_result];
@@ -247,7 +252,7 @@ struct pm_engine {
         launch_load_place(A, ntot, stream);
       }
     }
-    launch_relayout(A, nst, stream);  // gated: only when a push overflowed a bin
+    launch_relayout(A, ntot, stream);  // gated: only when a push overflowed a bin
     CU(mark());
     if ((flags >> 8) & 0xFF) launch_tile_sort(A, nst, stream);  // only with a refresh period
     CU(mark());
@@ -340,7 +345,7 @@ struct pm_engine {
     cudaFree(sort_dbg);
     void* bufs[] = {d_peaks, d_clocks, d_stats, d_st_base, d_st_ref, d_fix_ref, d_plan, d_p_base, d_mode_base, d_green_base, d_green_peak, d_gtab, epart,
                     wpart, eslice, ecount, pushed_a, bpos[0], bpos[1], bmom[0], bmom[1], lpos, lmom, lay[0], lay[1],
-                    fill[0], fill[1], ovf_n, ovf_in, new_count, load_count, keys[0], keys[1], vals[0], vals[1], sstart,
+                    fill[0], fill[1], ovf_n, ovf_in, new_count, load_count, moves, n_moves, keys[0], keys[1], vals[0], vals[1], sstart,
                     sort_gate, layout_gate, refresh_gate, face, halo};
     for (void* b : bufs) cudaFree(b);
     if (stream) cudaStreamDestroy(stream);
@@ -454,6 +459,8 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
     P.r_size = (npart + (npart >> BIN_SLACK_SHIFT) + (npart >> BIN_SPARE_SHIFT) +
                 (long long)(BIN_SLACK_MIN + BIN_ALIGN) * P.nst + BIN_ALIGN - 1) / BIN_ALIGN * BIN_ALIGN;
     roff += P.r_size;
+    P.mv_off = E->nmoves;
+    E->nmoves += npart / MOVE_PIECE + 2LL * P.nst;  // two runs per bin, each rounded up to whole pieces
     P.st_base = stb;
     P.sst_off = sso;
     P.face_off = fo;
@@ -621,6 +628,8 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   if ((r = E->alloc(&E->ovf_in, E->nst))) return r;
   if ((r = E->alloc(&E->new_count, E->nst))) return r;
   if ((r = E->alloc(&E->load_count, E->nst))) return r;
+  if ((r = E->alloc(&E->moves, E->nmoves))) return r;
+  if ((r = E->alloc(&E->n_moves, npeaks))) return r;
   if ((r = E->alloc(&E->epart, 4 * E->nst))) return r;
   if ((r = E->alloc(&E->wpart, E->nmodeblk * (PM_THREADS / 32)))) return r;
   if ((r = E->alloc(&E->eslice, (size_t)npeaks * ENERGY_SLICES * 5))) return r;
@@ -676,6 +685,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemset(E->ovf_in, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->new_count, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->load_count, 0, sizeof(u32) * E->nst));
+  CU(cudaMemset(E->n_moves, 0, sizeof(u32) * npeaks));
   CU(cudaMemset(E->layout_gate, 0, sizeof(u32)));
   CU(cudaMemset(E->epart, 0, sizeof(double2) * 4 * E->nst));
   CU(cudaMemset(E->wpart, 0, sizeof(double) * E->nmodeblk * (PM_THREADS / 32)));

@@ -408,12 +408,14 @@ __global__ void __launch_bounds__(PT, 1024 / PT) k_push(const __grid_constant__ 
 // current.  The region, n + n/8 + n/8 + (BIN_SLACK_MIN + BIN_ALIGN) nst slots, covers every base
 // layout.
 // The layout goes into generation clock.lgen (the clock advance switched to it).  When priming,
-// the fills are set to the counts, which the permutation then provides; on a relayout the counts
-// go to new_count, and the relayout copies set the fills.
+// the fills are set to the counts, which the placement then provides.  On a relayout the counts go
+// to new_count, and every bin that moves gets its new fill here, and its particles go as pieces of
+// at most MOVE_PIECE into the peak's list for the relayout copies.
 __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const PeakClock& C) {
-  __shared__ u32 s_w[LAYOUT_THREADS / 32];
+  static_assert(LAYOUT_THREADS == 1024, "one lane per warp of the CTA");
+  __shared__ u32 s_w[2][LAYOUT_THREADS / 32];
   __shared__ unsigned long long s_r[4][LAYOUT_THREADS / 32];
-  __shared__ long long s_carry;
+  __shared__ u32 s_moves;
   const PeakDesc& P = A.peaks[pk];
   const BinLayout* old = blay(A, C.lgen ^ 1) + P.st_base;
   BinLayout* lay = blay(A, C.lgen) + P.st_base;
@@ -498,10 +500,33 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
       want_tot = sg;
     }
   }
-  if (threadIdx.x == 0) s_carry = partial ? (long long)tail : 0;
+  if (threadIdx.x == 0) s_moves = 0u;
   __syncthreads();
   bool bad = false;
-  for (int base = 0; base < P.nst; base += LAYOUT_THREADS) {
+  // The particles of bin i's old place as pieces to its new one, then its new fill.
+  auto move = [&](int i, const BinLayout& to, u32 cnt) {
+    const BinRuns R = bin_runs(old[i], pushed[i]);
+    const int n = min(R.total(), (int)to.cap);
+    const int n0 = min(R.n0, n);
+    const u32 p0 = (u32)(n0 + MOVE_PIECE - 1) / MOVE_PIECE, p1 = (u32)(n - n0 + MOVE_PIECE - 1) / MOVE_PIECE;
+    u32 q = atomicAdd(&s_moves, p0 + p1);
+    if (q + p0 + p1 > (u32)(P.n / MOVE_PIECE + 2LL * P.nst)) {  // more particles than the peak has: corrupted bins
+      bad = true;
+      return;
+    }
+    auto run = [&](int from, int end, long long src) {
+      for (int k = from; k < end; k += MOVE_PIECE, ++q)
+        A.moves[P.mv_off + q] = make_uint4((u32)(src + k), to.base + (u32)k, (u32)min(MOVE_PIECE, end - k), 0u);
+    };
+    run(0, n0, R.b0);
+    run(n0, n, R.b1);
+    cnt = min(cnt, to.cap);
+    (partial ? cur : nxt)[i] = BinFill{cnt, cnt, 0u, 0u};  // a full relayout fills the other buffer
+  };
+  // One bin per thread and round, placed by a prefix sum over the CTA.  (Four consecutive bins per
+  // thread, for fewer rounds, read the tables in 64-byte strides and took 1.4 times as long.)
+  long long carry = partial ? (long long)tail : 0;
+  for (int base = 0, round = 0; base < P.nst; base += LAYOUT_THREADS, round ^= 1) {
     const int i = base + threadIdx.x;
     u32 cnt = 0, cap = 0;
     if (i < P.nst) {
@@ -519,23 +544,27 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
       const u32 t = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += t;
     }
-    if (lane == 31) s_w[warp] = incl;
+    if (lane == 31) s_w[round][warp] = incl;
     __syncthreads();
-    u32 off = 0;
-    for (int w = 0; w < warp; ++w) off += s_w[w];
-    const long long carry = s_carry;
+    u32 total = s_w[round][lane], before = lane < warp ? total : 0u;
+    for (int d = 16; d > 0; d >>= 1) {
+      before += __shfl_xor_sync(0xffffffffu, before, d);
+      total += __shfl_xor_sync(0xffffffffu, total, d);
+    }
     if (i < P.nst) {
       if (partial && cap == 0u) {
         lay[i] = old[i];  // not overflowed: stays where it is
       } else {
-        long long b = carry + off + incl - cap;  // bin start inside the peak's region
-        if (b + cap > P.r_size) {                // counts above the particle total: never past the region
+        long long b = carry + before + incl - cap;  // bin start inside the peak's region
+        if (b + cap > P.r_size) {                   // counts above the particle total: never past the region
           bad = true;
           b = min(b, P.r_size);
           cap = (u32)(P.r_size - b);
           cnt = min(cnt, cap);
         }
-        lay[i] = BinLayout{(u32)(P.r_off + b), cap};
+        const BinLayout to{(u32)(P.r_off + b), cap};
+        lay[i] = to;
+        if (C.relayout) move(i, to, cnt);
       }
       if (C.sortstep) {
         cur[i] = BinFill{cnt, cnt, 0u, 0u};
@@ -547,14 +576,13 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
         A.new_count[P.st_base + i] = cnt;
       }
     }
-    __syncthreads();
-    if (threadIdx.x == LAYOUT_THREADS - 1) s_carry = carry + off + incl;
-    __syncthreads();
+    carry += total;
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&A.stats[pk].status, 4u);
   if (threadIdx.x == 0) {
     if (C.sortstep) A.ovf_n[pk] = 0u;
     if (C.relayout) {
+      A.n_moves[pk] = s_moves;
       A.clocks[pk].relayout = partial ? 1 : 2;
       if (!partial) {  // the full relayout fills the other buffer, which becomes current
         A.clocks[pk].sbuf = C.sbuf ^ 1;
@@ -893,13 +921,14 @@ __global__ void k_permute(StepArgs A, long long ntot) {
 }
 
 // Relayout copies of the peaks whose push overflowed a bin, a grid-stride loop that returns at once
-// in the steps without one.  Full relayout (clock.relayout = 2): every bin the push filled (old
-// layout, other buffer) is copied in order to the start of its new bin in the current buffer.
-// Partial (1): only the bins that got a new place after the last bin move there, inside the
-// current buffer.  Either way the bin's fill is then set to its new count, and each particle of
-// the peak's overflow area goes to the end of its new bin (ovf_in counts down to zero, one rank
-// per particle).  The two parts write disjoint slots and read nothing the other writes, so they
-// need no order between them.
+// in the steps without one.  Full relayout (clock.relayout = 2): every bin is copied from the
+// buffer the push filled to its place in the current buffer.  Partial (1): only the bins that got
+// a new place after the last bin move there, inside the current buffer.  The list of pieces spreads
+// a dense bin over many CTAs (one CTA per bin took 78 us a step through a 256^3 collapse, whose
+// densest bins hold tens of thousands of particles; the pieces take 9).  Then each particle of the peak's
+// overflow area goes to the end of its new bin (ovf_in counts down to zero, one rank per
+// particle).  The two parts write disjoint slots and read nothing the other writes, so they need
+// no order between them.
 __global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__ StepArgs A) {
   pdl_wait();
   if (*A.layout_gate == 0u) return;
@@ -907,27 +936,30 @@ __global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__
     const PeakClock& C = A.clocks[pk];
     const int kind = C.relayout, sbuf = C.sbuf, lgen = C.lgen;
     const PeakDesc& P = A.peaks[pk];
-    const bool full = kind == 2;
-    const int src = full ? (sbuf ^ 1) : sbuf;
-    for (long long t = blockIdx.x; t < P.nst; t += gridDim.x) {
-      const long long g = P.st_base + t;
-      const BinLayout L0 = blay(A, lgen ^ 1)[g], L = blay(A, lgen)[g];
-      if (!full && L.base == L0.base) continue;  // partial relayout: this bin stays as it is (uniform)
-      const BinRuns R = bin_runs(L0, bfill(A, src)[g]);
-      const int4* ip = bpos(A, src);
-      const float4* im = bmom(A, src);
-      int4* op = bpos(A, sbuf) + L.base;
-      float4* om = bmom(A, sbuf) + L.base;
-      const int n = min(R.total(), (int)L.cap);
-      for (int k = threadIdx.x; k < n; k += PM_THREADS) {  // old and new places never overlap
-        const long long j = R.slot(k);
-        op[k] = ip[j];
-        om[k] = im[j];
-      }
-      __syncthreads();  // every thread has read the old fill (a partial relayout rewrites that entry)
-      if (threadIdx.x == 0) {
-        const u32 cnt = min(A.new_count[g], L.cap);
-        bfill(A, sbuf)[g] = BinFill{cnt, cnt, 0u, 0u};
+    const int src = kind == 2 ? (sbuf ^ 1) : sbuf;
+    const int4* ip = bpos(A, src);
+    const float4* im = bmom(A, src);
+    int4* op = bpos(A, sbuf);
+    float4* om = bmom(A, sbuf);
+    const u32 nmv = A.n_moves[pk];
+    for (u32 q = blockIdx.x; q < nmv; q += gridDim.x) {
+      const uint4 mv = A.moves[P.mv_off + q];
+      static_assert(MOVE_PIECE % (4 * PM_THREADS) == 0, "four particles per thread and round");
+      for (u32 k = threadIdx.x; k < mv.z; k += 4 * PM_THREADS) {  // old and new places never overlap
+        int4 p[4];
+        float4 m[4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          if (k + d * PM_THREADS < mv.z) {
+            p[d] = ip[mv.x + k + d * PM_THREADS];
+            m[d] = im[mv.x + k + d * PM_THREADS];
+          }
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          if (k + d * PM_THREADS < mv.z) {
+            op[mv.y + k + d * PM_THREADS] = p[d];
+            om[mv.y + k + d * PM_THREADS] = m[d];
+          }
       }
     }
     const long long novf = (long long)min(A.ovf_n[pk], (u32)P.n);
@@ -1980,8 +2012,8 @@ void launch_tile_sort(const StepArgs& A, long long nst, cudaStream_t s) {
   pdl_launch(k_tile_sort, dim3(stride_grid(nst, 1, 1)), TSORT_THREADS, pm_tile_sort_smem(), s, A, nst);
 }
 void launch_layout(const StepArgs& A, cudaStream_t s) { k_layout<<<(unsigned)A.npeaks, LAYOUT_THREADS, 0, s>>>(A); }
-void launch_relayout(const StepArgs& A, long long nst, cudaStream_t s) {
-  pdl_launch(k_relayout, dim3(stride_grid(nst, 1, RELAYOUT_CTAS_PER_SM)), PM_THREADS, 0, s, A);
+void launch_relayout(const StepArgs& A, long long ntot, cudaStream_t s) {
+  pdl_launch(k_relayout, dim3(stride_grid(ntot, MOVE_PIECE, RELAYOUT_CTAS_PER_SM)), PM_THREADS, 0, s, A);
 }
 void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, int only, cudaStream_t s) {
   const int necta = only < 0 ? A.npeaks * A.eslices : 0;

@@ -52,6 +52,7 @@
 #define BIN_SLACK_MIN 32
 #define BIN_ALIGN 8        // bin bases and capacities are multiples of 8 slots (128 bytes)
 #define LAYOUT_THREADS 1024
+#define MOVE_PIECE 1024        // most particles of one piece of a relayout
 #define RELAYOUT_CTAS_PER_SM 4  // grid of the relayout copies
 
 // Fill of one bin in one buffer: the stayers occupy [base, base + stay), the arrivals
@@ -96,6 +97,8 @@ struct StepArgs {
   u32* ovf_n;                  // [peak] particles in the overflow area (push), reset by the deposit
   u32* ovf_in;                 // [super-tile] overflowed particles whose destination it is
   u32* new_count;              // [super-tile] particles after a relayout; particles placed so far (priming)
+  uint4* moves;                // pieces of a relayout, from mv_off: {source slot, destination slot, particles, -}
+  u32* n_moves;                // [peak] their number
   u32* load_count;             // [super-tile] loaded particles (zero outside a priming step)
   int sorted;                  // this step primes by the radix sort
   u32* keys_push;              // Morton keys written by set_particles / reload (priming sort input)
@@ -134,7 +137,7 @@ void launch_load_place(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_permute(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_st_starts(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_layout(const StepArgs& A, cudaStream_t s);                     // priming peaks
-void launch_relayout(const StepArgs& A, long long nst, cudaStream_t s);    // gated
+void launch_relayout(const StepArgs& A, long long ntot, cudaStream_t s);    // gated
 void launch_tile_sort(const StepArgs& A, long long nst, cudaStream_t s);
 // only >= 0: deposit that peak alone, whether or not its clock asks for it.
 void launch_deposit(const StepArgs& A, long long nst, size_t smem, double* rho64, int only, cudaStream_t s);
