@@ -106,7 +106,7 @@ struct pm_engine {
   long long* halo = nullptr;
   SortPlan sort{};       // Morton-key sort used by priming
   int sort_result = 0;   // which (keys, vals) pair holds the sorted output
-  cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};  // replayed step: plain, priming, priming by sort
+  cudaGraphExec_t graph = nullptr;  // replayed step (one that does not prime)
   // The expansion factor a peak is known to be held at (PS_HOLD with forces there), set by an
   // explicit step that has completed and dropped by everything else that may move a clock; NaN:
   // not known, the clock has to be read back.
@@ -277,26 +277,25 @@ struct pm_engine {
     return 0;
   }
 
+  // One step: the captured graph, except that a step that primes is launched kernel by kernel (it
+  // comes once per load; capturing it cost each engine's first run 90 us, and its replay was no faster).
   int step() {
     held_at.assign(held_at.size(), NAN);
     const bool with_sort = prime_pending;
     prime_pending = false;
-    if ((flags & 2) && !(flags & 4)) {
-      cudaGraphExec_t& g = graph[!with_sort ? 0 : primes_sorted() ? 2 : 1];
-      if (!g) {
-        cudaGraph_t cg = nullptr;
-        CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        int r = launch_step(with_sort);
-        cudaError_t ce = cudaStreamEndCapture(stream, &cg);
-        if (r) return r;
-        CU(ce);
-        CU(cudaGraphInstantiate(&g, cg, 0));
-        cudaGraphDestroy(cg);
-      }
-      CU(cudaGraphLaunch(g, stream));
-      return 0;
+    if (with_sort || !(flags & 2) || (flags & 4)) return launch_step(with_sort);
+    if (!graph) {
+      cudaGraph_t cg = nullptr;
+      CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+      int r = launch_step(false);
+      cudaError_t ce = cudaStreamEndCapture(stream, &cg);
+      if (r) return r;
+      CU(ce);
+      CU(cudaGraphInstantiate(&graph, cg, 0));
+      cudaGraphDestroy(cg);
     }
-    return launch_step(with_sort);
+    CU(cudaGraphLaunch(graph, stream));
+    return 0;
   }
   int step_timed(cudaEvent_t* ev, double* phase_ms) {
     held_at.assign(held_at.size(), NAN);
@@ -319,8 +318,7 @@ struct pm_engine {
   }
 
   ~pm_engine() {
-    for (auto g : graph)
-      if (g) cudaGraphExecDestroy(g);
+    if (graph) cudaGraphExecDestroy(graph);
     for (auto& c : classes) {
       if (c.plans) {
         cufftDestroy(c.r2c);
@@ -643,23 +641,10 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemcpy(E->d_peaks, E->peaks.data(), sizeof(PeakDesc) * npeaks, cudaMemcpyHostToDevice));
   CU(cudaMemcpy(E->d_st_base, st_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   {
-    std::vector<int2> ref((size_t)E->nst);
-    std::vector<long long> fix(8 * (size_t)E->nst);
-    for (int i = 0; i < npeaks; ++i) {
-      const PeakDesc& P = E->peaks[i];
-      for (int t = 0; t < P.nst; ++t) {
-        const size_t g = (size_t)(st_base[i] + t);
-        ref[g] = make_int2(i | P.TS << 16, t);
-        const u32 sx = pm_compact3((u32)t >> 2), sy = pm_compact3((u32)t >> 1), sz = pm_compact3((u32)t), m = (u32)P.NS - 1;
-        fix[8 * g] = P.face_off + (long long)t * P.fc;
-        for (u32 o = 1; o < 8; ++o)
-          fix[8 * g + o] = P.halo_off + (long long)pm_morton3((sx - (o & 1)) & m, (sy - ((o >> 1) & 1)) & m, (sz - (o >> 2)) & m) * P.hc;
-      }
-    }
-    if ((r = E->alloc(&E->d_fix_ref, fix.size()))) return r;
-    CU(cudaMemcpy(E->d_fix_ref, fix.data(), sizeof(long long) * fix.size(), cudaMemcpyHostToDevice));
     if ((r = E->alloc(&E->d_st_ref, E->nst))) return r;
-    CU(cudaMemcpy(E->d_st_ref, ref.data(), sizeof(int2) * E->nst, cudaMemcpyHostToDevice));
+    if ((r = E->alloc(&E->d_fix_ref, 8 * E->nst))) return r;
+    launch_tables(E->d_peaks, E->d_st_base, npeaks, E->nst, E->d_st_ref, E->d_fix_ref, E->stream);
+    CU(cudaGetLastError());
   }
   CU(cudaMemcpy(E->d_p_base, p_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(E->d_mode_base, mode_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));

@@ -1727,6 +1727,21 @@ __global__ void k_release_peak(StepArgs A, int pk) {
   A.plan[pk] = plan_of(c, A.peaks[pk]);
 }
 
+__global__ void k_tables(const PeakDesc* peaks, const long long* st_base, int npeaks, long long nst, int2* st_ref,
+                         long long* fix_ref) {
+  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= nst) return;
+  const int pk = pm_find(st_base, npeaks, g);
+  const PeakDesc& P = peaks[pk];
+  const u32 t = (u32)(g - st_base[pk]), m = (u32)P.NS - 1;
+  const u32 sx = pm_compact3(t >> 2), sy = pm_compact3(t >> 1), sz = pm_compact3(t);
+  st_ref[g] = make_int2(pk | P.TS << 16, (int)t);
+  fix_ref[8 * g] = P.face_off + (long long)t * P.fc;
+  for (u32 o = 1; o < 8; ++o)
+    fix_ref[8 * g + o] =
+        P.halo_off + (long long)pm_morton3((sx - (o & 1)) & m, (sy - ((o >> 1) & 1)) & m, (sz - (o >> 2)) & m) * P.hc;
+}
+
 // A held peak's next explicit step.
 __global__ void k_begin_step(StepArgs A, int pk, double da) {
   PeakClock c = A.clocks[pk];
@@ -2028,6 +2043,10 @@ void launch_green(const StepArgs& A, long long nblocks, cudaStream_t s) {
 void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double param, double a_end,
                        int max_steps, int set_thr, double delta_collapse, int stop, cudaStream_t s) {
   k_reset_peak<<<1, 1, 0, s>>>(A, pk, a0, mode, param, a_end, max_steps, set_thr, delta_collapse, stop);
+}
+void launch_tables(const PeakDesc* peaks, const long long* st_base, int npeaks, long long nst, int2* st_ref,
+                   long long* fix_ref, cudaStream_t s) {
+  k_tables<<<nb(nst, PM_THREADS), PM_THREADS, 0, s>>>(peaks, st_base, npeaks, nst, st_ref, fix_ref);
 }
 void launch_begin_step(const StepArgs& A, int pk, double da, cudaStream_t s) { k_begin_step<<<1, 1, 0, s>>>(A, pk, da); }
 void launch_write_clock(const StepArgs& A, int pk, const PeakClock& c, cudaStream_t s) {

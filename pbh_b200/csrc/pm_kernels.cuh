@@ -153,6 +153,10 @@ int fft_native_init();
 int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
                      const int* slot_peak, int nslots, cudaStream_t s);
 
+// The per-super-tile tables st_ref and fix_ref (see StepArgs).
+void launch_tables(const PeakDesc* peaks, const long long* st_base, int npeaks, long long nst, int2* st_ref,
+                   long long* fix_ref, cudaStream_t s);
+
 // Host-requested per-peak operations.  reset: new schedule from a0, status and sort error
 // cleared; set_thr = 1 also sets the collapse threshold and its stop flag (else they are kept).
 void launch_reset_peak(const StepArgs& A, int pk, double a0, int mode, double param, double a_end,
