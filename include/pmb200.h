@@ -31,7 +31,8 @@ typedef struct pm_engine pm_engine;
 typedef struct {
   int N;          /* mesh side, power of two, 8..1024 */
   int Np;         /* particles per side (n = Np^3) */
-  int tile;       /* super-tile side for push/deposit/grouping: 4, 8 or 16 (0: min(16, N)) */
+  int tile;       /* super-tile side for push/deposit/grouping: 4, 8 or 16 (0: 16, or 8 in an engine with
+                     fewer super-tiles than the GPU has SMs, and at most N) */
   int gradient;   /* 0: spectral -i k (the reference, pm3d.py:111-112); 1: 2-point; 2: 4-point FD */
   double L;       /* box side */
   double smooth;  /* Gaussian force smoothing in cells (pm3d.py:107-108) */
@@ -88,11 +89,11 @@ typedef struct {
  * npeaks = 1 is the plain single run).  Allocates all device memory and cuFFT plans up front; no later call
  * allocates.  flags: bits 8..15 = re-sort every super-tile's particles by cell every that many
  * steps (never if 0, the default: the push keeps them binned by super-tile, and the order inside
- * a bin was measured not to matter); bit 1 = replay the step as a CUDA
+ * a bin was measured not to matter; with a period, loads are also put in cell order); bit 1 = replay the step as a CUDA
  * graph; bit 2 = dynamic mode for served runs: no graph, and each step's FFTs cover only the
  * slots up to the highest one in use in each mesh size (slots are the peaks of one size, in
- * order); bit 3 = the native transform with the Green multiply fused (pm_rfft3_native) for
- * meshes 64^3-512^3 instead of cuFFT; bit 16 = bins without spare capacity (a test mode: almost
+ * order); bit 3 = the native Poisson solve (transforms, Green multiply and gradient) for
+ * meshes 32^3-512^3 instead of cuFFT and a Green kernel; bit 16 = bins without spare capacity (a test mode: almost
  * every step overflows a bin and relayouts; results are the same bit for bit).
  * Replaces: PM3D(N, L, Np, seed, smooth) (pm3d.py:27-37), once per peak. */
 int pm_engine_create(const pm_peak_cfg* cfg, int npeaks, int device, int flags, pm_engine** out);
@@ -105,7 +106,7 @@ int pm_engine_sync(pm_engine* e);
 long long pm_engine_device_bytes(const pm_engine* e);
 
 /* Load particles (lattice order) for one peak at expansion factor a0 and choose its schedule.
- * The peak primes (sort + deposit + forces at a0) on the next pm_run step.
+ * The peak primes (bins, deposit, forces at a0) on the next pm_run step.
  * Replaces: assignment of PM3D.x / PM3D.p after make_ic (pm3d.py:67-68). */
 int pm_set_particles(pm_engine* e, int peak, const double* x, const double* p, double a0, int mode,
                      double param, double a_end, int max_steps);
@@ -115,10 +116,10 @@ int pm_set_particles(pm_engine* e, int peak, const double* x, const double* p, d
 int pm_run(pm_engine* e, int nsteps);
 
 /* pm_run without the graph, with a CUDA event between kernel phases on the engine's stream;
- * adds each phase's device time (ms) into phase_ms[8]: push, energy + clock advance, regroup
- * (priming radix sort with its permutation, bin layouts, relayouts of peaks whose push
- * overflowed a bin), super-tile re-sort (refresh steps), deposit (with the face fix-up), R2C,
- * Green, C2R.  For per-kernel rooflines (no counterpart; the reference times nothing finer than
+ * adds each phase's device time (ms) into phase_ms[8]: push, clock advance (with the bin layouts
+ * of relayouts), regroup (placing loaded particles, relayout copies of peaks whose push
+ * overflowed a bin), super-tile re-sort (refresh steps), deposit (with the face fix-up and the
+ * energies), R2C and Green of the meshes on cuFFT, then the native solves and cuFFT's C2R.  For per-kernel rooflines (no counterpart; the reference times nothing finer than
  * the driver's wall clock, pbhgr/scripts/pm3d_peak.py:24,32,35). */
 int pm_run_timed(pm_engine* e, int nsteps, double* phase_ms);
 /* The engine's CUDA stream (cudaStream_t), for events and stream ordering by callers (no
@@ -182,7 +183,8 @@ int pm_get_delta_async(pm_engine* e, int peak, void* dst);
  * of `peak`'s segment are never published in the first digit pass, so the bounded wait of the
  * tile after it runs out after spin_limit polls; the sort then proceeds with that tile counted
  * as empty (every write stays inside the peak's range, the peak's result is wrong) and the
- * peak's status gets bit 1.  peak < 0 or spin_limit <= 0 restores the normal sort.  The peak
+ * peak's status gets bit 1.  While it is set every load of the engine is grouped by the sort; peak < 0 or
+ * spin_limit <= 0 restores the normal way.  The peak
  * needs more than one sort tile (2048 particles); synchronizes the engine's stream.  No
  * counterpart (the reference has no device waits). */
 int pm_debug_sort_stall(pm_engine* e, int peak, int spin_limit);
@@ -223,7 +225,8 @@ typedef struct {
 int pm_make_ic(const pm_ic_params* prm, double* x_out, double* p_out, double* delta_lin_out, double* noise_rms_out);
 /* pm_make_ic for the recipe peak (kind 1, noise from a device array or noise_seed) ordered on
  * `stream` (a cudaStream_t): returns without waiting, allocates nothing after its first call
- * for a mesh size (its work area is separate from pm_make_ic's), and reports no noise rms.  The
+ * for a mesh size (unless Np exceeds 4 N and every Np before; its work area is separate from
+ * pm_make_ic's), and reports no noise rms.  The
  * same inputs give the same bits as pm_make_ic.  Calls for one mesh size share the work area:
  * issue them on one stream.  kind 0 returns -2003. */
 int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* p_out, void* stream);

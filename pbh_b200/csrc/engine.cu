@@ -228,8 +228,8 @@ struct pm_engine {
   }
 
   // One step for every peak.  With ev != nullptr an event is recorded after each phase and the
-  // phase times (push, energy + advance, relayout, priming sort and refresh, deposit with its face
-  // fix-up, R2C and Green of the cuFFT classes, native solves and C2R) are accumulated.
+  // phase times (push, clock, placing of loads and relayouts, refresh, deposit with its face fix-up
+  // and the energies, R2C and Green of the cuFFT classes, native solves and C2R) are accumulated.
   int launch_step(bool with_sort, cudaEvent_t* ev = nullptr, double* phase_ms = nullptr) {
     const StepArgs A = args();
     int k = 0;

@@ -401,7 +401,6 @@ int ic_work(int device, int N, int path, ICWork** out) {
   if (!w.ok) {
     const long long N3 = (long long)N * N * N, M = (long long)N * N * (N / 2 + 1);
     int rc = 0;
-    int n3[3] = {N, N, N};
     CU(cudaMalloc(&w.field, sizeof(double) * 2 * N3));
     CU(cudaMalloc(&w.spec, sizeof(cufftDoubleComplex) * 2 * M));
     CU(cudaMalloc(&w.spec4, sizeof(cufftDoubleComplex) * 4 * M));
@@ -410,10 +409,6 @@ int ic_work(int device, int N, int path, ICWork** out) {
     CU(cudaMalloc(&w.part, sizeof(double) * (kRmsBlocks + 1)));
     CU(cudaMalloc(&w.count, sizeof(u32)));
     CU(cudaMemset(w.count, 0, sizeof(u32)));
-    CF(cufftPlan3d(&w.d2z, N, N, N, CUFFT_D2Z));
-    CF(cufftPlanMany(&w.d2z2, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, 2));
-    CF(cufftPlanMany(&w.z2d3, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 3));
-    CF(cufftPlanMany(&w.z2d4, 3, n3, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 4));
     w.ok = true;
   done:
     if (rc) {
@@ -424,6 +419,19 @@ int ic_work(int device, int N, int path, ICWork** out) {
   }
   *out = &w;
   return 0;
+}
+
+// A plan of the work area, made when it is first used (each holds cuFFT scratch of its own).
+cufftResult use_plan(cufftHandle* h, int N, cufftType type, int batch, cudaStream_t s) {
+  if (!*h) {
+    int n3[3] = {N, N, N};
+    const cufftResult r = cufftPlanMany(h, 3, n3, nullptr, 1, 0, nullptr, 1, 0, type, batch);
+    if (r != CUFFT_SUCCESS) {
+      *h = 0;
+      return r;
+    }
+  }
+  return cufftSetStream(*h, s);
 }
 
 // Grows a kept buffer to n elements; the stream is drained first, since earlier work on it may
@@ -479,7 +487,7 @@ int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* de
   double* stat = w->part + kRmsBlocks;
   const bool want_noise = (prm->kind == 0 && prm->tail_rms > 0) || (prm->kind == 1 && prm->noise_frac > 0);
   const bool noisy = want_noise && (prm->noise || prm->noise_seed);
-  const cufftHandle inverse = nf == 4 ? w->z2d4 : w->z2d3;
+  cufftHandle& inverse = nf == 4 ? w->z2d4 : w->z2d3;
   Modes g{};
   g.N = N;
   while ((1 << g.l2) < N) ++g.l2;
@@ -490,7 +498,7 @@ int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* de
   g.spec = w->spec;
   g.ns = noisy ? w->spec + M : nullptr;
   g.shape = Shape{prm->kind, (double)N3, L, prm->tail_rms, prm->k1, prm->k2};
-  CU(grow(&w->axis, &w->axis_n, Np, s));
+  CU(grow(&w->axis, &w->axis_n, std::max(Np, 4 * N), s));  // most lattices fit from the first call on
   k_lattice_axis<<<nblk(Np), kThreads, 0, s>>>(N, Np, L, w->axis);
   if (noisy && !prm->noise) {  // seeded device noise
     k_philox_normal<<<nblk((N3 + 3) / 4), kThreads, 0, s>>>(w->field + N3, N3, prm->noise_seed);
@@ -501,14 +509,14 @@ int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* de
     k_field<<<nblk(N3), kThreads, 0, s>>>(N, L, prm->amp, prm->axes[0], prm->axes[1], prm->axes[2], w->spline,
                                           w->spline + m + 1, m, noisy ? prm->noise : nullptr, w->field);
     CU(cudaGetLastError());
-    const cufftHandle forward = noisy ? w->d2z2 : w->d2z;
-    CF(cufftSetStream(forward, s));
+    cufftHandle& forward = noisy ? w->d2z2 : w->d2z;
+    CF(use_plan(&forward, N, CUFFT_D2Z, noisy ? 2 : 1, s));
     CF(cufftExecD2Z(forward, w->field, w->spec));
   } else {
     k_gauss_lines<<<nblk(3LL * N * 32), kThreads, 0, s>>>(N, L, prm->axes[0], prm->axes[1], prm->axes[2], w->lines);
     CU(cudaGetLastError());
     if (noisy) {
-      CF(cufftSetStream(w->d2z, s));
+      CF(use_plan(&w->d2z, N, CUFFT_D2Z, 1, s));
       CF(cufftExecD2Z(w->d2z, prm->noise ? (double*)prm->noise : w->field + N3, w->spec + M));
     }
   }
@@ -520,7 +528,7 @@ int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* de
   }
   k_spectra<<<nblk(M), kThreads, 0, s>>>(g, prm->noise_frac, stat, nf, w->spec4);
   CU(cudaGetLastError());
-  CF(cufftSetStream(inverse, s));
+  CF(use_plan(&inverse, N, CUFFT_Z2D, nf, s));
   CF(cufftExecZ2D(inverse, w->spec4, w->real4));
   k_lattice<<<nblk((long long)Np * Np * Np), kThreads, 0, s>>>(N, Np, L, w->axis, w->real4, x_out, p_out);
   CU(cudaGetLastError());
@@ -566,5 +574,8 @@ extern "C" int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* 
   if (e != cudaSuccess) return -(int)e;
   ICWork* w = nullptr;
   if (int r = ic_work(device, prm->N, 1, &w)) return r;
+  cufftResult f = use_plan(&w->d2z, prm->N, CUFFT_D2Z, 1, (cudaStream_t)stream);  // both now, noise or not
+  if (f == CUFFT_SUCCESS) f = use_plan(&w->z2d3, prm->N, CUFFT_Z2D, 3, (cudaStream_t)stream);
+  if (f != CUFFT_SUCCESS) return -1000 - (int)f;
   return make_ic_on(prm, x_out, p_out, nullptr, w, (cudaStream_t)stream);
 }

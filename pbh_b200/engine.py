@@ -70,7 +70,7 @@ class Engine:
         # bins without spare capacity, so that almost every step overflows and relayouts (a test
         # of that path; same results).
         # dynamic: served runs; no graph, and each step's FFTs cover only the slots in use.
-        # native_fft: 64^3-512^3 meshes use the native transform with the Green multiply fused
+        # native_fft: 32^3-512^3 meshes use the native Poisson solve (native_fft.cu)
         # (False: cuFFT and the separate Green kernel, as for every other mesh size).
         flags = engine_flags(graph, full_every, dynamic, bucket_sort, native_fft, tight_bins)
         self.npeaks = len(self.cfgs)
