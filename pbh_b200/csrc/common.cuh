@@ -70,6 +70,7 @@ struct PeakDesc {
   u32 nh_magic;            // m / (N/2+1) = (umulhi(m, nh_magic) + m) >> nh_shift for 32-bit m
   int nh_shift;
   float* delta;            // N^3 FP32 density contrast (R2C input)
+  u64* rho;                // N^3 node sums of the deposit, zero between steps (null: face partials and k_fixup)
   float2* spec;            // N*N*(N/2+1) complex spectrum (R2C output)
   float2* gspec;           // 3 gradient spectra
   float* force;            // 3 force grids of N^3 (C2R output)

@@ -59,6 +59,7 @@ struct pm_engine {
   std::vector<PeakDesc> peaks;
   std::vector<MeshClass> classes;
   long long nmoves = 0;  // entries of the relayout piece lists
+  bool node_sums = false;  // the deposit adds to grids of node sums (PeakDesc::rho): no face partials
   long long ntot = 0, nst = 0, nmodeblk = 0, nsst = 0, nfc = 0, nhc = 0;
   int TSmax = 0;
   size_t smem_dep = 0, smem_push = 0;
@@ -215,7 +216,7 @@ struct pm_engine {
     for (auto& c : classes) {
       if (c.native) {
         const int x = (flags & 4) ? extent(c) : (int)c.peaks.size();
-        if (int r = fft_native_solve(c.N, c.delta, c.spec, c.gspec, c.force, A, c.slot_peak, x, stream))
+        if (int r = fft_native_solve(c.N, c.delta, c.spec, c.gspec, c.force, A, c.slot_peak, x, node_sums, stream))
           return r;
       } else if (flags & 4) {
         const int x = extent(c);
@@ -257,7 +258,7 @@ struct pm_engine {
     if ((flags >> 8) & 0xFF) launch_tile_sort(A, nst, stream);  // only with a refresh period
     CU(mark());
     launch_deposit(A, nst, smem_dep, nullptr, -1, stream);
-    launch_fixup(A, nst, nullptr, -1, stream);
+    if (!node_sums) launch_fixup(A, nst, nullptr, -1, stream);
     CU(mark());
     if ((r = fft_r2c())) return r;
     CU(mark());
@@ -501,6 +502,16 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   E->smem_dep = pm_deposit_smem(TSmax);
   E->smem_push = pm_push_smem(TSmax);
 
+  // Node sums instead of face partials and a fix-up launch: for engines of a few small meshes,
+  // whose step is a chain of short launches.
+  long long cells = 0;
+  E->node_sums = (E->flags & 8) != 0;
+  for (const PeakDesc& P : E->peaks) {
+    cells += (long long)P.N * P.N * P.N;
+    E->node_sums &= fft_solve_adds_nodes(P.N);
+  }
+  E->node_sums &= cells <= NODE_SUMS_MAX_CELLS;
+
   // Mesh arenas, one per mesh size, peaks of a class contiguous for batched cuFFT plans.
   for (auto& mc : E->classes) {
     const long long N = mc.N, N3 = N * N * N, M = N * N * (N / 2 + 1);
@@ -524,6 +535,13 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
       mc.native = true;
       if ((r = E->alloc(&mc.slot_peak, (size_t)B))) return r;
       CU(cudaMemcpy(mc.slot_peak, mc.peaks.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
+      if (E->node_sums) {  // in the second and third spectra, which the solve leaves alone
+        for (int k = 0; k < B; ++k) {
+          PeakDesc& P = E->peaks[mc.peaks[k]];
+          P.rho = (u64*)(P.gspec + M);
+          CU(cudaMemsetAsync(P.rho, 0, sizeof(u64) * N3, E->stream));
+        }
+      }
       for (int k = 0; k < B; ++k) {
         E->peaks[mc.peaks[k]].native_fft = 1;
         E->peaks[mc.peaks[k]].nwpart = fft_solve_partials((int)N);

@@ -31,7 +31,7 @@
 //   k_solve_rows  inverse Y of the three components
 //   k_fft_z_c2r   the real inverse along z of the three components, written as force rows
 // Up to 128^3 the y-z slab of one x fits an SM:
-//   k_slab_fwd    Z and Y of a slab
+//   k_slab_fwd    Z and Y of a slab (in engines of a few meshes up to 64^3, after finishing delta)
 //   k_solve_cols  as above
 //   k_slab_inv    inverse Y and Z of a slab, one component
 // Per cell the five passes move 8 + 8 + 12 + 20 + 24 = 72 bytes, the three 8 + 12 + 20 = 40; the six
@@ -564,6 +564,9 @@ struct SGeo {
   // The inverse runs at 64 registers; two CTAs of 128^3 then have 512 threads each, and its one line
   // too many takes a second round.
   static constexpr int ITHREADS = N == 128 ? 512 : THREADS;
+  // The forward kernel that finishes the deposit: more threads than lines, for the node sums.
+  static constexpr bool SUMS = N <= 64;
+  static constexpr int STHREADS = N == 64 ? 256 : 128;
   static constexpr long long N2 = (long long)N * N;
 };
 template <bool INV, int N, int THREADS>
@@ -574,29 +577,80 @@ __device__ __forceinline__ void load_slab_tw(float2* tz, float2* ty, float2* tw)
   for (int i = threadIdx.x; i <= G::M; i += THREADS) tw[i] = tw_global<INV, N>(i);
 }
 
-// Forward: densities in[slot][x][y][z] -> spectra out[slot][kz][x][ky].  grid (N, nslots).
-template <int N>
-__global__ void __launch_bounds__(SGeo<N>::THREADS, SGeo<N>::MINB)
+// The plane x of a mesh out of its node sums S (PeakDesc::rho, written by the deposit's adds): delta =
+// S / n_mean - 1 to the mesh and to the rows of buf (X float2 apart), the sums cleared for the next
+// step.  Latency is all of it, so a thread has all its loads in flight (four at a time, with the
+// clearing stores between them, took 5 us longer at 64^3).  And, as k_fixup does for other meshes, the next push's arrival counts and overflow area
+// emptied and this step's gates closed.  dsum, smax: the thread's part of the mass defect and of
+// the largest sum.
+template <int N, int THREADS, int X>
+__device__ __forceinline__ void finish_nodes(const StepArgs& A, int pk, int x, float2* buf, long long& dsum,
+                                             long long& smax) {
+  constexpr int PAIRS = N * N / 2, PER = PAIRS / THREADS;  // pairs per thread, all in flight at once
+  static_assert(PAIRS % THREADS == 0 && PER <= 8, "");
+  const PeakDesc& P = A.peaks[pk];
+  const long long nmf = P.n_mean_fix;
+  const double inv = P.inv_fix_nmean;
+  ulonglong2* const src = reinterpret_cast<ulonglong2*>(P.rho + (long long)x * N * N);
+  float2* const dst = reinterpret_cast<float2*>(P.delta + (long long)x * N * N);
+  ulonglong2 S[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) S[k] = __ldcg(src + threadIdx.x + k * THREADS);
+  dsum = smax = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = threadIdx.x + k * THREADS;
+    const long long a = (long long)S[k].x, b = (long long)S[k].y, da = a - nmf, db = b - nmf;
+    const float2 d = make_float2((float)((double)da * inv), (float)((double)db * inv));
+    buf[i / (N / 2) * X + i % (N / 2)] = d;
+    dst[i] = d;
+    src[i] = make_ulonglong2(0, 0);
+    dsum += da + db;
+    smax = max(smax, max(a, b));
+  }
+  BinFill* const next = (A.plan[pk].flags & PLAN_SBUF ? A.fill[0] : A.fill[1]) + P.st_base;
+  for (int i = x * THREADS + threadIdx.x; i < P.nst; i += N * THREADS) next[i].moved = 0u;
+  if (x == 0 && threadIdx.x == 0) {
+    A.ovf_n[pk] = 0u;
+    *A.sort_gate = *A.layout_gate = *A.refresh_gate = 0u;
+  }
+}
+
+// Forward: densities in[slot][x][y][z] (ADDS: made here from the deposit's node sums) -> spectra
+// out[slot][kz][x][ky].  grid (N, nslots).
+template <int N, int THREADS, bool ADDS>
+__global__ void __launch_bounds__(THREADS, ADDS ? 3 : SGeo<N>::MINB)
     k_slab_fwd(const float* in, float2* out, const __grid_constant__ StepArgs A, const int* slot_peak) {
   using G = SGeo<N>;
   extern __shared__ __align__(16) float2 s_slab[];
   float2 *const xb = s_slab, *const tz = xb + G::BUF, *const ty = tz + 16 * G::TZ, *const tw = ty + 16 * G::TY;
-  load_slab_tw<false, N, G::THREADS>(tz, ty, tw);
+  load_slab_tw<false, N, THREADS>(tz, ty, tw);
   const int x = blockIdx.x, slot = blockIdx.y;
   pdl_wait();
   if (!slot_active(A, slot_peak, slot)) return;
   float2 v[16], u[16];
+  [[maybe_unused]] long long dsum, smax;
   const int tid = threadIdx.x;
   const bool zt = tid < N * G::TZ;  // whole warps
   const int t = tid % G::TZ, y = tid / G::TZ;
-  if (zt) {
-    const float2* src = reinterpret_cast<const float2*>(in + ((long long)slot * N + x) * G::N2 + y * N);
+  float2* const row = xb + y * G::X;
+  if constexpr (ADDS) {
+    finish_nodes<N, THREADS, G::X>(A, slot_peak[slot], x, xb, dsum, smax);
+    __syncthreads();  // density rows and tables
+    if (zt) {
 #pragma unroll
-    for (int n1 = 0; n1 < 16; ++n1) v[n1] = __ldcg(src + G::TZ * n1 + t);
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = row[G::TZ * n1 + t];
+      __syncwarp();
+    }
+  } else {
+    if (zt) {
+      const float2* src = reinterpret_cast<const float2*>(in + ((long long)slot * N + x) * G::N2 + y * N);
+#pragma unroll
+      for (int n1 = 0; n1 < 16; ++n1) v[n1] = __ldcg(src + G::TZ * n1 + t);
+    }
+    __syncthreads();  // tables
   }
-  __syncthreads();  // tables
   if (zt) {
-    float2* const row = xb + y * G::X;
     line_fft<false, G::TZ>(v, u, row, tz, t);
     __syncwarp();
 #pragma unroll
@@ -615,11 +669,22 @@ __global__ void __launch_bounds__(SGeo<N>::THREADS, SGeo<N>::MINB)
     v[n1] = cadd(E, cmul(wk, O));
   }
   __syncthreads();  // the z lines are read; their memory becomes the exchange rows
-  line_fft<false, G::TY>(v, u, xb + k * G::C, ty, ty_);
-  if (tid / G::TY > G::M) return;
-  float2* dst = out + ((long long)slot * G::NH + k) * G::N2 + x * N;
+  if ((tid & ~31) / G::TY <= G::M) line_fft<false, G::TY>(v, u, xb + k * G::C, ty, ty_);  // whole warps
+  if (tid / G::TY <= G::M) {
+    float2* dst = out + ((long long)slot * G::NH + k) * G::N2 + x * N;
 #pragma unroll
-  for (int p = 0; p < 16; ++p) dst[line_k<G::TY>(ty_, p)] = u[p];
+    for (int p = 0; p < 16; ++p) dst[line_k<G::TY>(ty_, p)] = u[p];
+  }
+  if constexpr (ADDS) {  // the peak's statistics, off the path of the transform
+    for (int d = 16; d > 0; d >>= 1) {
+      dsum += __shfl_xor_sync(0xffffffffu, dsum, d);
+      smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, d));
+    }
+    if ((tid & 31) == 0) {
+      atomicAdd((u64*)&A.stats[slot_peak[slot]].mass_defect, (u64)dsum);
+      atomicMax(&A.stats[slot_peak[slot]].max_fix, (u64)smax);
+    }
+  }
 }
 
 // Inverse of one component: the x component from B (gspec's first field), y and z from A (spec) times
@@ -704,12 +769,16 @@ int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
 
 template <int N>
 int solve_n(const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A, const int* slot_peak,
-            int nslots, cudaStream_t s) {
+            int nslots, bool sums, cudaStream_t s) {
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nslots * G::NH);
   if constexpr (N <= 128) {
     using S = SGeo<N>;
-    pdl_launch(k_slab_fwd<N>, dim3(N, nslots), S::THREADS, S::SMEM, s, delta, spec, A, slot_peak);
+    if constexpr (S::SUMS) {
+      if (sums) pdl_launch(k_slab_fwd<N, S::STHREADS, true>, dim3(N, nslots), S::STHREADS, S::SMEM, s, delta, spec, A, slot_peak);
+    }
+    if (!S::SUMS || !sums)
+      pdl_launch(k_slab_fwd<N, S::THREADS, false>, dim3(N, nslots), S::THREADS, S::SMEM, s, delta, spec, A, slot_peak);
     pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
     pdl_launch(k_slab_inv<N>, dim3(3 * N, nslots), S::ITHREADS, S::SMEM, s, spec, gspec, force, A, slot_peak);
   } else {
@@ -740,6 +809,8 @@ int c2r_n(const float2* spec, float2* work, float* out, int nfields, cudaStream_
 
 bool fft_native_size(int N) { return N == 64 || N == 128 || N == 256 || N == 512; }
 bool fft_solve_size(int N) { return N == 32 || fft_native_size(N); }
+
+bool fft_solve_adds_nodes(int N) { return N == 32 || N == 64; }
 // Potential-energy partials of a solve: one per warp of k_solve_cols, N / 16 threads per column.
 long long fft_solve_partials(int N) { return (long long)(N / 2 + 1) * N * (N / 16) / 32; }
 
@@ -759,7 +830,7 @@ int fft_native_init() {
   smem(k_solve_cols<128>, PGeo<128>::COLS_SMEM);
   smem(k_solve_cols<256>, PGeo<256>::COLS_SMEM);
   smem(k_solve_cols<512>, PGeo<512>::COLS_SMEM);
-  smem(k_slab_fwd<128>, SGeo<128>::SMEM);
+  smem(k_slab_fwd<128, SGeo<128>::THREADS, false>, SGeo<128>::SMEM);
   smem(k_slab_inv<128>, SGeo<128>::SMEM);
   return e == cudaSuccess ? 0 : -(int)e;
 }
@@ -767,14 +838,14 @@ int fft_native_init() {
 // delta fields [slot][x][y][z] -> 3 force grids per slot [slot][comp][x][y][z] (the Poisson solve);
 // spec [slot][kz][.][.] and gspec [slot][comp][kz][.][.] are work space.
 int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
-                     const int* slot_peak, int nslots, cudaStream_t s) {
+                     const int* slot_peak, int nslots, bool sums, cudaStream_t s) {
   if (nslots <= 0) return 0;
   switch (N) {
-    case 32: return solve_n<32>(delta, spec, gspec, force, A, slot_peak, nslots, s);
-    case 64: return solve_n<64>(delta, spec, gspec, force, A, slot_peak, nslots, s);
-    case 128: return solve_n<128>(delta, spec, gspec, force, A, slot_peak, nslots, s);
-    case 256: return solve_n<256>(delta, spec, gspec, force, A, slot_peak, nslots, s);
-    case 512: return solve_n<512>(delta, spec, gspec, force, A, slot_peak, nslots, s);
+    case 32: return solve_n<32>(delta, spec, gspec, force, A, slot_peak, nslots, sums, s);
+    case 64: return solve_n<64>(delta, spec, gspec, force, A, slot_peak, nslots, sums, s);
+    case 128: return solve_n<128>(delta, spec, gspec, force, A, slot_peak, nslots, sums, s);
+    case 256: return solve_n<256>(delta, spec, gspec, force, A, slot_peak, nslots, sums, s);
+    case 512: return solve_n<512>(delta, spec, gspec, force, A, slot_peak, nslots, sums, s);
     default: return -2000;
   }
 }

@@ -29,6 +29,12 @@
 #define PUSH_THREADS_SMALL 128
 #define DEP_THREADS 256    // deposit CTA (4 per SM)
 #define GREEN_MODES 4      // modes per thread of the Green kernel (a block covers PM_THREADS * GREEN_MODES)
+// Most cells of an engine whose deposit adds its node sums to the meshes (PeakDesc::rho) instead of
+// leaving face partials to a fix-up launch.  Per step, fix-up and sums: 30.8 and 28.9 us for one
+// 32^3 peak, 41.0 and 37.0 for eight, 39.2 and 37.0-39.0 for one of 64^3, 51.3 and 47.3 for two
+// (2^19 cells), 72.1 and 72.1 for four, 117.6 and 121.5 for eight: the sums' 16 bytes per cell and
+// wider loads then cost more than the launch that they save.  At 128^3: 109 and 123.
+#define NODE_SUMS_MAX_CELLS (1LL << 19)
 #define ENERGY_SLICES 128  // most CTAs per peak of the energy reduction
 #define ENERGY_THREADS DEP_THREADS  // they ride in the deposit's launch
 #define FIX_THREADS 256    // face fix-up CTA
@@ -149,9 +155,10 @@ void launch_green(const StepArgs& A, long long nblocks, cudaStream_t s);
 bool fft_native_size(int N);
 bool fft_solve_size(int N);
 long long fft_solve_partials(int N);
+bool fft_solve_adds_nodes(int N);
 int fft_native_init();
 int fft_native_solve(int N, const float* delta, float2* spec, float2* gspec, float* force, const StepArgs& A,
-                     const int* slot_peak, int nslots, cudaStream_t s);
+                     const int* slot_peak, int nslots, bool sums, cudaStream_t s);
 
 // The per-super-tile tables st_ref and fix_ref (see StepArgs).
 void launch_tables(const PeakDesc* peaks, const long long* st_base, int npeaks, long long nst, int2* st_ref,
