@@ -54,7 +54,7 @@ def parse():
                     help="timed window of the CPU sample (default 30 s for --impl reference, 10 s for cpu_baseline)")
     ap.add_argument("--tiles", default="auto", help="super-tile side: 'auto' (autotuned per mesh size) or 4/8/16")
     ap.add_argument("--fft", choices=["cufft", "native"], default="native",
-                    help="64^3-512^3 transforms: cuFFT, or the native kernels with the Green multiply fused")
+                    help="forces of 32^3-512^3 meshes: cuFFT with a Green kernel, or the native solve")
     return ap.parse_args()
 
 
@@ -319,22 +319,35 @@ def algorithmic_bytes(phase: str, n: int, cells: int, modes: int, npass: int) ->
 
 
 PHASES = ["push", "advance", "regroup", "refresh", "deposit", "r2c", "green", "c2r"]
-NATIVE_FFT_SIZES = (64, 128, 256, 512)   # meshes the native transform serves (the others use cuFFT)
+NATIVE_FFT_SIZES = (64, 128, 256, 512)   # meshes with a plain native transform
+NATIVE_SOLVE_SIZES = (32, 64, 128, 256, 512)   # meshes whose forces the native solve makes (the others use cuFFT)
 
 
 def launches_per_step(sizes, fft: str) -> int:
-    """Our kernel launches in one steady (non-priming) step of an ensemble with these mesh sizes:
-    push, energy, advance, bin layout and 2 relayout copies (gated: they return at once unless a
+    """Kernel launches of one steady (non-priming) step when every stage is a launch of its own (the
+    engine merges several, see step_launches): push, energy, advance, bin layout and 2 relayout copies (gated: they return at once unless a
     push overflowed a bin), super-tile sort, deposit, fix-up and Green (10); the native
     transform adds 6 per mesh size it serves (3 passes each way) and drops the Green launch when
     it serves every mesh.  The radix sort runs only in steps that prime a peak."""
     native = {n for n in sizes if fft == "native" and n in NATIVE_FFT_SIZES}
     return 10 + 6 * len(native) - (1 if native and all(n in native for n in sizes) else 0)
 
+
+def step_launches(sizes, fft: str, refresh: bool = False) -> int:
+    """Our kernel launches in one steady (non-priming) step of an ensemble with these mesh sizes:
+    push, clock, relayout copies (gated: they return at once unless a push overflowed a bin),
+    deposit (with the energies) and fix-up; the super-tile re-sort with a refresh period; per
+    natively solved mesh size 3 launches up to 128^3 and 5 above; the Green kernel when a mesh size
+    is on cuFFT (whose own launches are not ours)."""
+    native = {n for n in sizes if fft == "native" and n in NATIVE_SOLVE_SIZES}
+    rest = any(n not in native for n in sizes)
+    return 5 + int(refresh) + sum(3 if n <= 128 else 5 for n in native) + int(rest)
+
+
 # DRAM bytes (read + write) per launch from single-kernel ncu captures of the plain 256^3 run
 # (the Green kernel's from the same run with cuFFT transforms), per particle (per mode for Green),
 # scaled to a launch by the particles (modes) it processes; deposit includes its face fix-up.
-NCU_TRAFFIC = {"push": 77.10, "deposit": 26.94, "green_per_mode": 25.89}
+NCU_TRAFFIC = {"push": 77.00, "deposit": 27.08, "green_per_mode": 25.89}
 
 
 def replica_throughput(t_local: float, n_local: int, steps: int, dist=None, device="cpu"):
@@ -499,8 +512,8 @@ def run_ours(args):
         ph_late = ens.timed_phases(4)
         late["phase_ms"] = {name: round(float(v), 4) for name, v in zip(PHASES, ph_late)}
     cells = sum(s.N ** 3 for s in specs)
-    # modes the Green kernel handles (the native 256^3 transform applies its own multiply)
-    modes = sum(s.N * s.N * (s.N // 2 + 1) for s in specs if not (args.fft == "native" and s.N in NATIVE_FFT_SIZES))
+    # modes the Green kernel handles (the native solve applies its own multiply)
+    modes = sum(s.N * s.N * (s.N // 2 + 1) for s in specs if not (args.fft == "native" and s.N in NATIVE_SOLVE_SIZES))
     kern = {}
     for k, name in enumerate(PHASES):
         b = algorithmic_bytes(name, n_step, cells, modes, npass)
@@ -539,8 +552,9 @@ def run_ours(args):
                                                                                        args.warmup + args.steps],
                        "super_tiles": {str(k): v for k, v in sorted(tiles.items())},
                        "relayouts_timed": relayouts,
-                       "fft_64_to_512": "native (Green fused into the inverse)" if args.fft == "native" else "cuFFT"},
-            "clocks": clocks, "gpu_launches": args.steps * launches_per_step([sp.N for sp in specs], args.fft),
+                       "fft_32_to_512": "native solve (Green multiply between the x transforms)" if args.fft == "native"
+                       else "cuFFT"},
+            "clocks": clocks, "gpu_launches": args.steps * step_launches([sp.N for sp in specs], args.fft, args.full_sort),
             "roofline": roofline}
     if late is not None:
         line["late_window"] = late

@@ -1136,7 +1136,7 @@ __global__ void __launch_bounds__(TSORT_THREADS) k_tile_sort(StepArgs A, long lo
 // neighbours) are written as 64-bit partials.
 //
 // The face fix-up (k_fixup, the next launch) completes the face nodes: own partial plus the
-// lower neighbours' halo partials.
+// lower neighbours' halo partials.  (Engines of a few small meshes: see add_nodes.)
 // Integer sums make the result independent of particle order, bit for bit; no float atomics.
 __device__ __forceinline__ int face_index(int lx, int ly, int lz, int T) {
   if (lx == 0) return ly * T + lz;

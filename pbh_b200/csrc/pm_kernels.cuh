@@ -10,16 +10,19 @@
 //              to the bin of the super-tile it is now in, in the other buffer (stayers ranked in
 //              shared memory, arrivals by an atomic on the destination's count); a particle
 //              for which the destination bin has no room goes to the peak's overflow area
-//   energy     per peak: momentum, kinetic and potential energy, Layzer-Irvine integral
-//   advance    per peak clock; a peak whose push overflowed relayouts this step
-//   regroup    relayout (new capacities from the counts, bins and overflow area copied into the
-//              buffer the push read); every full_every steps each super-tile's particles are
-//              re-sorted by cell (local counting sort); when particles are first loaded, a full
-//              Morton-key radix sort of the loading area and a permutation into fresh bins
+//   tick       per peak: the clock; a peak whose push overflowed gets a new layout and the list of
+//              pieces to move
+//   relayout   gated: those pieces, and the overflow area, into the buffer the push read (with a
+//              refresh period each super-tile's particles are then re-sorted by cell)
 //   deposit    per super-tile: CIC density of its particles into (TS+1)^3 nodes; interior nodes
-//              final, face and upper-halo nodes as 64-bit partials
+//              final, face and upper-halo nodes as 64-bit partials.  In front of its grid the
+//              energy CTAs: momentum, kinetic and potential energy, Layzer-Irvine integral
 //   fixup      per super-tile: face nodes = own partial + the lower neighbours' halo partials
-//   R2C, Green, C2R (x3)
+//   solve      delta -> three force grids (native_fft.cu; other sizes: cuFFT and k_green)
+// A step that primes a peak places its loaded particles before the relayout (k_load_count, k_layout,
+// k_load_place; with a refresh period a full Morton-key radix sort and a permutation).
+// Engines of a few small meshes have no fixup: the deposit adds every node sum to a grid
+// (NODE_SUMS_MAX_CELLS).
 #pragma once
 #include "common.cuh"
 #include "sort.cuh"
