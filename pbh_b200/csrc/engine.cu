@@ -656,9 +656,12 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   if ((r = E->alloc(&E->refresh_gate, 1))) return r;
   if ((r = E->alloc(&E->face, E->nfc))) return r;
   if ((r = E->alloc(&E->halo, E->nhc))) return r;
-  CU(cudaMemcpy(E->d_peaks, E->peaks.data(), sizeof(PeakDesc) * npeaks, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(E->d_st_base, st_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice));
   {
+    // On the engine's stream, like the kernel that reads them: a plain copy from pageable memory may
+    // return before it has landed, and the engine's stream does not wait for the default one.
+    CU(cudaMemcpyAsync(E->d_peaks, E->peaks.data(), sizeof(PeakDesc) * npeaks, cudaMemcpyHostToDevice, E->stream));
+    CU(cudaMemcpyAsync(E->d_st_base, st_base.data(), sizeof(long long) * (npeaks + 1), cudaMemcpyHostToDevice,
+                       E->stream));
     if ((r = E->alloc(&E->d_st_ref, E->nst))) return r;
     if ((r = E->alloc(&E->d_fix_ref, 8 * E->nst))) return r;
     launch_tables(E->d_peaks, E->d_st_base, npeaks, E->nst, E->d_st_ref, E->d_fix_ref, E->stream);
