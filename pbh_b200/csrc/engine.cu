@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <new>
@@ -921,11 +922,9 @@ int pm_get_counts(pm_engine* e, int peak, double* counts) {
   int r;
   if ((r = e->read_clock(peak, &c))) return r;
   if (!c.has_delta) return -2002;
-  PeakStats st;
-  CU(cudaMemcpy(&st, e->d_stats + peak, sizeof(PeakStats), cudaMemcpyDeviceToHost));
-  st.max_fix = 0;
-  st.mass_defect = 0;
-  CU(cudaMemcpy(e->d_stats + peak, &st, sizeof(PeakStats), cudaMemcpyHostToDevice));
+  // max_fix and mass_defect, cleared on the stream of the kernels that add to them.
+  static_assert(offsetof(PeakStats, max_fix) == 0 && offsetof(PeakStats, mass_defect) == 8, "the first two fields");
+  CU(cudaMemsetAsync(e->d_stats + peak, 0, 16, e->stream));
   // Same kernels with the extra float64 output; delta is rewritten with identical values.
   launch_deposit(e->args(), e->nst, e->smem_dep, counts, peak, e->stream);
   launch_fixup(e->args(), e->nst, counts, peak, e->stream);

@@ -45,3 +45,9 @@ def test_the_kernel_of_the_engine_s_creation_reads_finished_tables():
         read = re.findall(r"E->d_\w+", m.group(1))
         late = [c for c in unordered(text, m.start()) if any(re.match(re.escape(r) + r"\s*,", c) for r in read)]
         assert not late, late
+
+
+def test_the_counts_kernels_start_from_cleared_statistics():
+    text = body("engine.cu", "int pm_get_counts(")
+    at = text.index("launch_deposit(")
+    assert "max_fix" in text[:at] and not unordered(text, at)
