@@ -822,6 +822,9 @@ int fft_native_init() {
     h[k] = make_float2((float)cos(a), (float)sin(a));
   }
   cudaError_t e = cudaMemcpyToSymbol(g_tw, h, sizeof(h));
+  // The copy may return before it has landed, and the first transform may be on a stream that does
+  // not wait for the default one.
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   auto smem = [&](auto* kernel, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };

@@ -51,3 +51,11 @@ def test_the_counts_kernels_start_from_cleared_statistics():
     text = body("engine.cu", "int pm_get_counts(")
     at = text.index("launch_deposit(")
     assert "max_fix" in text[:at] and not unordered(text, at)
+
+
+@pytest.mark.parametrize("file,head", [
+    ("native_fft.cu", "int fft_native_init("),   # the twiddle table, read by the first transform on any stream
+])
+def test_set_up_is_complete_when_it_returns(file, head):
+    text = body(file, head)
+    assert LEGACY.search(text) and not unordered(text, len(text))
