@@ -409,6 +409,7 @@ int ic_work(int device, int N, int path, ICWork** out) {
     CU(cudaMalloc(&w.part, sizeof(double) * (kRmsBlocks + 1)));
     CU(cudaMalloc(&w.count, sizeof(u32)));
     CU(cudaMemset(w.count, 0, sizeof(u32)));
+    CU(cudaStreamSynchronize(0));  // the caller's stream may not wait for the default one
     w.ok = true;
   done:
     if (rc) {

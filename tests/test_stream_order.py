@@ -55,6 +55,7 @@ def test_the_counts_kernels_start_from_cleared_statistics():
 
 @pytest.mark.parametrize("file,head", [
     ("native_fft.cu", "int fft_native_init("),   # the twiddle table, read by the first transform on any stream
+    ("ic.cu", "int ic_work("),                   # the rms kernel's ticket, counted on the caller's stream
 ])
 def test_set_up_is_complete_when_it_returns(file, head):
     text = body(file, head)
