@@ -460,7 +460,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
                 (long long)(BIN_SLACK_MIN + BIN_ALIGN) * P.nst + BIN_ALIGN - 1) / BIN_ALIGN * BIN_ALIGN;
     roff += P.r_size;
     P.mv_off = E->nmoves;
-    E->nmoves += npart / MOVE_PIECE + 2LL * P.nst;  // two runs per bin, each rounded up to whole pieces
+    E->nmoves += piece_room(npart, P.nst);
     P.st_base = stb;
     P.sst_off = sso;
     P.face_off = fo;
@@ -693,6 +693,7 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemset(E->new_count, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->load_count, 0, sizeof(u32) * E->nst));
   CU(cudaMemset(E->n_moves, 0, sizeof(u32) * npeaks));
+  CU(cudaMemset(E->moves, 0, sizeof(uint4) * (E->nmoves ? E->nmoves : 1)));
   CU(cudaMemset(E->layout_gate, 0, sizeof(u32)));
   CU(cudaMemset(E->epart, 0, sizeof(double2) * 4 * E->nst));
   CU(cudaMemset(E->wpart, 0, sizeof(double) * E->nmodeblk * (PM_THREADS / 32)));

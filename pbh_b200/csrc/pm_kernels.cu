@@ -510,7 +510,7 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
     const int n0 = min(R.n0, n);
     const u32 p0 = (u32)(n0 + MOVE_PIECE - 1) / MOVE_PIECE, p1 = (u32)(n - n0 + MOVE_PIECE - 1) / MOVE_PIECE;
     u32 q = atomicAdd(&s_moves, p0 + p1);
-    if (q + p0 + p1 > (u32)(P.n / MOVE_PIECE + 2LL * P.nst)) {  // more particles than the peak has: corrupted bins
+    if (!piece_fits(q, p0 + p1, piece_room(P.n, P.nst))) {  // more particles than the peak has: corrupted bins
       bad = true;
       return;
     }
@@ -582,7 +582,7 @@ __device__ __forceinline__ void layout_peak(const StepArgs& A, int pk, const Pea
   if (threadIdx.x == 0) {
     if (C.sortstep) A.ovf_n[pk] = 0u;
     if (C.relayout) {
-      A.n_moves[pk] = s_moves;
+      A.n_moves[pk] = pieces_published(s_moves, piece_room(P.n, P.nst));
       A.clocks[pk].relayout = partial ? 1 : 2;
       if (!partial) {  // the full relayout fills the other buffer, which becomes current
         A.clocks[pk].sbuf = C.sbuf ^ 1;
@@ -941,9 +941,13 @@ __global__ void __launch_bounds__(PM_THREADS) k_relayout(const __grid_constant__
     const float4* im = bmom(A, src);
     int4* op = bpos(A, sbuf);
     float4* om = bmom(A, sbuf);
-    const u32 nmv = A.n_moves[pk];
+    const u32 nmv = min(A.n_moves[pk], (u32)piece_room(P.n, P.nst));
     for (u32 q = blockIdx.x; q < nmv; q += gridDim.x) {
       const uint4 mv = A.moves[P.mv_off + q];
+      if (!piece_inside(mv.x, mv.y, mv.z, P.r_off, P.r_size)) {  // never outside the peak's bins
+        if (threadIdx.x == 0) atomicOr(&A.stats[pk].status, 4u);
+        continue;
+      }
       static_assert(MOVE_PIECE % (4 * PM_THREADS) == 0, "four particles per thread and round");
       for (u32 k = threadIdx.x; k < mv.z; k += 4 * PM_THREADS) {  // old and new places never overlap
         int4 p[4];

@@ -75,6 +75,20 @@ struct BinLayout {
   u32 base, cap;  // slot offset in a bin buffer, capacity
 };
 
+// The list of pieces of a peak's relayout (StepArgs::moves).  Bins that hold together what the peak
+// has fit piece_room entries: two runs per bin, each rounded up to whole pieces.  Bins that disagree with
+// their peak (corrupted fills) may ask for more: a bin that finds no room writes no entry, and
+// then the list is not published at all, so that no entry is copied that was not written.
+__host__ __device__ __forceinline__ long long piece_room(long long n, long long nst) { return n / MOVE_PIECE + 2 * nst; }
+__host__ __device__ __forceinline__ bool piece_fits(u32 first, u32 pieces, long long room) {
+  return (long long)first + pieces <= room;
+}
+__host__ __device__ __forceinline__ u32 pieces_published(u32 asked, long long room) { return asked <= room ? asked : 0u; }
+// Whether a piece reads and writes inside the peak's bin region [r_off, r_off + r_size).
+__host__ __device__ __forceinline__ bool piece_inside(u32 src, u32 dst, u32 count, long long r_off, long long r_size) {
+  return src >= r_off && dst >= r_off && (long long)src + count <= r_off + r_size && (long long)dst + count <= r_off + r_size;
+}
+
 // Views of the engine's device arrays handed to every kernel.
 struct StepArgs {
   const PeakDesc* peaks;
