@@ -856,6 +856,7 @@ int pm_step_explicit(pm_engine* e, int peak, double a, double da) {
   if (!e || peak < 0 || peak >= e->npeaks) return -2000;
   if (!(a > 0) || !(da > 0)) return -2001;
   CU(cudaSetDevice(e->device));
+  e->occupied[peak] = 1;  // dynamic mode: the solve covers this slot from here on, also after a release
   int r;
   // A run of steps that each start where the last one ended (the driver's loop): nothing to read
   // back, one round trip per step instead of two.
