@@ -237,7 +237,7 @@ struct pm_engine {
     int k = 0;
     auto mark = [&]() -> cudaError_t { return ev ? cudaEventRecord(ev[k++], stream) : cudaSuccess; };
     CU(mark());
-    launch_push(A, nst, smem_push, stream);
+    launch_push(A, nst, ntot, smem_push, stream);
     CU(mark());
     launch_tick(A, stream);
     CU(mark());

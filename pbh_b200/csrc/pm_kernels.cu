@@ -346,9 +346,8 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
   }
 }
 
-// PT threads per CTA: PUSH_THREADS, or PUSH_THREADS_SMALL when no super-tile is larger than 8^3 cells
-// (512 particles are then four sweeps, whose loads overlap, instead of one).
-template <int PT>
+// PT threads per CTA (push_threads).  TS16: the engine has super-tiles of 16^3 cells.
+template <int PT, bool TS16>
 __global__ void __launch_bounds__(PT, 1024 / PT) k_push(const __grid_constant__ StepArgs A) {
   extern __shared__ __align__(16) float s_f[];
   __shared__ u32 s_stay;
@@ -382,7 +381,7 @@ __global__ void __launch_bounds__(PT, 1024 / PT) k_push(const __grid_constant__ 
       else push_super<8, 0, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       break;
     default:
-      if (PT == PUSH_THREADS_SMALL) break;
+      if (!TS16) break;
       if (sb) push_super<16, 1, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       else push_super<16, 0, PT>(A, P, tr.pk, st, s_f, &s_stay, K, L, F);
       break;
@@ -2010,7 +2009,7 @@ size_t pm_tile_sort_smem() {
 
 int pm_kernels_init() {
   cudaError_t e =
-      cudaFuncSetAttribute(k_push<PUSH_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      cudaFuncSetAttribute(k_push<PUSH_THREADS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pm_tile_sort_smem());
@@ -2019,21 +2018,48 @@ int pm_kernels_init() {
 
 static unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// Grid of a grid-stride kernel: enough CTAs to fill every SM `per_sm` times, fewer for small n.
-static unsigned stride_grid(long long n, int t, int per_sm) {
+static int num_sms() {
   static int sms = 0;
   if (!sms) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       sms = 148;
   }
-  const long long g = std::min<long long>((long long)nb(n, t), (long long)sms * per_sm);
+  return sms;
+}
+
+// Grid of a grid-stride kernel: enough CTAs to fill every SM `per_sm` times, fewer for small n.
+static unsigned stride_grid(long long n, int t, int per_sm) {
+  const long long g = std::min<long long>((long long)nb(n, t), (long long)num_sms() * per_sm);
   return (unsigned)std::max<long long>(g, 1);
 }
 
-void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s) {
-  if (smem <= pm_push_smem(8)) pdl_launch(k_push<PUSH_THREADS_SMALL>, dim3((unsigned)nst), PUSH_THREADS_SMALL, smem, s, A);
-  else pdl_launch(k_push<PUSH_THREADS>, dim3((unsigned)nst), PUSH_THREADS, smem, s, A);
+// Threads of a push CTA when no super-tile is larger than 8^3 cells.  Narrow CTAs let more super-tiles
+// reside at once, and 512 particles are then several sweeps whose loads overlap; wide ones take a
+// dense super-tile (collapse, many particles per cell) in fewer sweeps.  So the widest with which
+// every super-tile still resides at once (1024 threads an SM), 128 beyond that; 512 only for
+// super-tiles that fill them.  us a step with 128, 256, 512 threads: 64 super-tiles (one 32^3 peak)
+// 28.8, 26.9, 27.0, of 64 particles 27.0, 27.0, 29.0, of 4096 46.0, 40.3, 39.3, of 32768 257, 190, 167; 512
+// (one 64^3 peak) 37.5, 37.1, 42.3, in collapse (maximum density contrast 450) 65.5, 57.1, 55.1; 1024
+// (two 64^3 peaks) 47.2, 49.3, 55.6; 4096 (a 128^3 mesh of 8^3 super-tiles) 137, 145, 175.  What stays is
+// that beyond 592 super-tiles a cloud that lies in a few of them waits for its 128 threads: 2e6
+// particles in 2 % of a 128^3 box 25.7 ms a step, 16.0 with 512.
+static int push_threads(long long nst, long long ntot) {
+  const long long sms = num_sms();
+  if (nst <= 2 * sms && ntot >= 512 * nst) return 512;
+  return nst <= 4 * sms ? 256 : 128;
+}
+void launch_push(const StepArgs& A, long long nst, long long ntot, size_t smem, cudaStream_t s) {
+  const dim3 grid((unsigned)nst);
+  if (smem > pm_push_smem(8)) {
+    pdl_launch(k_push<PUSH_THREADS, true>, grid, PUSH_THREADS, smem, s, A);
+    return;
+  }
+  switch (push_threads(nst, ntot)) {
+    case 512: pdl_launch(k_push<512, false>, grid, 512, smem, s, A); break;
+    case 256: pdl_launch(k_push<256, false>, grid, 256, smem, s, A); break;
+    default: pdl_launch(k_push<128, false>, grid, 128, smem, s, A); break;
+  }
 }
 void launch_tick(const StepArgs& A, cudaStream_t s) {
   pdl_launch(k_tick, dim3(A.npeaks), LAYOUT_THREADS, 0, s, A);

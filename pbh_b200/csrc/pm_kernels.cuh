@@ -29,7 +29,6 @@
 
 #define PM_THREADS 256
 #define PUSH_THREADS 512
-#define PUSH_THREADS_SMALL 128
 #define DEP_THREADS 256    // deposit CTA (4 per SM)
 #define GREEN_MODES 4      // modes per thread of the Green kernel (a block covers PM_THREADS * GREEN_MODES)
 // Most cells of an engine whose deposit adds its node sums to the meshes (PeakDesc::rho) instead of
@@ -153,7 +152,7 @@ int pm_kernels_init();  // kernel attributes; call once per device before launch
 size_t pm_deposit_smem(int TSmax);
 size_t pm_push_smem(int TSmax);
 
-void launch_push(const StepArgs& A, long long nst, size_t smem, cudaStream_t s);
+void launch_push(const StepArgs& A, long long nst, long long ntot, size_t smem, cudaStream_t s);
 void launch_tick(const StepArgs& A, cudaStream_t s);
 void launch_load_count(const StepArgs& A, long long ntot, cudaStream_t s);
 void launch_load_place(const StepArgs& A, long long ntot, cudaStream_t s);
