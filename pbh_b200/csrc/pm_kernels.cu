@@ -1847,79 +1847,134 @@ __global__ void __launch_bounds__(PM_THREADS) k_reload(StepArgs A, int pk, PeakD
 // per super-tile of the peak walks its bin; a peak loaded but not yet primed has its particles in
 // the loading area instead, where CTA t takes the t-th slice.
 //
+// What a particle's output rows are made of.  id: its row, -1 when there is none.
+struct ReadRow {
+  int id, ii[3];
+  float f[3], mv[3];
+  double g[3];
+};
+__device__ __forceinline__ ReadRow read_row(const StepArgs& A, int pk, const PeakDesc& P, bool valid, bool need_g, int4 ps,
+                                            float4 m) {
+  const int N = P.N;
+  ReadRow r{valid ? __float_as_int(m.w) : -1,
+            {(ps.x >> (2 * P.log2N)) & (N - 1), (ps.x >> P.log2N) & (N - 1), ps.x & (N - 1)},
+            {__int_as_float(ps.y), __int_as_float(ps.z), __int_as_float(ps.w)},
+            {m.x, m.y, m.z},
+            {0.0, 0.0, 0.0}};
+  if (valid && (r.id < 0 || r.id >= P.n)) {  // never write through an id that is not a lattice index
+    atomicOr(&A.stats[pk].status, 8u);
+    r.id = -1;
+  }
+  if (need_g && r.id >= 0) {
+    const long long N3 = (long long)N * N * N;
+    for (int c = 0; c < 8; ++c) {
+      const int cx = c >> 2, cy = (c >> 1) & 1, cz = c & 1;
+      const float w = (cx ? r.f[0] : 1.0f - r.f[0]) * (cy ? r.f[1] : 1.0f - r.f[1]) * (cz ? r.f[2] : 1.0f - r.f[2]);
+      const long long o =
+          ((long long)((r.ii[0] + cx) & (N - 1)) * N + ((r.ii[1] + cy) & (N - 1))) * N + ((r.ii[2] + cz) & (N - 1));
+      r.g[0] += w * P.force[o];
+      r.g[1] += w * P.force[N3 + o];
+      r.g[2] += w * P.force[2 * N3 + o];
+    }
+  }
+  return r;
+}
+__device__ __forceinline__ double row_x(const PeakDesc& P, const ReadRow& r, int d) {
+  const double X = ((double)r.ii[d] + (double)r.f[d] + 0.5) * P.dx;
+  return X >= P.L ? X - P.L : X;
+}
+// kick: the pending closing kick for forces of unit expansion factor; scale: the forces' factor.
+struct ReadScale {
+  double kick, scale;
+  bool need_g;
+};
+__device__ __forceinline__ ReadScale read_scale(const PeakClock& C, const double* p, const double* acc, double a_acc) {
+  return ReadScale{C.kpend != 0.0 ? C.kpend * (C.a_grid / C.a) : 0.0, C.a_grid / a_acc,
+                   C.has_delta && ((p && C.kpend != 0.0) || acc)};
+}
+
+// One particle, its lane writing the rows.
+__device__ __forceinline__ void get_one(const StepArgs& A, int pk, const PeakDesc& P, const ReadScale& S, int4 ps, float4 m,
+                                        double* __restrict__ x, double* __restrict__ p, double* __restrict__ acc) {
+  const ReadRow r = read_row(A, pk, P, true, S.need_g, ps, m);
+  if (r.id < 0) return;
+  const long long o = 3LL * r.id;
+  for (int d = 0; d < 3; ++d) {
+    if (x) x[o + d] = row_x(P, r, d);
+    if (p) p[o + d] = (double)r.mv[d] + S.kick * r.g[d];
+    if (acc) acc[o + d] = r.g[d] * S.scale;
+  }
+}
+
 // A warp takes 32 particles (`valid` lanes) and writes their 24-byte rows of each output through
 // `row` (96 doubles of shared memory per warp), eight bytes per lane in the rows' own order: a
 // bin's neighbours are lattice neighbours, so this covers whole sectors, where one row per lane and
 // one column at a time touched each of them three times (256^3: 679 -> 303 us, 658 -> 507
-// with a pending kick, whose gather from the force grids then dominates).
-__device__ __forceinline__ void get_warp(const StepArgs& A, int pk, const PeakDesc& P, const PeakClock& C, bool valid,
+// with a pending kick, whose gather from the force grids then dominates).  STAGED false: each lane writes
+// its own row (see k_get_particles).
+template <bool STAGED>
+__device__ __forceinline__ void get_warp(const StepArgs& A, int pk, const PeakDesc& P, const ReadScale& S, bool valid,
                                          int4 ps, float4 m, double* row, double* __restrict__ x,
-                                         double* __restrict__ p, double* __restrict__ acc, double a_acc) {
-  const int N = P.N, lane = threadIdx.x & 31;
-  const int ii[3] = {(ps.x >> (2 * P.log2N)) & (N - 1), (ps.x >> P.log2N) & (N - 1), ps.x & (N - 1)};
-  const float f[3] = {__int_as_float(ps.y), __int_as_float(ps.z), __int_as_float(ps.w)};
-  int id = valid ? __float_as_int(m.w) : -1;
-  if (valid && (id < 0 || id >= P.n)) {  // never write through an id that is not a lattice index
-    atomicOr(&A.stats[pk].status, 8u);
-    id = -1;
-  }
-  double g[3] = {0.0, 0.0, 0.0};
-  const bool need_g = C.has_delta && ((p && C.kpend != 0.0) || acc);
-  if (need_g && valid) {
-    const long long N3 = (long long)N * N * N;
-    for (int c = 0; c < 8; ++c) {
-      const int cx = c >> 2, cy = (c >> 1) & 1, cz = c & 1;
-      const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-      const long long o = ((long long)((ii[0] + cx) & (N - 1)) * N + ((ii[1] + cy) & (N - 1))) * N + ((ii[2] + cz) & (N - 1));
-      g[0] += w * P.force[o];
-      g[1] += w * P.force[N3 + o];
-      g[2] += w * P.force[2 * N3 + o];
-    }
-  }
+                                         double* __restrict__ p, double* __restrict__ acc) {
+  const int lane = threadIdx.x & 31;
+  const ReadRow r = read_row(A, pk, P, valid, S.need_g, ps, m);
   auto put = [&](double* __restrict__ out, const double (&v)[3]) {
+    if (!STAGED) {
+      if (r.id >= 0)
+        for (int d = 0; d < 3; ++d) out[3LL * r.id + d] = v[d];
+      return;
+    }
     __syncwarp();
     for (int d = 0; d < 3; ++d) row[3 * lane + d] = v[d];
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const int e = 32 * k + lane, q = e / 3;
-      const int to = __shfl_sync(0xffffffffu, id, q);
+      const int to = __shfl_sync(0xffffffffu, r.id, q);
       if (to >= 0) out[3LL * to + (e - 3 * q)] = row[e];
     }
   };
   double v[3];
   if (x) {
-    for (int d = 0; d < 3; ++d) {
-      v[d] = ((double)ii[d] + (double)f[d] + 0.5) * P.dx;
-      if (v[d] >= P.L) v[d] -= P.L;
-    }
+    for (int d = 0; d < 3; ++d) v[d] = row_x(P, r, d);
     put(x, v);
   }
   if (p) {
-    const double mv[3] = {m.x, m.y, m.z}, k = C.kpend != 0.0 ? C.kpend * (C.a_grid / C.a) : 0.0;
-    for (int d = 0; d < 3; ++d) v[d] = mv[d] + k * g[d];
+    for (int d = 0; d < 3; ++d) v[d] = (double)r.mv[d] + S.kick * r.g[d];
     put(p, v);
   }
   if (acc) {
-    for (int d = 0; d < 3; ++d) v[d] = g[d] * (C.a_grid / a_acc);
+    for (int d = 0; d < 3; ++d) v[d] = r.g[d] * S.scale;
     put(acc, v);
   }
 }
 
+// DENSE: bins of more than a few warps (READ_MEAN particles in the mean).  Many such bins share the
+// memory system, and their rows go through shared memory.  A bin denser than READ_DENSE times the mean,
+// and each of a few (READ_BINS), is alone with its CTA's latency, where lanes that write their own rows are
+// faster.  us with own and staged rows: 262144 particles in one bin 569 and 724, in 1/1000 of a 64^3 mesh
+// 568 and 722, eight bins of 32768 107 and 121; 512 bins of 1728 56 and 44, 256^3 483 and 349.  Smaller bins
+// (a 128^3 mesh of 4^3 super-tiles, 64 particles each) need many CTAs on an SM: 48 registers and no shared
+// memory 116, own rows in the larger kernel 129, staged 132.
+#define READ_DENSE 32
+#define READ_BINS 128
+#define READ_MEAN 128
+template <bool DENSE>
 __global__ void __launch_bounds__(PM_THREADS) k_get_particles(StepArgs A, int pk, PeakDesc P, double* __restrict__ x,
                                                               double* __restrict__ p, double* __restrict__ acc,
                                                               double a_acc) {
-  __shared__ double s_row[PM_THREADS * 3];
-  double* const row = s_row + (threadIdx.x >> 5) * 96;
-  const PeakClock C = A.clocks[pk];
+  __shared__ double s_row[DENSE ? PM_THREADS * 3 : 1];
+  double* const row = s_row + (DENSE ? (threadIdx.x >> 5) * 96 : 0);
   const int lane = threadIdx.x & 31;
-  if (C.state == PS_PRIME) {
-    const long long per = (P.n + P.nst - 1) / P.nst;
-    const long long i0 = per * blockIdx.x, i1 = min(P.n, i0 + per);
-    for (long long i = i0 + threadIdx.x; i - lane < i1; i += PM_THREADS) {
-      const bool v = i < i1;
+  const PeakClock C = A.clocks[pk];
+  const ReadScale S = read_scale(C, p, acc, a_acc);
+  if (C.state == PS_PRIME) {  // still in the loading area
+    const long long per = (P.n + P.nst - 1) / P.nst, i0 = per * blockIdx.x, i1 = min(P.n, i0 + per);
+    for (long long i = i0 + threadIdx.x; i - (DENSE ? lane : 0) < i1; i += PM_THREADS) {
+      const bool v = !DENSE || i < i1;
       const long long j = P.p_off + (v ? i : i0);
-      get_warp(A, pk, P, C, v, A.lpos[j], A.lmom[j], row, x, p, acc, a_acc);
+      if (DENSE) get_warp<true>(A, pk, P, S, v, A.lpos[j], A.lmom[j], row, x, p, acc);
+      else get_one(A, pk, P, S, A.lpos[j], A.lmom[j], x, p, acc);
     }
     return;
   }
@@ -1928,10 +1983,18 @@ __global__ void __launch_bounds__(PM_THREADS) k_get_particles(StepArgs A, int pk
   const int4* ip = bpos(A, C.sbuf);
   const float4* im = bmom(A, C.sbuf);
   const int n = R.total();
-  for (int k = threadIdx.x; k - lane < n; k += PM_THREADS) {
-    const bool v = k < n;
-    const long long j = R.slot(v ? k : 0);
-    get_warp(A, pk, P, C, v, ip[j], im[j], row, x, p, acc, a_acc);
+  if (DENSE && P.nst >= READ_BINS && n <= READ_DENSE * (P.n / P.nst)) {
+    for (int k = threadIdx.x; k - lane < n; k += PM_THREADS) {
+      const bool v = k < n;
+      const long long j = R.slot(v ? k : 0);
+      get_warp<true>(A, pk, P, S, v, ip[j], im[j], row, x, p, acc);
+    }
+  } else {
+    for (int k = threadIdx.x; k < n; k += PM_THREADS) {
+      const long long j = R.slot(k);
+      if (DENSE) get_warp<false>(A, pk, P, S, true, ip[j], im[j], row, x, p, acc);
+      else get_one(A, pk, P, S, ip[j], im[j], x, p, acc);
+    }
   }
 }
 
@@ -2116,7 +2179,8 @@ void launch_reload(const StepArgs& A, int pk, const PeakDesc& P, cudaStream_t s)
 }
 void launch_get_particles(const StepArgs& A, int pk, const PeakDesc& P, double* x, double* p, double* acc,
                           double a_acc, cudaStream_t s) {
-  k_get_particles<<<(unsigned)P.nst, PM_THREADS, 0, s>>>(A, pk, P, x, p, acc, a_acc);
+  auto* kernel = P.n >= (long long)READ_MEAN * P.nst ? k_get_particles<true> : k_get_particles<false>;
+  kernel<<<(unsigned)P.nst, PM_THREADS, 0, s>>>(A, pk, P, x, p, acc, a_acc);
 }
 void launch_interp64(const double* F, const double* X, long long n, int N, double dx, double* out, cudaStream_t s) {
   k_interp64<<<nb(n, PM_THREADS), PM_THREADS, 0, s>>>(F, X, n, N, dx, out);
