@@ -391,10 +391,13 @@ __device__ __forceinline__ void col_fft(float2 (&v)[16], float2 (&u)[16], float2
   }
 }
 
-// Rows x = B rb + r of kz planes, T threads per row, [f][kz][.][.] (the plain transforms; in place
-// allowed: a CTA reads its rows before it writes them).  grid (N/B * nplanes).
+// Rows x = B rb + r of kz planes, T threads per row, [f][kz][.][.] (in place allowed: a CTA reads its
+// rows before it writes them).  slot_peak (engine solve): field f is slot f's spectrum, idle slots are
+// skipped.  grid (N/B * nplanes).
 template <int N, bool INV>
-__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_rows(const float2* in, float2* out) {
+__global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_rows(const float2* in, float2* out,
+                                                                           const __grid_constant__ StepArgs A,
+                                                                           const int* slot_peak) {
   using G = PGeo<N>;
   constexpr int T = G::T;
   __shared__ float2 tl[16 * T];
@@ -402,6 +405,7 @@ __global__ void __launch_bounds__(cta<N>(), 1024 / cta<N>()) k_fft_rows(const fl
   load_ptw<N>(tl);
   pdl_wait();
   const int rb = blockIdx.x % G::R, pl = blockIdx.x / G::R;
+  if (slot_peak && !slot_active(A, slot_peak, pl / G::NH)) return;
   const int t = threadIdx.x % T, r = threadIdx.x / T;
   const long long o = (long long)pl * G::N2 + (long long)(G::B * rb + r) * N;
   float2 v[16], u[16];
@@ -761,7 +765,7 @@ int r2c_n(const float* x, float2* spec, int nfields, cudaStream_t s) {
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
   pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s, x, spec, StepArgs{}, nullptr);
-  pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
+  pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec, StepArgs{}, nullptr);
   pdl_launch(k_fft_cols<N, false>, dim3(blocks), G::CTA, 0, s, spec);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e;
@@ -784,7 +788,7 @@ int solve_n(const float* delta, float2* spec, float2* gspec, float* force, const
   } else {
     using Z = ZGeo<N>;
     pdl_launch(k_fft_z_r2c<N>, dim3((unsigned)(Z::N2 / Z::L), nslots), G::CTA, 0, s, delta, spec, A, slot_peak);
-    pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec);
+    pdl_launch(k_fft_rows<N, false>, dim3(blocks), G::CTA, 0, s, spec, spec, A, slot_peak);
     pdl_launch(k_solve_cols<N>, dim3(blocks), G::CTA, G::COLS_SMEM, s, spec, gspec, A, slot_peak);
     pdl_launch(k_solve_rows<N>, dim3(3 * blocks), G::CTA, 0, s, spec, gspec, A, slot_peak);
     pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), 3 * nslots), G::CTA, 0, s, gspec, force, A, slot_peak);
@@ -798,7 +802,7 @@ int c2r_n(const float2* spec, float2* work, float* out, int nfields, cudaStream_
   using Z = ZGeo<N>;
   using G = PGeo<N>;
   const unsigned blocks = (unsigned)G::R * (unsigned)(nfields * G::NH);
-  pdl_launch(k_fft_rows<N, true>, dim3(blocks), G::CTA, 0, s, spec, work);
+  pdl_launch(k_fft_rows<N, true>, dim3(blocks), G::CTA, 0, s, spec, work, StepArgs{}, nullptr);
   pdl_launch(k_fft_cols<N, true>, dim3(blocks), G::CTA, 0, s, work);
   pdl_launch(k_fft_z_c2r<N>, dim3((unsigned)(Z::N2 / Z::L), nfields), G::CTA, 0, s, work, out, StepArgs{}, nullptr);
   const cudaError_t e = cudaGetLastError();
