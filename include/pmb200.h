@@ -228,7 +228,7 @@ int pm_make_ic(const pm_ic_params* prm, double* x_out, double* p_out, double* de
  * for a mesh size (unless Np exceeds 4 N and every Np before; its work area is separate from
  * pm_make_ic's), and reports no noise rms.  The
  * same inputs give the same bits as pm_make_ic.  Calls for one mesh size share the work area:
- * issue them on one stream.  kind 0 returns -2003. */
+ * issue them on one stream (from any host thread).  kind 0 returns -2003. */
 int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* p_out, void* stream);
 /* pm_make_ic and pm_make_ic_async keep their float64 work buffers and cuFFT plans per (device,
  * N) after the first call; this frees them (no counterpart: the reference's make_ic keeps no

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
 #include <utility>
@@ -373,13 +374,16 @@ struct ICWork {
   double* spline = nullptr;              // [spline_n] knots, coefficients
   int spline_n = 0;
   cufftHandle d2z = 0, d2z2 = 0, z2d3 = 0, z2d4 = 0;
-  bool ok = false;
-  std::mutex busy;                       // held through a synchronous call
+  bool ok = false;                       // the buffers are there
+  bool gone = false;                     // released, or could not be made: not in the table any more
+  // Held through a synchronous call, and by an asynchronous one while it plans, grows buffers and
+  // enqueues (host threads that share a work area: their calls follow one another on the stream).
+  std::mutex busy;
 };
-std::mutex g_ic_mu;
+std::mutex g_ic_mu;  // the table; never held while an entry's `busy` is waited for
 // Keyed by (device, N, path): the synchronous pm_make_ic and the stream-ordered
 // pm_make_ic_async keep separate work areas, so the two never share buffers in flight.
-std::map<std::tuple<int, int, int>, ICWork> g_ic;
+std::map<std::tuple<int, int, int>, std::shared_ptr<ICWork>> g_ic;
 
 void ic_free(ICWork& w) {
   cudaFree(w.field);
@@ -395,10 +399,10 @@ void ic_free(ICWork& w) {
     if (h) cufftDestroy(h);
 }
 
-int ic_work(int device, int N, int path, ICWork** out) {
-  std::lock_guard<std::mutex> lock(g_ic_mu);
-  ICWork& w = g_ic[{device, N, path}];
-  if (!w.ok) {
+// The work area, its `busy` held by the caller from here on.
+int ic_work(int device, int N, int path, std::shared_ptr<ICWork>* out, std::unique_lock<std::mutex>* hold) {
+  const std::tuple<int, int, int> key{device, N, path};
+  auto make = [N](ICWork& w) {
     const long long N3 = (long long)N * N * N, M = (long long)N * N * (N / 2 + 1);
     int rc = 0;
     CU(cudaMalloc(&w.field, sizeof(double) * 2 * N3));
@@ -412,14 +416,32 @@ int ic_work(int device, int N, int path, ICWork** out) {
     CU(cudaStreamSynchronize(0));  // the caller's stream may not wait for the default one
     w.ok = true;
   done:
-    if (rc) {
-      ic_free(w);
-      g_ic.erase({device, N, path});
-      return rc;
+    return rc;
+  };
+  for (;;) {
+    std::shared_ptr<ICWork> w;
+    {
+      std::lock_guard<std::mutex> lock(g_ic_mu);
+      std::shared_ptr<ICWork>& e = g_ic[key];
+      if (!e) e = std::make_shared<ICWork>();
+      w = e;
     }
+    std::unique_lock<std::mutex> busy(w->busy);
+    if (w->gone) continue;  // released while this thread waited: a new one
+    if (!w->ok) {
+      if (int rc = make(*w)) {
+        ic_free(*w);
+        w->gone = true;
+        std::lock_guard<std::mutex> lock(g_ic_mu);
+        const auto it = g_ic.find(key);
+        if (it != g_ic.end() && it->second == w) g_ic.erase(it);
+        return rc;
+      }
+    }
+    *out = std::move(w);
+    *hold = std::move(busy);
+    return 0;
   }
-  *out = &w;
-  return 0;
 }
 
 // A plan of the work area, made when it is first used (each holds cuFFT scratch of its own).
@@ -452,12 +474,19 @@ cudaError_t grow(T** buf, int* have, int n, cudaStream_t s) {
 }  // namespace
 
 extern "C" int pm_ic_release_cache(void) {
-  std::lock_guard<std::mutex> lock(g_ic_mu);
-  for (auto& kv : g_ic) {
-    cudaSetDevice(std::get<0>(kv.first));
-    ic_free(kv.second);
+  std::map<std::tuple<int, int, int>, std::shared_ptr<ICWork>> all;
+  {
+    std::lock_guard<std::mutex> lock(g_ic_mu);
+    all.swap(g_ic);
   }
-  g_ic.clear();
+  for (auto& kv : all) {
+    std::lock_guard<std::mutex> busy(kv.second->busy);  // a call that has it finishes first
+    if (kv.second->gone) continue;
+    kv.second->gone = true;
+    cudaSetDevice(std::get<0>(kv.first));
+    cudaDeviceSynchronize();  // what asynchronous calls have enqueued
+    ic_free(*kv.second);
+  }
   return 0;
 }
 
@@ -546,19 +575,18 @@ extern "C" int pm_make_ic(const pm_ic_params* prm, double* x_out, double* p_out,
   if (int r = check_params(prm, x_out, p_out)) return r;
   int rc = 0, device = 0;
   double rms = 0.0;
-  ICWork* w = nullptr;
-  std::unique_lock<std::mutex> hold;
+  std::shared_ptr<ICWork> w;
+  std::unique_lock<std::mutex> hold;  // released before w
   CU(cudaGetDevice(&device));
-  rc = ic_work(device, prm->N, 0, &w);
+  rc = ic_work(device, prm->N, 0, &w, &hold);
   if (rc) return rc;
-  hold = std::unique_lock<std::mutex>(w->busy);
   if (prm->kind == 0) {
     const int m = prm->spline_m;
     CU(grow(&w->spline, &w->spline_n, 5 * m + 1, 0));
     CU(cudaMemcpyAsync(w->spline, prm->spline_x, sizeof(double) * (m + 1), cudaMemcpyHostToDevice, 0));
     CU(cudaMemcpyAsync(w->spline + m + 1, prm->spline_c, sizeof(double) * 4 * m, cudaMemcpyHostToDevice, 0));
   }
-  rc = make_ic_on(prm, x_out, p_out, delta_lin_out, w, 0);
+  rc = make_ic_on(prm, x_out, p_out, delta_lin_out, w.get(), 0);
   if (rc) goto done;
   CU(cudaMemcpyAsync(&rms, w->part + kRmsBlocks, sizeof(rms), cudaMemcpyDeviceToHost, 0));
   CU(cudaDeviceSynchronize());
@@ -573,10 +601,11 @@ extern "C" int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* 
   int device = 0;
   const cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return -(int)e;
-  ICWork* w = nullptr;
-  if (int r = ic_work(device, prm->N, 1, &w)) return r;
+  std::shared_ptr<ICWork> w;
+  std::unique_lock<std::mutex> hold;  // released before w
+  if (int r = ic_work(device, prm->N, 1, &w, &hold)) return r;
   cufftResult f = use_plan(&w->d2z, prm->N, CUFFT_D2Z, 1, (cudaStream_t)stream);  // both now, noise or not
   if (f == CUFFT_SUCCESS) f = use_plan(&w->z2d3, prm->N, CUFFT_Z2D, 3, (cudaStream_t)stream);
   if (f != CUFFT_SUCCESS) return -1000 - (int)f;
-  return make_ic_on(prm, x_out, p_out, nullptr, w, (cudaStream_t)stream);
+  return make_ic_on(prm, x_out, p_out, nullptr, w.get(), (cudaStream_t)stream);
 }
