@@ -225,8 +225,7 @@ typedef struct {
 int pm_make_ic(const pm_ic_params* prm, double* x_out, double* p_out, double* delta_lin_out, double* noise_rms_out);
 /* pm_make_ic for the recipe peak (kind 1, noise from a device array or noise_seed) ordered on
  * `stream` (a cudaStream_t): returns without waiting, allocates nothing after its first call
- * for a mesh size (unless Np exceeds 4 N and every Np before; its work area is separate from
- * pm_make_ic's), and reports no noise rms.  The
+ * for a mesh size (its work area is separate from pm_make_ic's), and reports no noise rms.  The
  * same inputs give the same bits as pm_make_ic.  Calls for one mesh size share the work area:
  * issue them on one stream (from any host thread).  kind 0 returns -2003. */
 int pm_make_ic_async(const pm_ic_params* prm, double* x_out, double* p_out, void* stream);

@@ -356,6 +356,9 @@ __global__ void __launch_bounds__(kThreads) k_lattice(int N, int Np, double L, c
 }
 
 constexpr int kRmsBlocks = 592;
+// Entries of the axis table from the first call on: particles of more per side (48 bytes each, 412 GB)
+// do not fit the GPU, so that no later call grows it.
+constexpr int kAxis = 2048;
 
 unsigned nblk(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
@@ -528,7 +531,7 @@ int make_ic_on(const pm_ic_params* prm, double* x_out, double* p_out, double* de
   g.spec = w->spec;
   g.ns = noisy ? w->spec + M : nullptr;
   g.shape = Shape{prm->kind, (double)N3, L, prm->tail_rms, prm->k1, prm->k2};
-  CU(grow(&w->axis, &w->axis_n, std::max(Np, 4 * N), s));  // most lattices fit from the first call on
+  CU(grow(&w->axis, &w->axis_n, std::max(Np, kAxis), s));
   k_lattice_axis<<<nblk(Np), kThreads, 0, s>>>(N, Np, L, w->axis);
   if (noisy && !prm->noise) {  // seeded device noise
     k_philox_normal<<<nblk((N3 + 3) / 4), kThreads, 0, s>>>(w->field + N3, N3, prm->noise_seed);

@@ -88,3 +88,26 @@ def test_host_threads_that_share_a_work_area(release):
     for (N, Np, seed), (x, p) in zip(jobs, out):
         a, b, _, _ = _sync(N, Np, seed)
         assert torch.equal(x, a) and torch.equal(p, b), (N, Np, seed)
+
+
+def test_later_calls_of_a_mesh_size_allocate_nothing():
+    import torch
+    from pbh_b200 import _lib
+    lib = _lib.load()
+    lib.pm_ic_release_cache()
+    s = torch.cuda.Stream()
+    bufs = {Np: _buffers(Np) for Np in (8, 33, 96, 200)}
+    torch.cuda.synchronize()
+    for k, (Np, (x, p)) in enumerate(bufs.items()):
+        prm = _params(8, Np, seed=k + 1)
+        if k == 0:
+            _lib.check(lib.pm_make_ic_async(C.byref(prm), x.data_ptr(), p.data_ptr(), s.cuda_stream), "async")
+            s.synchronize()
+            continue
+        g = torch.cuda.CUDAGraph()      # a capture refuses the calls that an allocation needs
+        with torch.cuda.graph(g, stream=s):
+            rc = lib.pm_make_ic_async(C.byref(prm), x.data_ptr(), p.data_ptr(), s.cuda_stream)
+        assert rc == 0
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(x, _sync(8, Np, k + 1)[0])
