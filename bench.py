@@ -321,6 +321,7 @@ def algorithmic_bytes(phase: str, n: int, cells: int, modes: int, npass: int) ->
 PHASES = ["push", "advance", "regroup", "refresh", "deposit", "r2c", "green", "c2r"]
 NATIVE_FFT_SIZES = (64, 128, 256, 512)   # meshes with a plain native transform
 NATIVE_SOLVE_SIZES = (32, 64, 128, 256, 512)   # meshes whose forces the native solve makes (the others use cuFFT)
+NODE_SUM_CELLS = 2 ** 19                 # most cells of an engine whose deposit needs no fix-up launch
 
 
 def launches_per_step(sizes, fft: str) -> int:
@@ -338,10 +339,12 @@ def step_launches(sizes, fft: str, refresh: bool = False) -> int:
     push, clock, relayout copies (gated: they return at once unless a push overflowed a bin),
     deposit (with the energies) and fix-up; the super-tile re-sort with a refresh period; per
     natively solved mesh size 3 launches up to 128^3 and 5 above; the Green kernel when a mesh size
-    is on cuFFT (whose own launches are not ours)."""
+    is on cuFFT (whose own launches are not ours).  No fix-up when every mesh is natively solved,
+    32^3 or 64^3, and they have at most NODE_SUM_CELLS cells in all."""
     native = {n for n in sizes if fft == "native" and n in NATIVE_SOLVE_SIZES}
     rest = any(n not in native for n in sizes)
-    return 5 + int(refresh) + sum(3 if n <= 128 else 5 for n in native) + int(rest)
+    node_sums = not rest and all(n <= 64 for n in sizes) and sum(n ** 3 for n in sizes) <= NODE_SUM_CELLS
+    return 5 - int(node_sums) + int(refresh) + sum(3 if n <= 128 else 5 for n in native) + int(rest)
 
 
 # DRAM bytes (read + write) per launch from single-kernel ncu captures of the plain 256^3 run
