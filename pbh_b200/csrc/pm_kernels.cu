@@ -322,7 +322,7 @@ __device__ __forceinline__ void push_super(const StepArgs& A, const PeakDesc& P,
   }
   // Super-tile partials of the momentum and p^2 sums, in a fixed order: a plain FP64 tree over
   // the 32 lanes of a warp (about 5e-16 of the sum of magnitudes; compensating it cost 4 % of the
-  // push), then compensated merges across the warps here and across super-tiles in k_tick.
+  // push), then compensated merges across the warps here and across super-tiles in the energy CTAs.
   __shared__ double s_e[PT / 32][4];
   const double ea[4] = {ex, ey, ez, ep};
 #pragma unroll
@@ -1889,8 +1889,8 @@ struct ReadScale {
   bool need_g;
 };
 __device__ __forceinline__ ReadScale read_scale(const PeakClock& C, const double* p, const double* acc, double a_acc) {
-  return ReadScale{C.kpend != 0.0 ? C.kpend * (C.a_grid / C.a) : 0.0, C.a_grid / a_acc,
-                   C.has_delta && ((p && C.kpend != 0.0) || acc)};
+  const bool kick = p && C.kpend != 0.0;
+  return ReadScale{kick ? C.kpend * (C.a_grid / C.a) : 0.0, acc ? C.a_grid / a_acc : 0.0, C.has_delta && (kick || acc)};
 }
 
 // One particle, its lane writing the rows.
@@ -1983,7 +1983,7 @@ __global__ void __launch_bounds__(PM_THREADS) k_get_particles(StepArgs A, int pk
   const int4* ip = bpos(A, C.sbuf);
   const float4* im = bmom(A, C.sbuf);
   const int n = R.total();
-  if (DENSE && P.nst >= READ_BINS && n <= READ_DENSE * (P.n / P.nst)) {
+  if (DENSE && P.nst >= READ_BINS && (long long)n * P.nst <= READ_DENSE * P.n) {
     for (int k = threadIdx.x; k - lane < n; k += PM_THREADS) {
       const bool v = k < n;
       const long long j = R.slot(v ? k : 0);
@@ -2099,18 +2099,18 @@ static unsigned stride_grid(long long n, int t, int per_sm) {
 
 // Threads of a push CTA when no super-tile is larger than 8^3 cells.  Narrow CTAs let more super-tiles
 // reside at once, and 512 particles are then several sweeps whose loads overlap; wide ones take a
-// dense super-tile (collapse, many particles per cell) in fewer sweeps.  So the widest with which
-// every super-tile still resides at once (1024 threads an SM), 128 beyond that; 512 only for
-// super-tiles that fill them.  us a step with 128, 256, 512 threads: 64 super-tiles (one 32^3 peak)
-// 28.8, 26.9, 27.0, of 64 particles 27.0, 27.0, 29.0, of 4096 46.0, 40.3, 39.3, of 32768 257, 190, 167; 512
-// (one 64^3 peak) 37.5, 37.1, 42.3, in collapse (maximum density contrast 450) 65.5, 57.1, 55.1; 1024
-// (two 64^3 peaks) 47.2, 49.3, 55.6; 4096 (a 128^3 mesh of 8^3 super-tiles) 137, 145, 175.  What stays is
-// that beyond 592 super-tiles a cloud that lies in a few of them waits for its 128 threads: 2e6
-// particles in 2 % of a 128^3 box 25.7 ms a step, 16.0 with 512.
+// dense super-tile (collapse, many particles per cell) in fewer sweeps.  So wide ones where all reside
+// at once anyway (1024 threads an SM) and the particles fill them.  us a step with 128, 256, 512 threads:
+// 64 super-tiles (one 32^3 peak) 28.8, 26.9, 27.0, of 64 particles 27.0, 27.0, 29.0, of 4096 46.0, 40.3,
+// 39.3, of 32768 257, 190, 167; 512 (one 64^3 peak) 37.5, 37.1, 42.3 or, on another GPU, 37.7, 39.4, -, of 4096
+// 88.9, 85.8, 89.4; 1024 (two 64^3 peaks) 47.2, 49.3, 55.6; 4096 (a 128^3 mesh of 8^3 super-tiles) 137, 145,
+// 175.  What stays is that a cloud in a few of many super-tiles waits for its 128 threads: a 64^3 peak
+// in collapse (maximum density contrast 450) 65.5, 57.1, 55.1; 2e6 particles in 2 % of the side of a 128^3
+// box 25.7 ms, 16.0 with 512.
 static int push_threads(long long nst, long long ntot) {
   const long long sms = num_sms();
-  if (nst <= 2 * sms && ntot >= 512 * nst) return 512;
-  return nst <= 4 * sms ? 256 : 128;
+  if (nst <= 2 * sms) return ntot >= 512 * nst ? 512 : 256;
+  return nst <= 4 * sms && ntot >= 2048 * nst ? 256 : 128;
 }
 void launch_push(const StepArgs& A, long long nst, long long ntot, size_t smem, cudaStream_t s) {
   const dim3 grid((unsigned)nst);

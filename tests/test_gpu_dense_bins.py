@@ -32,6 +32,7 @@ def _outputs(N, Np, tile, x, p, peaks=1):
     (32, 16, 1.0, [(4, 1), (8, 1), (8, 10), (16, 1)]),   # sparser than the widest push; 640 super-tiles
     (64, 64, 0.08, [(4, 1), (8, 1), (8, 2), (16, 1)]),   # one place far denser than the mean
     (64, 33, 1.0, [(4, 1), (8, 1), (16, 1)]),
+    (64, 104, 1.0, [(8, 1), (8, 2), (16, 1)]),           # 512 super-tiles of 2197, 1024
 ])
 def test_density_and_number_of_bins_change_no_bit(N, Np, size, forms):
     import torch
