@@ -347,8 +347,8 @@ def step_launches(sizes, fft: str, refresh: bool = False) -> int:
     return 5 - int(node_sums) + int(refresh) + sum(3 if n <= 128 else 5 for n in native) + int(rest)
 
 
-# DRAM bytes (read + write) per launch from single-kernel ncu captures of the plain 256^3 run
-# (the Green kernel's from the same run with cuFFT transforms), per particle (per mode for Green),
+# DRAM bytes (read + write) per launch from ncu captures of the large kernels of one step of the plain
+# 256^3 run (the Green kernel's from the same run with cuFFT transforms), per particle (per mode for Green),
 # scaled to a launch by the particles (modes) it processes; deposit includes its face fix-up.
 NCU_TRAFFIC = {"push": 77.00, "deposit": 27.08, "green_per_mode": 25.89}
 

@@ -218,8 +218,6 @@ __host__ __device__ __forceinline__ u32 pm_morton3(u32 x, u32 y, u32 z) {
 // triple.  Codes nest: key >> (3 log2 TS) is the Morton code of the super-tile.
 __host__ __device__ __forceinline__ u32 pm_cell_key(int ix, int iy, int iz) { return pm_morton3(ix, iy, iz); }
 
-__host__ __device__ __forceinline__ double pm_hubble(double a) { return PM_H_I / (a * sqrt(a)); }
-
 // Unsigned division by an invariant divisor d >= 1 (Granlund & Montgomery 1994, the round-up
 // method for 32-bit operands): with l = ceil(log2 d) and magic = floor(2^32 (2^l - d) / d) + 1,
 // n / d = (umulhi(n, magic) + n) >> l for every 32-bit n (the sum is formed in 64 bits).

@@ -702,8 +702,8 @@ int engine_init(pm_engine* E, const pm_peak_cfg* cfg, int npeaks) {
   CU(cudaMemset(E->refresh_gate, 0, sizeof(u32)));
   CU(cudaMemset(E->sstart, 0, sizeof(u32) * E->nsst));
 
-  // Sort plan: one segment per peak over the whole Morton key (sorted at priming and every
-  // full_every steps; the segment of a peak is active only on those steps).
+  // Sort plan: one segment per peak over the whole Morton key, active in the steps that prime the peak
+  // (run only in engines with a refresh period, or while the sort's test hook is set).
   std::vector<SortSeg> segs(npeaks);
   for (int i = 0; i < npeaks; ++i) {
     const PeakDesc& P = E->peaks[i];

@@ -62,7 +62,8 @@ constexpr int TWN = 512;           // entries of the twiddle table
 
 // Threads per CTA for mesh N: 256, fewer where the mesh has few lines, so that a single small mesh
 // still spreads over the SMs (a pass over the planes of one 64^3 mesh is 132 CTAs of 64 threads
-// rather than 33 of 256; its five launches 34.8 -> 33.7 us, 58 -> 55 us at 128^3).
+// rather than 33 of 256; a solve of five such passes, before the slab kernels, 34.8 -> 33.7 us, 58 ->
+// 55 us at 128^3).
 template <int N>
 __host__ __device__ constexpr int cta() { return N <= 64 ? 64 : N == 128 ? 128 : 256; }
 

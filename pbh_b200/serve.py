@@ -85,7 +85,7 @@ def ic_buffer_bytes(N: int) -> int:
 @dataclass
 class ServerConfig:
     slots: dict = field(default_factory=lambda: {64: 32, 128: 32, 256: 32})
-    tiles: object = None            # {N: super-tile side}, "auto" (autotuned) or None (default 16)
+    tiles: object = None            # {N: super-tile side}, "auto" (autotuned) or None (the engine's own choice)
     budget_bytes: float = 150e9
     delta_collapse: float = 50.0
     keep_delta: bool = True
