@@ -537,7 +537,7 @@ def run_ours(args):
         return NCU_TRAFFIC[name] * n_step if name in NCU_TRAFFIC else None
     roofline = {"bound": "hbm", "kernel": top, "achieved": kern[top]["gbs"], "peak": hbm, "unit": "GB/s",
                 "frac": kern[top]["gbs"] / hbm, "traffic": traffic(top),
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of single-kernel captures of the "
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the large kernels of one step of the "
                                   "plain 256^3 run, per particle, times this launch's particles",
                 "algorithmic_bytes": kern[top]["algorithmic_bytes"], "peak_source": hbm_src,
                 "per_kernel": {k: {"ms": round(v["ms"], 4), "gbs": None if v["gbs"] is None else round(v["gbs"], 1),

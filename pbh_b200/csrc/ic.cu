@@ -505,7 +505,7 @@ int check_params(const pm_ic_params* prm, const double* x_out, const double* p_o
 }
 
 // Bounded by the float64 transforms (cuFFT, 4 back and at most 2 forward: 1.05 of the 1.43 ms of a
-// 256^3 call) and, below 64^3, by its launches (nine).  Before the lines, the Parseval sum, the
+// 256^3 call) and, up to 64^3, by its launches (eleven at 64^3, six of them cuFFT's).  Before the lines, the Parseval sum, the
 // fused spectra and the axis table (a field transform, an inverse transform with two grid
 // reductions for the rms, four passes over the spectra, 64-bit remainders per particle):
 // 2.51 ms at 256^3 with noise and delta_lin, 270 -> 147 us for a 64^3 curvature profile.
